@@ -477,17 +477,18 @@ gw_status gw_close(gw_ctx* ctx) {
                        &ctx->d_status,
                        &ctx->d_walks, &ctx->d_words, &ctx->d_ids, &ctx->d_counts, &ctx->d_paths,
                        &ctx->d_plen, &ctx->d_closure, &ctx->d_pool_offsets, &ctx->d_dest,
-                       &ctx->d_tile_hist, &ctx->d_tile_off, &ctx->d_totals, &ctx->d_minhop,
-                       &ctx->d_scan_temp, &ctx->d_out_ptr, &ctx->d_out_base, &ctx->d_q_sources,
+                       &ctx->d_tile_hist, &ctx->d_minhop, &ctx->d_pool_table, &ctx->d_q_sources,
                        &ctx->d_q_prefix, &ctx->d_q_idbase, &ctx->d_q_toff, &ctx->d_q_tmask, &ctx->d_q_tables,
                        &ctx->d_q_full, &ctx->d_q_ids, &ctx->d_q_counts, &ctx->d_q_visits,
                        &ctx->d_q_cursor, &ctx->d_q_segs, &ctx->d_q_cand})
     b->release();
-  for (gw_devbuf& b : ctx->pools) b.release();
+  ctx->release_pools();
   ctx->h_rowptr.release();
   ctx->h_colidx.release();
   ctx->h_status.release();
   ctx->pool_arena.release();
+  ctx->h_xfer.release();
+  ctx->slots.release();
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->aux_stream) cudaStreamDestroy(ctx->aux_stream);
@@ -542,6 +543,7 @@ gw_status gw_set_residency(gw_ctx* ctx, uint32_t residency, uint32_t nmblocks) {
     ctx->d_vrec.release();
     ctx->d_erec.release();
   } else {
+    ctx->slots.release();
     GW_CUDA(ctx, ctx->d_rowptr.ensure(rp), "rowptr alloc");
     GW_CUDA(ctx, ctx->d_colidx.ensure(ci), "colidx alloc");
     GW_CUDA(ctx, ctx->d_vrec.ensure(gw::vrec_bytes(ctx->nv)), "vrec alloc");

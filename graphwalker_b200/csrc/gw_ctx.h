@@ -110,9 +110,38 @@ struct gw_ctx {
   gw_run_stats stats{};
 
   // blocked engine scratch
-  gw_devbuf d_dest, d_tile_hist, d_tile_off, d_totals, d_minhop, d_scan_temp, d_out_ptr,
-      d_out_base;
-  std::vector<gw_devbuf> pools;   // per-block device pools
+  gw_devbuf d_dest, d_tile_hist, d_minhop, d_pool_table;
+  gw_hostbuf h_xfer;              // what a superstep's kernels and the host tell each other (mapped)
+  // Device slots of the streamed blocks, kept between runs while they are
+  // small (kKeptSlotBytes): allocating and freeing two dozen of them takes
+  // longer than a short run.
+  struct BlockSlots {
+    static constexpr size_t kKeptSlotBytes = 1ull << 30;
+    std::vector<gw_devbuf> csr;
+    std::vector<cudaEvent_t> ready;    // copy finished
+    std::vector<cudaEvent_t> free_ev;  // last kernel reading the slot finished
+    void release() {
+      for (auto& b : csr) b.release();
+      for (auto e : ready) cudaEventDestroy(e);
+      for (auto e : free_ev) cudaEventDestroy(e);
+      csr.clear();
+      ready.clear();
+      free_ev.clear();
+    }
+  } slots;
+  std::vector<gw_devbuf> pools;   // per-block device pools: parts of pool_slab, or allocations of their own
+  gw_devbuf pool_slab;
+  bool in_slab(const void* p) const {
+    const char *q = static_cast<const char*>(p), *s = pool_slab.as<char>();
+    return s && q >= s && q < s + pool_slab.bytes;
+  }
+  void release_pools() {
+    for (gw_devbuf& b : pools) {
+      if (in_slab(b.p)) b = gw_devbuf{};
+      b.release();
+    }
+    pool_slab.release();
+  }
   // The older part of each block's pool, moved to host memory when the device
   // pools exceed pool_budget bytes (0 = no limit): pool_host_n[b] records in
   // the pinned arena's chunks pool_chunks[b], in order.  A block's pool is

@@ -103,6 +103,11 @@ __device__ __forceinline__ void red_add_u32(uint32_t* a, uint32_t v, uint64_t po
                : "memory");
 }
 
+// Programmatic dependent launch: wait until every kernel before this one on
+// the stream has finished and its writes are visible; let the next one start.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Launch-constant parameters of a walk kernel (passed by value, lands in the
 // constant bank).
 struct WalkArgs {

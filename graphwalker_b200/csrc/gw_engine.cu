@@ -13,9 +13,14 @@
 // or a slot filled from pinned host memory by async copies on a side stream),
 // advances every walk of its pool while it stays inside the block, and stably
 // partitions the walks that left into the pools of their new blocks.  The
-// per-block pending counts and minimum hops the policy reads come back from
-// the partition's histogram each superstep, through mapped pinned memory, so
-// no small copy of a superstep queues behind a block copy.
+// three kernels of a superstep (walk, scan, scatter) are queued together: the
+// device keeps the table of pools, so the scatter needs nothing from the
+// host, and the pending counts and minimum hops the policy reads reach the
+// host through mapped pinned memory as soon as the scan is done, while the
+// scatter runs.  Only a superstep that outgrows a pool waits for the host.
+// (At R-MAT scale 22 with 33 blocks and 4.2 M walks, 299 supersteps: 64 us a
+// superstep with five partition launches and a synchronisation before the
+// scatter; see gw_partition.cu.)
 //
 // Streaming differs from findSubGraph in three ways that change neither the
 // order of blocks nor any walk:
@@ -49,22 +54,6 @@ constexpr uint64_t kMappedBytesPerWalk = 128;
 // Blocks copied ahead of their turn at most (1 to 5 measured within 2 % of
 // one another on an out-of-core scale-27 graph, the deeper the faster).
 constexpr size_t kCopyAhead = 3;
-
-struct Slots {
-  // One device slot holds the column slice of one block,
-  //   csr[beg_pos[blocks[b]] .. beg_pos[blocks[b+1]]);
-  // the row pointer of every block stays in HBM.
-  std::vector<gw_devbuf> csr;
-  std::vector<uint32_t> block;      // block held, kNoBlock if empty
-  std::vector<cudaEvent_t> ready;   // copy finished
-  std::vector<cudaEvent_t> free_ev; // last kernel reading the slot finished
-  std::vector<int> slot_of;         // per block: slot index or -1
-  ~Slots() {
-    for (auto& b : csr) b.release();
-    for (auto e : ready) cudaEventDestroy(e);
-    for (auto e : free_ev) cudaEventDestroy(e);
-  }
-};
 
 // chooseBlock (walk.hpp:245-252) over the engine's pending counts.
 uint32_t block_with_max_walks(const std::vector<uint64_t>& walknum) {
@@ -109,7 +98,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   if (p->sink == GW_SINK_PATH_RECORD)
     return ctx->fail(GW_E_INVALID, "PATH_RECORD needs GW_MODE_RESIDENT");
   const uint32_t nb = ctx->nblocks;
-  if (nb + 1 > 8000) return ctx->fail(GW_E_INVALID, "at most 7999 blocks in blocked mode");
+  if (nb >= kMaxBuckets) return ctx->fail(GW_E_INVALID, "at most 7999 blocks in blocked mode");
   // Owned blocks (one rank of a vertex-partitioned run): only the blocks in
   // [own_lo, own_hi) execute, and walks that move to other blocks wait in
   // those blocks' pools for gw_read_pool.  block_hi = 0: every block.
@@ -127,12 +116,49 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   ctx->pool_size.assign(nb, 0);
   ctx->minstep.assign(nb, 0xffff);
   ctx->stats = gw_run_stats{};
+  // Without a budget the pools start as parts of one allocation, each with
+  // room for its walks and an even share of all: one allocation instead of
+  // one per block, and few pools that must grow.  (A budget moves pools out
+  // one by one, so each is then its own.)
+  {
+    uint64_t all = 0, want = 0;
+    bool fits = true;
+    for (uint32_t b = 0; b < nb; ++b) all += ctx->pool_words[b].size();
+    std::vector<uint64_t> room(nb);
+    for (uint32_t b = 0; b < nb; ++b) {
+      const uint64_t m = ctx->pool_words[b].size(), held = ctx->pools[b].bytes / sizeof(gw_walk_rec);
+      if (held < m) fits = false;
+      room[b] = std::max<uint64_t>(held, m + all / nb + 1024);
+      want += room[b];
+    }
+    if (ctx->pool_budget) {
+      if (ctx->pool_slab.p) ctx->release_pools();
+    } else if (!fits) {
+      ctx->release_pools();
+      if (ctx->pool_slab.ensure(want * sizeof(gw_walk_rec)) == cudaSuccess) {
+        uint64_t at = 0;
+        for (uint32_t b = 0; b < nb; ++b) {
+          ctx->pools[b].p = ctx->pool_slab.as<gw_walk_rec>() + at;
+          ctx->pools[b].bytes = room[b] * sizeof(gw_walk_rec);
+          at += room[b];
+        }
+      } else {
+        cudaGetLastError();  // no room for all at once: each pool by itself, below
+      }
+    }
+  }
   std::vector<uint64_t> cap(nb, 0);
   for (uint32_t b = 0; b < nb; ++b) cap[b] = ctx->pools[b].bytes / sizeof(gw_walk_rec);
   // Grown pools come from the stream-ordered allocator, so replacing one
-  // queues its free behind the copy out of it; a pool from gw_walks_add is
-  // retired instead and freed with the events.
+  // queues its free behind the copy out of it; a pool from an earlier run is
+  // retired instead and freed with the events, and a part of the slab stays
+  // with the slab.
   std::vector<char> pool_async(nb, 0);
+  auto retire = [&](uint32_t d, std::vector<void*>* retired) {
+    if (!ctx->pools[d].p || ctx->in_slab(ctx->pools[d].p)) return;
+    if (pool_async[d]) cudaFreeAsync(ctx->pools[d].p, st);
+    else retired->push_back(ctx->pools[d].p);
+  };
   // records of block d's pool held on the device (after its host part)
   auto dev_n = [&](uint32_t d) { return ctx->pool_size[d] - ctx->pool_host_n[d]; };
   constexpr uint64_t kChunk = gw_ctx::kPoolChunk;
@@ -151,11 +177,12 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   // memory, empty pools first giving back their room, until they hold half
   // of it: the headroom takes many supersteps' arrivals before the next
   // spill, so pools move out in a few large batches, not a few every step.
-  auto spill_to_budget = [&]() -> cudaError_t {
+  auto spill_to_budget = [&](bool* moved) -> cudaError_t {
     if (!ctx->pool_budget) return cudaSuccess;
     uint64_t held = 0;
     for (uint32_t d = 0; d < nb; ++d) held += cap[d];
     if (held * sizeof(gw_walk_rec) <= ctx->pool_budget) return cudaSuccess;
+    *moved = true;
     const uint64_t low = ctx->pool_budget / 2;
     uint32_t fullest = 0;
     for (uint32_t d = 1; d < nb; ++d)
@@ -210,6 +237,36 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   for (uint32_t b = 0; b < nb; ++b) maxpool = std::max<uint64_t>(maxpool, ctx->pool_words[b].size());
   GW_CUDA(ctx, ctx->d_words.ensure(maxpool * 8), "word alloc");
   if (ctx->pools_have_ids) GW_CUDA(ctx, ctx->d_ids.ensure(maxpool * 4), "id alloc");
+  // Mapped pinned memory the host and a superstep's kernels share, reached by
+  // the device at its mapped address, so the small transfers of a superstep
+  // never wait behind a block copy on the copy engine: what the scan reports
+  // per block (moved_word), and two copies of the pool table (one for the next
+  // superstep's launch, one for pools grown in the middle of a superstep: each
+  // is read by a kernel the host has waited for before it writes that copy
+  // again).
+  GW_CUDA(ctx, ctx->h_xfer.ensure(9 * (size_t)nb * 8), "pinned scratch");
+  volatile uint64_t* const h_moved = ctx->h_xfer.as<uint64_t>();
+  uint64_t* const h_table = ctx->h_xfer.as<uint64_t>() + nb;
+  void* m_xfer = nullptr;
+  GW_CUDA(ctx, cudaHostGetDevicePointer(&m_xfer, ctx->h_xfer.p, 0), "mapped scratch");
+  uint64_t* const m_moved = static_cast<uint64_t*>(m_xfer);
+  const uint64_t* const m_table = m_moved + nb;
+  std::vector<uint32_t> h_minhop(nb), h_totals(nb);
+  // device: minimum hops (reset by each scan after it has read them), the
+  // pool table, and the superstep clock
+  GW_CUDA(ctx, ctx->d_minhop.ensure((size_t)nb * 4), "minhop alloc");
+  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_minhop.p, 0xff, (size_t)nb * 4, st), "minhop clear");
+  GW_CUDA(ctx, ctx->d_pool_table.ensure(4 * (size_t)nb * 8 + 8 + 4 * 8), "pool table alloc");
+  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_pool_table.p, 0, 4 * (size_t)nb * 8 + 8 + 4 * 8, st), "pool table clear");
+  PoolTable table;
+  table.ptr = ctx->d_pool_table.as<gw_walk_rec*>();
+  table.n = ctx->d_pool_table.as<uint64_t>() + nb;
+  table.cap = table.n + nb;
+  table.place = table.cap + nb;
+  table.full = reinterpret_cast<uint32_t*>(table.place + nb);
+  PartitionScratch ps{};
+  ps.minhop = ctx->d_minhop.as<uint32_t>();
+  ps.clock = reinterpret_cast<unsigned long long*>(table.full + 2);
   for (uint32_t b = 0; b < nb; ++b) {
     const uint64_t m = ctx->pool_words[b].size();
     if (!m) continue;
@@ -224,12 +281,18 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
                                    cudaMemcpyHostToDevice, st), "id upload");
     GW_CUDA(ctx, launch_unpack_words(ctx->d_words.as<uint64_t>(),
                                      ctx->pools_have_ids ? ctx->d_ids.as<uint32_t>() : nullptr, m,
-                                     ctx->blocks[b], ctx->pools[b].as<gw_walk_rec>(), st), "unpack");
-    GW_CUDA(ctx, cudaStreamSynchronize(st), "walk upload");  // host words are reused next block
+                                     ctx->blocks[b], ctx->pools[b].as<gw_walk_rec>(), st, ps.minhop + b), "unpack");
     ctx->pool_size[b] = m;
-    for (uint64_t w : ctx->pool_words[b]) ctx->minstep[b] = std::min<uint32_t>(ctx->minstep[b], gw_get_hop(w));
     walksum += m;
-    GW_CUDA(ctx, spill_to_budget(), "pool spill");
+    bool moved = false;
+    GW_CUDA(ctx, spill_to_budget(&moved), "pool spill");
+  }
+  GW_CUDA(ctx, cudaMemcpyAsync(h_minhop.data(), ps.minhop, (size_t)nb * 4, cudaMemcpyDeviceToHost, st), "minimum hops");
+  GW_CUDA(ctx, cudaMemsetAsync(ps.minhop, 0xff, (size_t)nb * 4, st), "minhop clear");
+  GW_CUDA(ctx, cudaStreamSynchronize(st), "walk upload");
+  for (uint32_t b = 0; b < nb; ++b) {
+    ctx->minstep[b] = std::min<uint32_t>(h_minhop[b], 0xffffu);
+    h_moved[b] = 0;
   }
   const uint64_t nwalks = walksum;
   walksum = 0;  // from here on: walks pending in the owned blocks
@@ -246,44 +309,42 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   sv.counts = ctx->d_counts.as<uint32_t>();
   sv.closure = ctx->d_closure.as<unsigned long long>();
 
-  // ---- partition scratch ----
-  const uint32_t nbk = nb + 1;  // + the "ended" bucket
-  GW_CUDA(ctx, ctx->d_totals.ensure(nbk * 4), "minhop alloc");  // per-bucket minimum hop
-  // cleared once; each superstep's totals kernel resets it after reading it
-  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_totals.p, 0xff, nbk * 4, st), "minhop clear");
-  GW_CUDA(ctx, ctx->d_out_ptr.ensure(nbk * sizeof(void*)), "ptr alloc");
-  GW_CUDA(ctx, ctx->d_out_base.ensure(nbk * 8), "base alloc");
-  gw_hostbuf h_xfer;  // pinned: totals|minhop down, ptr|base up
-  GW_CUDA(ctx, h_xfer.ensure(2 * nbk * 4 + nbk * (sizeof(void*) + 8)), "pinned scratch");
-  uint32_t* h_totals = h_xfer.as<uint32_t>();
-  uint32_t* h_minhop = h_totals + nbk;
-  gw_walk_rec** h_ptr = reinterpret_cast<gw_walk_rec**>(h_totals + 2 * nbk);
-  uint64_t* h_base = reinterpret_cast<uint64_t*>(h_ptr + nbk);
-  // The device reaches h_xfer at its mapped address: the totals kernel writes
-  // totals|minhop there and a fetch kernel reads ptr|base, so the small
-  // transfers of a superstep never wait behind a block copy on the copy engine.
-  void* m_xfer = nullptr;
-  GW_CUDA(ctx, cudaHostGetDevicePointer(&m_xfer, h_xfer.p, 0), "mapped scratch");
-  uint32_t* m_totals = static_cast<uint32_t*>(m_xfer);
-  const uint64_t* m_ptr = reinterpret_cast<const uint64_t*>(m_totals + 2 * nbk);
-  const uint64_t* m_base = m_ptr + nbk;
-
   // ---- streamed block slots ----
-  Slots slots;
+  // One device slot holds the column slice of one block,
+  //   csr[beg_pos[blocks[b]] .. beg_pos[blocks[b+1]]);
+  // the row pointer of every block stays in HBM.
+  auto& slots = ctx->slots;
+  std::vector<uint32_t> slot_block;  // block held, kNoBlock if empty
+  std::vector<int> slot_of;          // per block: slot index or -1
   const uint32_t nslots = streaming ? std::max<uint32_t>(2, std::min(ctx->nmblocks, nb)) : 0;
+  uint64_t max_e = 0;
   if (streaming) {
-    uint64_t max_e = 0;
     const uint64_t* hr = ctx->h_rowptr.as<uint64_t>();
     for (uint32_t b = 0; b < nb; ++b) max_e = std::max<uint64_t>(max_e, hr[ctx->blocks[b + 1]] - hr[ctx->blocks[b]]);
+  }
+  struct SlotRelease {  // large slots go back to the device when the run ends
+    gw_ctx* ctx;
+    bool drop;
+    ~SlotRelease() {
+      if (!drop) return;
+      cudaStreamSynchronize(ctx->copy_stream);
+      cudaStreamSynchronize(ctx->stream);
+      ctx->slots.release();
+    }
+  } slot_release{ctx, streaming && nslots * max_e * 4 > gw_ctx::BlockSlots::kKeptSlotBytes};
+  if (streaming) {
+    slot_block.assign(nslots, kNoBlock);
+    slot_of.assign(nb, -1);
+    if (slots.csr.size() != nslots) slots.release();
     slots.csr.resize(nslots);
-    slots.block.assign(nslots, kNoBlock);
-    slots.ready.resize(nslots);
-    slots.free_ev.resize(nslots);
-    slots.slot_of.assign(nb, -1);
+    while (slots.ready.size() < nslots) {
+      cudaEvent_t ev[2] = {};
+      for (auto& x : ev) GW_CUDA(ctx, cudaEventCreateWithFlags(&x, cudaEventDisableTiming), "slot event");
+      slots.ready.push_back(ev[0]);
+      slots.free_ev.push_back(ev[1]);
+    }
     for (uint32_t i = 0; i < nslots; ++i) {
       GW_CUDA(ctx, slots.csr[i].ensure(std::max<uint64_t>(max_e, 1) * 4), "slot alloc");
-      cudaEventCreateWithFlags(&slots.ready[i], cudaEventDisableTiming);
-      cudaEventCreateWithFlags(&slots.free_ev[i], cudaEventDisableTiming);
       cudaEventRecord(slots.free_ev[i], st);
     }
   }
@@ -312,22 +373,22 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   std::vector<uint32_t> ahead;  // blocks copied ahead of their turn, not yet run
   // findSubGraph: make block b resident in a slot (never the slot `keep`).
   auto load_block = [&](uint32_t b, int keep) -> int {
-    if (slots.slot_of[b] >= 0) return slots.slot_of[b];
+    if (slot_of[b] >= 0) return slot_of[b];
     int victim = -1;
     for (uint32_t i = 0; i < nslots && victim < 0; ++i)
-      if (slots.block[i] == kNoBlock && (int)i != keep) victim = (int)i;
+      if (slot_block[i] == kNoBlock && (int)i != keep) victim = (int)i;
     if (victim < 0) {  // swapOut: resident block with the fewest pending walks
       uint64_t minw = ~0ull;
       for (uint32_t i = 0; i < nslots; ++i) {
         if ((int)i == keep) continue;
-        const uint64_t w = ctx->pool_size[slots.block[i]];
+        const uint64_t w = ctx->pool_size[slot_block[i]];
         if (w < minw) {
           minw = w;
           victim = (int)i;
         }
       }
-      slots.slot_of[slots.block[victim]] = -1;
-      ahead.erase(std::remove(ahead.begin(), ahead.end(), slots.block[victim]), ahead.end());
+      slot_of[slot_block[victim]] = -1;
+      ahead.erase(std::remove(ahead.begin(), ahead.end(), slot_block[victim]), ahead.end());
     }
     const uint64_t* hr = ctx->h_rowptr.as<uint64_t>();
     const uint32_t v0 = ctx->blocks[b], v1 = ctx->blocks[b + 1];
@@ -337,21 +398,19 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
       cudaMemcpyAsync(slots.csr[victim].p, ctx->h_colidx.as<uint32_t>() + e0, (e1 - e0) * 4,
                       cudaMemcpyHostToDevice, xs);
     cudaEventRecord(slots.ready[victim], xs);
-    slots.block[victim] = b;
-    slots.slot_of[b] = victim;
+    slot_block[victim] = b;
+    slot_of[b] = victim;
     ctx->stats.block_loads++;
     ctx->stats.bytes_h2d += (e1 - e0) * 4;
     return victim;
   };
 
-  double ms_walk = 0, ms_partition = 0, ms_copy_wait = 0;
-  // run start/end, and the phases of each superstep in two alternating sets
-  // (a superstep's set is read after the next superstep's synchronisation):
-  // ph[0] before the copy wait, ph[1] walk start, ph[2] walk end, ph[3]
-  // partition end.  Destroyed on every return; so are the pools that grown
-  // pools replaced, once no queued copy reads them.
+  double ms_copy_wait = 0;
+  // run start/end, and a superstep's wait for a block copy.  Destroyed on
+  // every return; so are the pools that grown pools replaced, once no queued
+  // copy reads them.
   struct Events {
-    cudaEvent_t e[10];
+    cudaEvent_t e[4];
     std::vector<void*> retired;
     Events() {
       for (auto& x : e) cudaEventCreate(&x);
@@ -362,16 +421,38 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
     }
   } evs;
   cudaEvent_t t0 = evs.e[0], t1 = evs.e[1];
-  auto phase_set = [&](uint64_t step) { return evs.e + 2 + 4 * (step & 1); };
-  auto add_phases = [&](uint64_t step) {
-    cudaEvent_t* q = phase_set(step);
-    float a = 0.f, w = 0.f, m = 0.f;
-    cudaEventElapsedTime(&a, q[0], q[1]);
-    cudaEventElapsedTime(&w, q[1], q[2]);
-    cudaEventElapsedTime(&m, q[2], q[3]);
-    ms_copy_wait += a;
-    ms_walk += w;
-    ms_partition += m;
+  // The device's pool table from the host's, by a kernel on st: `at` is the
+  // copy in mapped memory (0: before a superstep, 1: pools grown inside one),
+  // `arrived` the walks the queued scatter adds to each pool (NULL: none).
+  auto upload_table = [&](int at, const uint32_t* arrived) {
+    uint64_t* t = h_table + (size_t)at * 4 * nb;
+    for (uint32_t d = 0; d < nb; ++d) {
+      t[d] = reinterpret_cast<uint64_t>(ctx->pools[d].p);
+      t[nb + d] = dev_n(d) + (arrived ? arrived[d] : 0);
+      t[2 * nb + d] = cap[d];
+      t[3 * nb + d] = dev_n(d);
+    }
+    return launch_fetch_pools(m_table + (size_t)at * 4 * nb, table, nb, st);
+  };
+  // Waits for the scan's words of superstep `seq`: the totals and minimum hops
+  // are then on the host, usually while the scatter still runs.
+  auto wait_totals = [&](uint16_t seq) -> cudaError_t {
+    uint32_t d = 0;
+    for (uint32_t spin = 1, idle = 0; d < nb; ++spin) {
+      const uint64_t w = h_moved[d];
+      if ((uint16_t)(w >> 48) == seq) {
+        h_totals[d] = (uint32_t)w;
+        h_minhop[d] = (uint32_t)(w >> 32) & 0xffffu;
+        ++d;
+        continue;
+      }
+      if (spin & 0xfff) continue;
+      const cudaError_t q = cudaStreamQuery(st);  // a failed or finished stream ends the wait
+      if (q == cudaErrorNotReady) cudaGetLastError();  // not an error of a later launch
+      else if (q != cudaSuccess) return q;
+      else if (++idle > 2) return cudaErrorUnknown;
+    }
+    return cudaSuccess;
   };
   cudaEventRecord(t0, st);
   uint64_t superstep = 0;
@@ -379,6 +460,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   // The scatter of superstep k is left queued: the host next waits on the
   // stream for the partition totals of superstep k + 1, which orders it.
   bool pending = false;
+  bool stale = true;  // the device's pool table is behind the host's
   while (walksum > 0 && e == cudaSuccess &&
          (p->max_supersteps == 0 || superstep < p->max_supersteps)) {
     uint32_t b;
@@ -414,12 +496,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
       if (e == cudaSuccess && dn)
         e = cudaMemcpyAsync(static_cast<gw_walk_rec*>(np) + hn, ctx->pools[b].p, dn * sizeof(gw_walk_rec),
                             cudaMemcpyDeviceToDevice, st);
-      if (ctx->pools[b].p) {
-        if (pool_async[b])
-          cudaFreeAsync(ctx->pools[b].p, st);
-        else
-          evs.retired.push_back(ctx->pools[b].p);
-      }
+      retire(b, &evs.retired);
       pool_async[b] = 1;
       ctx->pools[b].p = np;
       ctx->pools[b].bytes = ncap * sizeof(gw_walk_rec);
@@ -428,6 +505,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
       ctx->pool_chunks[b].clear();
       ctx->pool_host_n[b] = 0;
       ctx->stats.pools_refilled++;
+      stale = true;
       if (e != cudaSuccess) break;
     }
     WalkArgs ab = a;
@@ -436,42 +514,53 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
     const unsigned long long* beg_pos = nullptr;
     const uint32_t* csr = nullptr;
     int slot = -1;
-    const PartitionPlan plan = partition_plan(n, nbk);
-    const size_t hist_n = (size_t)plan.nbuckets * plan.ntiles;
-    if (pending && (n * 4 > ctx->d_dest.bytes || hist_n * 4 > ctx->d_tile_hist.bytes ||
-                    hist_n * 4 > ctx->d_tile_off.bytes || plan.scan_temp_bytes > ctx->d_scan_temp.bytes)) {
+    const PartitionPlan plan = partition_plan(n, nb);
+    const size_t hist_bytes = (size_t)nb * plan.ntiles * 4;
+    if (pending && (n * 4 > ctx->d_dest.bytes || hist_bytes > ctx->d_tile_hist.bytes)) {
       // a buffer the queued scatter reads is about to be replaced
       e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) break;
     }
     GW_CUDA(ctx, ctx->d_dest.grow(n * 4), "dest alloc");
-    GW_CUDA(ctx, ctx->d_tile_hist.grow(hist_n * 4), "hist alloc");
-    GW_CUDA(ctx, ctx->d_tile_off.grow(hist_n * 4), "hist alloc");
-    GW_CUDA(ctx, ctx->d_scan_temp.grow(plan.scan_temp_bytes), "scan alloc");
-    cudaEvent_t* ph = phase_set(superstep);
-    cudaEventRecord(ph[0], st);
+    GW_CUDA(ctx, ctx->d_tile_hist.grow(hist_bytes), "hist alloc");
+    ps.dest = ctx->d_dest.as<uint32_t>();
+    ps.tile_hist = ctx->d_tile_hist.as<uint32_t>();
+    if (stale) {
+      e = upload_table(0, nullptr);
+      if (e != cudaSuccess) break;
+      stale = false;
+    }
+    bool waits = false;  // the walk kernel waits for its block's copy
     if (streaming) {
       ahead.erase(std::remove(ahead.begin(), ahead.end(), b), ahead.end());
       beg_pos = ctx->d_rowptr.as<unsigned long long>() + ab.lo;
-      if (slots.slot_of[b] < 0 && n <= mapped_limit(b)) {
+      if (slot_of[b] < 0 && n <= mapped_limit(b)) {
         csr = m_colidx + ctx->h_rowptr.as<uint64_t>()[ab.lo];
         ctx->stats.mapped_supersteps++;
         ctx->stats.mapped_walks += n;
       } else {
         slot = load_block(b, -1);
+        waits = cudaEventQuery(slots.ready[slot]) == cudaErrorNotReady;
+        cudaGetLastError();  // "not ready" is no error of the launches below
+        if (waits) cudaEventRecord(evs.e[2], st);
         cudaStreamWaitEvent(st, slots.ready[slot], 0);
+        if (waits) cudaEventRecord(evs.e[3], st);
         csr = slots.csr[slot].as<uint32_t>();
       }
     }
     // ---- exec_updates ----
-    cudaEventRecord(ph[1], st);
     e = launch_walk_block((int)p->rule, (int)p->sink, p->aggregate != 0, ctx->pools[b].as<gw_walk_rec>(),
-                          n, ctx->view(), beg_pos, csr, ab, sv, ctx->d_blocks.as<uint32_t>(), nb,
-                          ctx->d_dest.as<uint32_t>(), ctx->d_status.as<uint32_t>(), st);
+                          n, ctx->view(), beg_pos, csr, ab, sv, ctx->d_blocks.as<uint32_t>(), plan, ps,
+                          ctx->d_status.as<uint32_t>(), st);
     if (e != cudaSuccess) break;
-    cudaEventRecord(ph[2], st);
+    if (slot >= 0) cudaEventRecord(slots.free_ev[slot], st);
+    // ---- moveWalk: stable partition by destination block ----
+    const uint16_t seq = (uint16_t)(superstep + 1);
+    e = launch_partition_scan(plan, ps, table, b, m_moved, seq, st);
+    if (e == cudaSuccess)
+      e = launch_partition_scatter(ctx->pools[b].as<gw_walk_rec>(), n, plan, ps, table.ptr, table.place, table.full, st);
+    if (e != cudaSuccess) break;
     if (streaming) {
-      if (slot >= 0) cudaEventRecord(slots.free_ev[slot], st);
       // Copy ahead: keep up to kCopyAhead blocks copied before their turn,
       // so the host link stays busy while blocks in slots run.  The candidate
       // is the block in no slot with the most pending walks (more than it
@@ -481,7 +570,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
         uint64_t best = 0;
         uint32_t nxt = kNoBlock;
         for (uint32_t q = 0; q < nb; ++q)
-          if (q != b && slots.slot_of[q] < 0 && ctx->pool_size[q] > best && ctx->pool_size[q] > mapped_limit(q)) {
+          if (q != b && slot_of[q] < 0 && ctx->pool_size[q] > best && ctx->pool_size[q] > mapped_limit(q)) {
             best = ctx->pool_size[q];
             nxt = q;
           }
@@ -490,89 +579,78 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
         uint64_t minw = ~0ull;
         for (uint32_t i = 0; i < nslots; ++i) {
           if ((int)i == slot) continue;
-          if (slots.block[i] == kNoBlock) room = true;
-          else minw = std::min<uint64_t>(minw, ctx->pool_size[slots.block[i]]);
+          if (slot_block[i] == kNoBlock) room = true;
+          else minw = std::min<uint64_t>(minw, ctx->pool_size[slot_block[i]]);
         }
         if (!room && best <= minw) break;
         load_block(nxt, slot);
         ahead.push_back(nxt);
       }
     }
-    // ---- moveWalk: stable partition by destination block ----
-    uint32_t* d_minhop = ctx->d_totals.as<uint32_t>();
-    e = launch_partition_hist(ctx->pools[b].as<gw_walk_rec>(), ctx->d_dest.as<uint32_t>(), n, plan,
-                              ctx->d_tile_hist.as<uint32_t>(), d_minhop, st);
-    if (e == cudaSuccess)
-      e = launch_partition_scan(ctx->d_tile_hist.as<uint32_t>(), ctx->d_tile_off.as<uint32_t>(), m_totals,
-                                plan, ctx->d_scan_temp.p, st, d_minhop, m_totals + nbk);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    e = wait_totals(seq);
     if (e != cudaSuccess) break;
-    if (superstep > 0) add_phases(superstep - 1);
-    // updateWalkNum: grow destination pools, then scatter into them
+    if (waits) {
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, evs.e[2], evs.e[3]);
+      ms_copy_wait += ms;
+    }
+    // updateWalkNum: pools too small for their new walks grow, and the
+    // scatter, which has found the same and done nothing, runs again
+    bool grown = false;
+    ctx->pool_size[b] = 0;
     for (uint32_t d = 0; d < nb; ++d) {
       const uint64_t held = dev_n(d);  // the device part; a host part stays where it is
       const uint64_t need = held + h_totals[d];
-      if (d != b && need > cap[d]) {
-        uint64_t ncap = std::max<uint64_t>(need, cap[d] * 2);
-        ncap = std::max<uint64_t>(ncap, 1024);
-        void* np = nullptr;
-        e = cudaMallocAsync(&np, ncap * sizeof(gw_walk_rec), st);
-        if (e != cudaSuccess) break;
-        if (held)
-          e = cudaMemcpyAsync(np, ctx->pools[d].p, held * sizeof(gw_walk_rec), cudaMemcpyDeviceToDevice, st);
-        if (ctx->pools[d].p) {
-          if (pool_async[d])
-            cudaFreeAsync(ctx->pools[d].p, st);
-          else
-            evs.retired.push_back(ctx->pools[d].p);
-        }
-        pool_async[d] = 1;
-        ctx->pools[d].p = np;
-        ctx->pools[d].bytes = ncap * sizeof(gw_walk_rec);
-        cap[d] = ncap;
-        if (e != cudaSuccess) break;
-      }
-      h_ptr[d] = ctx->pools[d].as<gw_walk_rec>();
-      h_base[d] = dev_n(d);
+      if (need <= cap[d]) continue;
+      grown = true;
+      uint64_t ncap = std::max<uint64_t>({need, cap[d] * 2, 1024});
+      void* np = nullptr;
+      e = cudaMallocAsync(&np, ncap * sizeof(gw_walk_rec), st);
+      if (e != cudaSuccess) break;
+      if (held)
+        e = cudaMemcpyAsync(np, ctx->pools[d].p, held * sizeof(gw_walk_rec), cudaMemcpyDeviceToDevice, st);
+      retire(d, &evs.retired);
+      pool_async[d] = 1;
+      ctx->pools[d].p = np;
+      ctx->pools[d].bytes = ncap * sizeof(gw_walk_rec);
+      cap[d] = ncap;
+      if (e != cudaSuccess) break;
+    }
+    if (e == cudaSuccess && grown) {
+      e = upload_table(1, h_totals.data());
+      if (e == cudaSuccess)
+        e = launch_partition_scatter(ctx->pools[b].as<gw_walk_rec>(), n, plan, ps, table.ptr, table.place, table.full,
+                                     st);
     }
     if (e != cudaSuccess) break;
-    h_ptr[nb] = nullptr;
-    h_base[nb] = 0;
-    e = launch_fetch_u64_pair(m_ptr, ctx->d_out_ptr.as<uint64_t>(), m_base, ctx->d_out_base.as<uint64_t>(),
-                              nbk, st);
-    if (e == cudaSuccess)
-      e = launch_partition_scatter(ctx->pools[b].as<gw_walk_rec>(), ctx->d_dest.as<uint32_t>(), n, plan,
-                                   ctx->d_tile_off.as<uint32_t>(),
-                                   ctx->d_out_ptr.as<gw_walk_rec* const>(),
-                                   ctx->d_out_base.as<uint64_t>(), st);
-    if (e != cudaSuccess) break;
-    cudaEventRecord(ph[3], st);
-    // h_ptr/h_base are rewritten only after the next totals wait, when the
-    // fetch kernel has read them
     pending = true;
     uint64_t forwarded = 0;
     for (uint32_t d = 0; d < nb; ++d) {
       if (!h_totals[d]) continue;
       ctx->pool_size[d] += h_totals[d];
       if (d >= own_lo && d < own_hi) forwarded += h_totals[d];
-      ctx->minstep[d] = std::min<uint32_t>(ctx->minstep[d], std::min<uint32_t>(h_minhop[d], 0xffff));
+      ctx->minstep[d] = std::min<uint32_t>(ctx->minstep[d], h_minhop[d]);
     }
     walksum = walksum - n + forwarded;
-    ctx->pool_size[b] = 0;
     ctx->minstep[b] = 0xffff;
     ++superstep;
-    e = spill_to_budget();
+    e = spill_to_budget(&stale);
   }
   cudaEventRecord(t1, st);
   if (e != cudaSuccess) return ctx->cuda_fail(e, "blocked engine");
+  struct {
+    uint32_t full, unused;
+    unsigned long long clock[4];
+  } last = {};  // the end of the pool table's buffer
+  GW_CUDA(ctx, cudaMemcpyAsync(&last, table.full, sizeof last, cudaMemcpyDeviceToHost, st), "clock read");
   s = take_status(ctx, st);  // synchronises the stream
-  if (superstep > 0) add_phases(superstep - 1);
+  if (s == GW_OK && last.full) s = ctx->fail(GW_E_STATE, "a superstep's walks were left unplaced");
   float ms = 0.f;
   cudaEventElapsedTime(&ms, t0, t1);
   ctx->stats.supersteps = superstep;
   ctx->stats.ms_total = ms;
-  ctx->stats.ms_walk = ms_walk;
-  ctx->stats.ms_partition = ms_partition;
+  ctx->stats.ms_walk = last.clock[2] * 1e-6;  // the device's clock, stamped by the kernels' first CTAs
+  ctx->stats.ms_partition = last.clock[3] * 1e-6;
   ctx->stats.ms_copy_wait = ms_copy_wait;
   ctx->last_nwalks = nwalks;
   ctx->last_sink = p->sink;

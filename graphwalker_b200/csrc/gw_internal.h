@@ -30,19 +30,13 @@ cudaError_t launch_walk_resident(int rule, int sink, bool agg, const gw_walk_rec
                                  const GraphView& g, const WalkArgs& a, const SinkView& s,
                                  uint32_t* status, int grid, cudaStream_t stream,
                                  const cudaAccessPolicyWindow* window = nullptr);
-// Blocked-mode superstep: advances the n walks of one block while they stay
-// inside [a.lo, a.hi); writes them back in place and dest[i] = destination
-// block (nblocks when the walk ended).  beg_pos/csr non-null = block slice.
-cudaError_t launch_walk_block(int rule, int sink, bool agg, gw_walk_rec* walks, uint64_t n,
-                              const GraphView& g, const unsigned long long* beg_pos,
-                              const uint32_t* csr, const WalkArgs& a, const SinkView& s,
-                              const uint32_t* blocks, uint32_t nblocks, uint32_t* dest,
-                              uint32_t* status, cudaStream_t stream);
 int walk_resident_grid(int rule, int sink, bool agg, uint64_t n);
 
 // ---- codec kernels (gw_walk.cu) ----
+// minhop (may be NULL): atomicMin of the walks' lowest hop.
 cudaError_t launch_unpack_words(const uint64_t* words, const uint32_t* ids, uint64_t n,
-                                uint32_t block_base, gw_walk_rec* out, cudaStream_t stream);
+                                uint32_t block_base, gw_walk_rec* out, cudaStream_t stream,
+                                uint32_t* minhop = nullptr);
 // Words of several pools laid end to end: pool p = [pool_offsets[p], pool_offsets[p+1]).
 cudaError_t launch_unpack_pools(const uint64_t* words, const uint32_t* ids, uint64_t first,
                                 uint64_t n, const uint64_t* pool_offsets, const uint32_t* blocks,
@@ -79,42 +73,99 @@ cudaError_t rmat_build_csr(uint32_t scale, uint64_t nedges_raw, uint64_t seed, u
                            uint32_t tab, uint32_t tabc, unsigned long long** rowptr_out,
                            uint32_t** colidx_out, uint64_t* nedges, cudaStream_t stream);
 
-// ---- partition kernels (gw_partition.cu) ----
+// Launches k so that its CTAs may start while the kernel before it on the
+// stream drains (programmatic dependent launch): k must call
+// wait_for_previous() before it touches anything an earlier kernel writes or
+// reads.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                             A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
+// ---- block supersteps: walk + stable partition (gw_walk.cu, gw_partition.cu) ----
+constexpr uint32_t kNoDest = 0xffffffffu;    // dest[] of a walk that ended
+constexpr uint32_t kStagedBlocks = 2048;     // block ranges up to here are searched in shared memory
+constexpr uint32_t kMaxRows = 64;            // rows of a tile: ranks stay below 2^16
+constexpr uint32_t kMaxBuckets = 8000;       // shared memory of the walk kernel: 16 bytes per destination
+
+// The walks of a superstep in tiles of `rows` x kWalkThreads; one CTA walks a tile.
 struct PartitionPlan {
-  uint32_t nbuckets = 0;  // destination blocks + 1 (the "ended" bucket)
+  uint32_t nbuckets = 0;  // destination blocks
   uint32_t ntiles = 0;
-  size_t scan_temp_bytes = 0;
+  uint32_t rows = 1;
+  __host__ __device__ uint32_t tile() const { return rows * kWalkThreads; }
 };
-constexpr int kPartThreads = 256;
-constexpr int kPartItems = 8;  // walks per thread per tile
-constexpr uint32_t kPartTile = kPartThreads * kPartItems;
 PartitionPlan partition_plan(uint64_t n, uint32_t nbuckets);
-// Histogram of dest over tiles (tile_hist[bucket * ntiles + tile]) and the
-// per-bucket minimum hop (atomicMin into minhop[bucket]).
-cudaError_t launch_partition_hist(const gw_walk_rec* walks, const uint32_t* dest, uint64_t n,
-                                  const PartitionPlan& plan, uint32_t* tile_hist,
-                                  uint32_t* minhop, cudaStream_t stream);
-// Exclusive scan of tile_hist (bucket-major) into tile_off, and per-bucket
-// totals; with minhop_src, also moves the nbuckets minimum hops to
-// minhop_dst and resets minhop_src to 0xffffffff for the next histogram
-// (totals and minhop_dst may be mapped pinned host memory, which the host
-// reads after a stream synchronisation, with no copy call).
-cudaError_t launch_partition_scan(const uint32_t* tile_hist, uint32_t* tile_off, uint32_t* totals,
-                                  const PartitionPlan& plan, void* temp, cudaStream_t stream,
-                                  uint32_t* minhop_src = nullptr, uint32_t* minhop_dst = nullptr);
-// dst_a[i] = src_a[i], dst_b[i] = src_b[i] for i < n, by a kernel: the
-// sources may be mapped pinned host memory written by the host before the
-// launch.  Unlike an async host-to-device copy this does not queue behind
-// large block copies on the copy engine.
-cudaError_t launch_fetch_u64_pair(const uint64_t* src_a, uint64_t* dst_a, const uint64_t* src_b,
-                                  uint64_t* dst_b, uint32_t n, cudaStream_t stream);
-// Stable scatter: walk i with dest d lands at out_ptr[d][out_base[d] + rank],
-// rank = position among the walks with dest d in input order.  Bucket
-// nbuckets-1 (ended walks) is not written.
-cudaError_t launch_partition_scatter(const gw_walk_rec* walks, const uint32_t* dest, uint64_t n,
-                                     const PartitionPlan& plan, const uint32_t* tile_off,
-                                     gw_walk_rec* const* out_ptr, const uint64_t* out_base,
-                                     cudaStream_t stream);
+
+// Device arrays a superstep's kernels hand on.
+struct PartitionScratch {
+  uint32_t* dest;       // per walk: destination | rank in the tile << 16, or kNoDest
+  uint32_t* tile_hist;  // [bucket * ntiles + tile]: walk counts, then their exclusive scan per bucket
+  uint32_t* minhop;     // per bucket: lowest hop of the walks that move there (0xffffffff = none)
+  unsigned long long* clock;  // NULL, or device clock: walk start, partition start, ns walking, ns partitioning
+};
+
+// The device pools a superstep's walks move to, one entry per block.  The scan
+// places the new walks behind the n held, advances n and empties the block
+// that ran.  When a pool is too small for its new walks it sets *full: the
+// scatter then does nothing, and the host grows the pools, uploads the table
+// (launch_fetch_pools) and launches the scatter again.
+struct PoolTable {
+  gw_walk_rec** ptr;
+  uint64_t* n;      // records held
+  uint64_t* cap;    // records the pool has room for
+  uint64_t* place;  // where the scatter puts a bucket's first walk
+  uint32_t* full;   // some pool is too small: the scatter does nothing
+};
+
+// What the scan tells the host about a bucket, one 64-bit word in mapped
+// pinned memory written by one store: total | min(minimum hop, 0xffff) << 32 |
+// seq << 48.  The host polls every bucket's word for the superstep's seq, so
+// the scan needs no fence and no last CTA before its kernel can end.
+__host__ __device__ inline uint64_t moved_word(uint32_t total, uint32_t minhop, uint16_t seq) {
+  return total | (uint64_t)(minhop < 0xffffu ? minhop : 0xffffu) << 32 | (uint64_t)seq << 48;
+}
+
+// Blocked-mode superstep: advances the n walks of one block while they stay
+// inside [a.lo, a.hi), writes them back in place, and leaves ps.dest,
+// ps.tile_hist (one column per tile) and ps.minhop.  beg_pos/csr non-null =
+// block slice.
+cudaError_t launch_walk_block(int rule, int sink, bool agg, gw_walk_rec* walks, uint64_t n,
+                              const GraphView& g, const unsigned long long* beg_pos,
+                              const uint32_t* csr, const WalkArgs& a, const SinkView& s,
+                              const uint32_t* blocks, const PartitionPlan& plan, const PartitionScratch& ps,
+                              uint32_t* status, cudaStream_t stream);
+// Exclusive scan of every bucket's tile counts in place.  The totals and the
+// minimum hops (reset for the next superstep) go to totals[b] and
+// minhop_out[b], or, with a pool table, to moved[b] (moved_word), and the
+// buckets are placed in their pools (`block` is the one that ran).
+cudaError_t launch_partition_scan(const PartitionPlan& plan, const PartitionScratch& ps, uint32_t* totals,
+                                  uint32_t* minhop_out, cudaStream_t stream);
+cudaError_t launch_partition_scan(const PartitionPlan& plan, const PartitionScratch& ps, const PoolTable& pools,
+                                  uint32_t block, uint64_t* moved, uint16_t seq, cudaStream_t stream);
+// Copies the host's table (src: nbuckets entries each of ptr, n, cap, place)
+// into `pools` and clears *full, by a kernel: src may be mapped pinned host
+// memory written by the host before the launch.  Unlike an async
+// host-to-device copy this does not queue behind large block copies on the
+// copy engine.
+cudaError_t launch_fetch_pools(const uint64_t* src, const PoolTable& pools, uint32_t nbuckets, cudaStream_t stream);
+// Stable scatter: walk i with destination d and rank r lands at
+// ptr[d][place[d] + tile_hist[d][its tile] + r]; does nothing when *full
+// (full NULL: never).  Ended walks are not written.
+cudaError_t launch_partition_scatter(const gw_walk_rec* walks, uint64_t n, const PartitionPlan& plan,
+                                     const PartitionScratch& ps, gw_walk_rec* const* ptr, const uint64_t* place,
+                                     const uint32_t* full, cudaStream_t stream);
 
 // ---- measurement ----
 cudaError_t launch_gather_probe(const uint32_t* buf, uint64_t n_words, uint64_t loads,

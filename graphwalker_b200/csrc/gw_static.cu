@@ -14,7 +14,7 @@
 // Limits and sharing: the array holds scratch for at most kStaticMaxWalks
 // walks and kStaticMaxBlocks blocks per call (larger requests are rejected
 // with GW_E_INVALID).  Every GPU that loads this library reserves the array
-// (about 12 MiB) until the process exits.  All calls share it and it keeps
+// (about 8 MiB) until the process exits.  All calls share it and it keeps
 // the previous call's contents: this file clears what must start from a known
 // value on every call, and two calls whose work overlaps on the GPU (for
 // instance on two streams without ordering between them) race on the array.
@@ -27,18 +27,17 @@ namespace {
 
 constexpr uint64_t kStaticMaxWalks = 1ull << 20;
 constexpr uint32_t kStaticMaxBlocks = 256;
-constexpr uint32_t kStaticBuckets = kStaticMaxBlocks + 1;        // + "walk ended"
-constexpr uint32_t kStaticWarpTile = kPartTile / (kPartThreads / 32);  // walks per warp tile
-constexpr uint64_t kStaticMaxTiles = kStaticMaxWalks / kStaticWarpTile;
+// tiles of a call, at least 256 walks each
+constexpr uint64_t kStaticMaxTiles = kStaticMaxWalks / kWalkThreads;
 
 constexpr uint64_t align256(uint64_t x) { return (x + 255) & ~255ull; }
 constexpr uint64_t kOffDest = 0;
 constexpr uint64_t kOffHist = align256(kOffDest + kStaticMaxWalks * 4);
-constexpr uint64_t kOffTileOff = align256(kOffHist + kStaticMaxTiles * kStaticBuckets * 4);
-constexpr uint64_t kOffMinhop = align256(kOffTileOff + kStaticMaxTiles * kStaticBuckets * 4);
-constexpr uint64_t kOffPtr = align256(kOffMinhop + kStaticBuckets * 4);
-constexpr uint64_t kOffBase = align256(kOffPtr + kStaticBuckets * 8);
-constexpr uint64_t kStaticBytes = align256(kOffBase + kStaticBuckets * 8);
+constexpr uint64_t kOffMinhop = align256(kOffHist + kStaticMaxTiles * kStaticMaxBlocks * 4);
+constexpr uint64_t kOffTotals = align256(kOffMinhop + kStaticMaxBlocks * 4);
+constexpr uint64_t kOffPtr = align256(kOffTotals + kStaticMaxBlocks * 4);
+constexpr uint64_t kOffPlace = align256(kOffPtr + kStaticMaxBlocks * 8);
+constexpr uint64_t kStaticBytes = align256(kOffPlace + kStaticMaxBlocks * 8);
 
 // The scratch of every gw_superstep_static call on this device.  In host code
 // this name is only a stand-in for the symbol; the device address comes from
@@ -106,59 +105,30 @@ struct DeviceGuard {
   }
 };
 
-// Exclusive scan of the bucket-major tile histogram in one CTA, then the
-// bucket starts: offsets[d] (first moved walk of destination d), and the
-// per-bucket output pointers the partition scatter writes through.  Each warp
-// owns one contiguous segment of the histogram and reads it in rows of 32
-// consecutive entries (coalesced): once to total the segment, and once more,
-// after the segment totals are scanned, to write the offsets.
-constexpr int kScanThreads = 1024;
-constexpr int kScanWarps = kScanThreads / 32;
-
-__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t x, uint32_t lane) {
+// The destinations' starts in d_moved: offsets[d] is the first moved walk of
+// destination d, offsets[nb] the number of walks that moved; one CTA, a
+// destination per thread.
+__global__ void __launch_bounds__(kStaticMaxBlocks)
+    static_place_kernel(const uint32_t* __restrict__ totals, uint32_t nb, gw_walk_rec* moved,
+                        gw_walk_rec** __restrict__ ptr, uint64_t* __restrict__ place,
+                        uint32_t* __restrict__ offsets) {
+  __shared__ uint32_t wsum[kStaticMaxBlocks / 32];
+  const uint32_t d = threadIdx.x, lane = d & 31, warp = d >> 5;
+  const uint32_t c = d < nb ? totals[d] : 0u;
+  uint32_t incl = c;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-    if (lane >= (uint32_t)d) x += y;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(~0u, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
   }
-  return x;
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    static_scan_kernel(const uint32_t* __restrict__ hist, uint32_t* __restrict__ off, uint32_t m,
-                       uint32_t nbuckets, uint32_t ntiles, gw_walk_rec* moved,
-                       gw_walk_rec** __restrict__ out_ptr, uint64_t* __restrict__ out_base,
-                       uint32_t* __restrict__ offsets) {
-  __shared__ uint32_t seg_base[kScanWarps];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t seg = ((m + kScanWarps - 1) / kScanWarps + 31) & ~31u;  // whole rows per warp
-  const uint32_t lo = min(m, warp * seg), hi = min(m, lo + seg);
-  uint32_t part = 0;
-  for (uint32_t i = lo + lane; i < hi; i += 32) part += hist[i];
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
-  if (lane == 0) seg_base[warp] = part;
+  if (lane == 31) wsum[warp] = incl;
   __syncthreads();
-  if (warp == 0) {
-    const uint32_t t = seg_base[lane];
-    const uint32_t incl = warp_inclusive_scan(t, lane);
-    seg_base[lane] = incl - t;
-  }
-  __syncthreads();
-  uint32_t carry = seg_base[warp];
-  for (uint32_t row = lo; row < hi; row += 32) {
-    const uint32_t i = row + lane;
-    const uint32_t h = i < hi ? hist[i] : 0u;
-    const uint32_t incl = warp_inclusive_scan(h, lane);
-    if (i < hi) off[i] = carry + incl - h;
-    carry += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  __syncthreads();
-  for (uint32_t d = threadIdx.x; d < nbuckets; d += kScanThreads) {
-    const uint32_t start = off[(uint64_t)d * ntiles];
-    offsets[d] = start;
-    out_ptr[d] = d + 1 < nbuckets ? moved + start : nullptr;
-    out_base[d] = 0;
+  for (uint32_t w = 0; w < warp; ++w) incl += wsum[w];
+  if (d < nb) {
+    offsets[d] = incl - c;
+    ptr[d] = moved;
+    place[d] = incl - c;
+    if (d + 1 == nb) offsets[nb] = incl;
   }
 }
 
@@ -197,38 +167,29 @@ extern "C" gw_status gw_superstep_static(gw_ctx* ctx, const gw_walk_params* para
   GW_CUDA(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
   unsigned char* base = nullptr;
   GW_CUDA(ctx, static_scratch_address(ctx->device, &base), "cudaGetSymbolAddress(scratch)");
-  uint32_t* dest = reinterpret_cast<uint32_t*>(base + kOffDest);
-  uint32_t* tile_hist = reinterpret_cast<uint32_t*>(base + kOffHist);
-  uint32_t* tile_off = reinterpret_cast<uint32_t*>(base + kOffTileOff);
-  uint32_t* minhop = reinterpret_cast<uint32_t*>(base + kOffMinhop);
-  gw_walk_rec** out_ptr = reinterpret_cast<gw_walk_rec**>(base + kOffPtr);
-  uint64_t* out_base = reinterpret_cast<uint64_t*>(base + kOffBase);
+  PartitionScratch ps{};
+  ps.dest = reinterpret_cast<uint32_t*>(base + kOffDest);
+  ps.tile_hist = reinterpret_cast<uint32_t*>(base + kOffHist);
+  ps.minhop = reinterpret_cast<uint32_t*>(base + kOffMinhop);
+  uint32_t* totals = reinterpret_cast<uint32_t*>(base + kOffTotals);
+  gw_walk_rec** ptr = reinterpret_cast<gw_walk_rec**>(base + kOffPtr);
+  uint64_t* place = reinterpret_cast<uint64_t*>(base + kOffPlace);
 
-  const uint32_t nbk = ctx->nblocks + 1;
-  PartitionPlan plan;
-  plan.nbuckets = nbk;
-  plan.ntiles = (uint32_t)((n + kStaticWarpTile - 1) / kStaticWarpTile);
-  if (plan.ntiles == 0) plan.ntiles = 1;
-  plan.scan_temp_bytes = 0;
-
+  const uint32_t nb = ctx->nblocks;
+  const PartitionPlan plan = partition_plan(n, nb);
   SinkView sv{};
   sv.counts = d_counts;
-  // minhop starts at "no walk": the previous call left its own values there
-  GW_CUDA(ctx, cudaMemsetAsync(minhop, 0xff, nbk * sizeof(uint32_t), st), "clear minhop");
+  // minhop starts at "no walk", whatever an interrupted call left there
+  GW_CUDA(ctx, cudaMemsetAsync(ps.minhop, 0xff, nb * sizeof(uint32_t), st), "clear minhop");
   if (n) {
     GW_CUDA(ctx, launch_walk_block((int)params->rule, (int)params->sink, params->aggregate != 0, d_walks, n,
-                                   ctx->view(), nullptr, nullptr, a, sv, ctx->d_blocks.as<uint32_t>(),
-                                   ctx->nblocks, dest, ctx->d_status.as<uint32_t>(), st),
+                                   ctx->view(), nullptr, nullptr, a, sv, ctx->d_blocks.as<uint32_t>(), plan, ps,
+                                   ctx->d_status.as<uint32_t>(), st),
             "advance");
   }
-  // every (bucket, tile) histogram entry is written, so no clearing is needed
-  GW_CUDA(ctx, launch_partition_hist(d_walks, dest, n, plan, tile_hist, minhop, st), "histogram");
-  static_scan_kernel<<<1, kScanThreads, 0, st>>>(tile_hist, tile_off, plan.nbuckets * plan.ntiles,
-                                                 plan.nbuckets, plan.ntiles, d_moved, out_ptr, out_base,
-                                                 d_offsets);
-  GW_CUDA(ctx, cudaGetLastError(), "scan");
-  GW_CUDA(ctx, launch_partition_scatter(d_walks, dest, n, plan, tile_off, out_ptr, out_base, st), "scatter");
-  GW_CUDA(ctx, cudaMemcpyAsync(d_minhop, minhop, ctx->nblocks * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st),
-          "minhop out");
+  GW_CUDA(ctx, launch_partition_scan(plan, ps, totals, d_minhop, st), "scan");
+  static_place_kernel<<<1, kStaticMaxBlocks, 0, st>>>(totals, nb, d_moved, ptr, place, d_offsets);
+  GW_CUDA(ctx, cudaGetLastError(), "place");
+  GW_CUDA(ctx, launch_partition_scatter(d_walks, n, plan, ps, ptr, place, nullptr, st), "scatter");
   return GW_OK;
 }

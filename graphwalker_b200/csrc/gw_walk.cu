@@ -125,79 +125,157 @@ __device__ __forceinline__ uint32_t find_block(const uint32_t* __restrict__ bloc
   uint32_t lo = 0, hi = nblocks;
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (v < __ldg(blocks + mid + 1)) hi = mid;
+    if (v < blocks[mid + 1]) hi = mid;
     else lo = mid + 1;
   }
   return lo;
 }
 
+__device__ __forceinline__ unsigned long long clock_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
 // Blocked-mode superstep over the walks of block [a.lo, a.hi): the in-block
 // loop of updateByWalk and, on leaving, getblock + moveWalk
-// (randomwalkwithjump.hpp:40-60 and siblings).
+// (randomwalkwithjump.hpp:40-60 and siblings), with the first half of the
+// stable partition by destination block folded in.
+//
+// One CTA owns one tile of plan.tile() consecutive walks, a row of 256 at a
+// time.  After a row's walks have stopped, each walk's rank among the tile's
+// earlier walks of the same destination comes from a warp match, the counts
+// of the lower warps of the row and the running counts of the tile; the walk
+// leaves dest = destination | rank << 16 and the tile leaves one count per
+// destination, so placing the walks needs one scan of the tile counts and one
+// elementwise scatter (gw_partition.cu).
+//
+// A superstep of a few 100,000 walks is bound by latency: the pool record, the
+// vertex record and the column are three dependent loads, and every further
+// launch adds its own start and tail.  A separate histogram pass over the
+// walks (one warp per 256 walks, eight rows in sequence) took 10.4 us beside
+// 9.6 us for the walk itself at 126 k walks and 33 blocks.
 template <int RULE, int SINK, bool AGG, bool SLICE>
 __global__ void __launch_bounds__(kWalkThreads)
     walk_block_kernel(gw_walk_rec* __restrict__ walks, uint64_t n, GraphView g,
                       const unsigned long long* __restrict__ beg_pos,
                       const uint32_t* __restrict__ csr, WalkArgs a, SinkView s,
-                      const uint32_t* __restrict__ blocks, uint32_t nblocks,
-                      uint32_t* __restrict__ dest, uint32_t* __restrict__ status) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+                      const uint32_t* __restrict__ blocks, PartitionPlan plan, PartitionScratch ps,
+                      uint32_t* __restrict__ status) {
+  extern __shared__ uint32_t smem[];
+  const uint32_t nb = plan.nbuckets;
+  uint32_t* const total = smem;       // per destination: walks of the rows done
+  uint32_t* const minhop = smem + nb; // per destination: lowest hop
+  uint32_t* const sblk = smem + 2 * nb;
+  const bool staged = nb <= kStagedBlocks;
+  uint8_t* const wcnt = reinterpret_cast<uint8_t*>(sblk + (staged ? nb + 1 : 0));  // [warp][destination], this row
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint64_t base = (uint64_t)blockIdx.x * plan.tile();
+  let_next_start();
+  if (ps.clock && blockIdx.x == 0 && threadIdx.x == 0) ps.clock[0] = clock_ns();
+  uint64_t i = base + threadIdx.x;
+  uint4 w = make_uint4(0, 0, 0, 0);
+  if (i < n) w = *(reinterpret_cast<const uint4*>(walks) + i);
+  for (uint32_t b = threadIdx.x; b < nb; b += kWalkThreads) {
+    total[b] = 0;
+    minhop[b] = 0xffffffffu;
+  }
+  for (uint32_t b = threadIdx.x; b < nb * (kWalkThreads / 32); b += kWalkThreads) wcnt[b] = 0;
+  if (staged)
+    for (uint32_t b = threadIdx.x; b <= nb; b += kWalkThreads) sblk[b] = __ldg(blocks + b);
+  const uint32_t* const bl = staged ? sblk : blocks;
+  __syncthreads();
   uint32_t st = 0, clos = 0;
   const L2Hints hp = make_hints(a.hints);
   DrawCache dc;
   // the slice's first edge index (csr[0] is edge b0); read once, since the
   // slice may be pinned host memory read over the host link
   const unsigned long long b0 = SLICE && n ? __ldg(beg_pos) : 0ull;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    uint4 w = *(reinterpret_cast<const uint4*>(walks) + i);
-    uint32_t v = w.x, id = w.y, src = w.z, hop = w.w;
-    bool ended = false;
-    dc.reset();
-    while (v >= a.lo && v < a.hi) {
-      if (rule_capped<RULE>() && hop >= a.L) break;
-      if (RULE == GW_RULE_PROB && hop >= a.max_hops) {
-        st |= kStHops;
-        ended = true;
-        break;
-      }
-      if (v >= g.nv) {
-        st |= kStBounds;
-        ended = true;
-        break;
-      }
-      if (SINK == GW_SINK_VERTEX_COUNT) count_visit<AGG>(s.counts, v, hp.cnt);
-      else if (SINK == GW_SINK_CLOSURE_COUNT)
-        clos += ((int)hop >= (int)a.L - 1 && v == src) ? 1u : 0u;
-      if (last_visit<RULE>(a, hop)) {  // its move is never observed: the walk ends here
+  for (uint32_t row = 0;;) {
+    uint32_t d = kNoDest;
+    uint32_t hop = 0;
+    if (i < n) {
+      uint32_t v = w.x;
+      const uint32_t id = w.y, src = w.z;
+      hop = w.w;
+      bool ended = false;
+      dc.reset();
+      while (v >= a.lo && v < a.hi) {
+        if (rule_capped<RULE>() && hop >= a.L) break;
+        if (RULE == GW_RULE_PROB && hop >= a.max_hops) {
+          st |= kStHops;
+          ended = true;
+          break;
+        }
+        if (v >= g.nv) {
+          st |= kStBounds;
+          ended = true;
+          break;
+        }
+        if (SINK == GW_SINK_VERTEX_COUNT) count_visit<AGG>(s.counts, v, hp.cnt);
+        else if (SINK == GW_SINK_CLOSURE_COUNT)
+          clos += ((int)hop >= (int)a.L - 1 && v == src) ? 1u : 0u;
+        if (last_visit<RULE>(a, hop)) {  // its move is never observed: the walk ends here
+          ++hop;
+          ended = true;
+          break;
+        }
+        bool moved;
+        if (SLICE) moved = hop_advance_slice<RULE>(beg_pos, csr, b0, a, id, src, hop, v, dc);
+        else moved = hop_advance<RULE>(g, a, hp, id, src, hop, v, dc);
+        if (!moved) {
+          ended = true;
+          break;
+        }
         ++hop;
-        ended = true;
-        break;
+        if (RULE == GW_RULE_RESTART && hop % a.L == a.L - 1) {
+          ended = true;
+          break;
+        }
       }
-      bool moved;
-      if (SLICE) moved = hop_advance_slice<RULE>(beg_pos, csr, b0, a, id, src, hop, v, dc);
-      else moved = hop_advance<RULE>(g, a, hp, id, src, hop, v, dc);
-      if (!moved) {
-        ended = true;
-        break;
+      if (!ended) {
+        bool alive;
+        if (rule_capped<RULE>()) alive = hop < a.L;
+        else if (RULE == GW_RULE_RESTART) alive = hop % a.L != a.L - 1;
+        else alive = true;
+        if (alive) {
+          const uint32_t to = find_block(bl, nb, v);
+          if (to < nb) d = to;  // v >= N: dropped
+        }
       }
-      ++hop;
-      if (RULE == GW_RULE_RESTART && hop % a.L == a.L - 1) {
-        ended = true;
-        break;
-      }
+      w.x = v;
+      w.w = hop;
+      *(reinterpret_cast<uint4*>(walks) + i) = w;
     }
-    uint32_t d = nblocks;
-    if (!ended) {
-      bool alive;
-      if (rule_capped<RULE>()) alive = hop < a.L;
-      else if (RULE == GW_RULE_RESTART) alive = hop % a.L != a.L - 1;
-      else alive = true;
-      if (alive) d = find_block(blocks, nblocks, v);  // nblocks = dropped (v >= N)
+    // rank among the row's walks of the same destination
+    __syncwarp();
+    const uint32_t peers = __match_any_sync(~0u, d);
+    const uint32_t before = __popc(peers & ((1u << lane) - 1u));
+    const bool leads = d != kNoDest && before == 0;
+    if (leads) wcnt[warp * nb + d] = (uint8_t)__popc(peers);
+    if (d != kNoDest) atomicMin(minhop + d, hop);
+    __syncthreads();
+    if (i < n) {
+      uint32_t rank = before;
+      if (d != kNoDest) {
+        rank += total[d];
+        for (uint32_t x = 0; x < warp; ++x) rank += wcnt[x * nb + d];
+      }
+      ps.dest[i] = d == kNoDest ? kNoDest : d | rank << 16;
     }
-    w.x = v;
-    w.w = hop;
-    *(reinterpret_cast<uint4*>(walks) + i) = w;
-    dest[i] = d;
+    __syncthreads();
+    if (leads) {
+      atomicAdd(total + d, (uint32_t)__popc(peers));
+      wcnt[warp * nb + d] = 0;
+    }
+    if (++row == plan.rows || base + (uint64_t)row * kWalkThreads >= n) break;
+    i += kWalkThreads;
+    if (i < n) w = *(reinterpret_cast<const uint4*>(walks) + i);
+  }
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < nb; b += kWalkThreads) {
+    ps.tile_hist[(uint64_t)b * plan.ntiles + blockIdx.x] = total[b];
+    if (total[b]) atomicMin(ps.minhop + b, minhop[b]);
   }
   if (st) atomicOr(status, st);
   if (SINK == GW_SINK_CLOSURE_COUNT && clos) atomicAdd(s.closure, (unsigned long long)clos);
@@ -205,7 +283,9 @@ __global__ void __launch_bounds__(kWalkThreads)
 
 __global__ void unpack_words_kernel(const uint64_t* __restrict__ words,
                                     const uint32_t* __restrict__ ids, uint64_t n,
-                                    uint32_t block_base, gw_walk_rec* __restrict__ out) {
+                                    uint32_t block_base, gw_walk_rec* __restrict__ out,
+                                    uint32_t* __restrict__ minhop) {
+  uint32_t low = 0xffffffffu;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t wd = words[i];
@@ -215,7 +295,12 @@ __global__ void unpack_words_kernel(const uint64_t* __restrict__ words,
     r.y = ids ? ids[i] : src;
     r.z = src;
     r.w = (uint32_t)(wd & 0x3fffu);
+    low = min(low, r.w);
     *(reinterpret_cast<uint4*>(out) + i) = r;
+  }
+  if (minhop) {  // the lowest hop of the block's walks (the launch's threads are whole warps)
+    low = __reduce_min_sync(~0u, low);
+    if ((threadIdx.x & 31) == 0 && low != 0xffffffffu) atomicMin(minhop, low);
   }
 }
 
@@ -359,17 +444,16 @@ template <int RULE, int SINK, bool AGG>
 cudaError_t block_dispatch(gw_walk_rec* walks, uint64_t n, const GraphView& g,
                            const unsigned long long* beg_pos, const uint32_t* csr,
                            const WalkArgs& a, const SinkView& s, const uint32_t* blocks,
-                           uint32_t nblocks, uint32_t* dest, uint32_t* status,
+                           const PartitionPlan& plan, const PartitionScratch& ps, uint32_t* status,
                            cudaStream_t stream) {
-  if (beg_pos) {
-    auto k = walk_block_kernel<RULE, SINK, AGG, true>;
-    k<<<occupancy_grid(k, n), kWalkThreads, 0, stream>>>(walks, n, g, beg_pos, csr, a, s, blocks,
-                                                        nblocks, dest, status);
-  } else {
-    auto k = walk_block_kernel<RULE, SINK, AGG, false>;
-    k<<<occupancy_grid(k, n), kWalkThreads, 0, stream>>>(walks, n, g, beg_pos, csr, a, s, blocks,
-                                                        nblocks, dest, status);
+  auto k = beg_pos ? walk_block_kernel<RULE, SINK, AGG, true> : walk_block_kernel<RULE, SINK, AGG, false>;
+  const size_t nb = plan.nbuckets;
+  const size_t smem = nb * (8 + kWalkThreads / 32) + (nb <= kStagedBlocks ? (nb + 1) * 4 : 0);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
   }
+  k<<<plan.ntiles, kWalkThreads, smem, stream>>>(walks, n, g, beg_pos, csr, a, s, blocks, plan, ps, status);
   return cudaGetLastError();
 }
 
@@ -411,12 +495,11 @@ int walk_resident_grid(int rule, int sink, bool agg, uint64_t n) {
 cudaError_t launch_walk_block(int rule, int sink, bool agg, gw_walk_rec* walks, uint64_t n,
                               const GraphView& g, const unsigned long long* beg_pos,
                               const uint32_t* csr, const WalkArgs& a, const SinkView& s,
-                              const uint32_t* blocks, uint32_t nblocks, uint32_t* dest,
+                              const uint32_t* blocks, const PartitionPlan& plan, const PartitionScratch& ps,
                               uint32_t* status, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   if (sink == GW_SINK_PATH_RECORD) return cudaErrorInvalidValue;
-  GW_RULE_CASES(block_dispatch, walks, n, g, beg_pos, csr, a, s, blocks, nblocks, dest, status,
-                stream)
+  GW_RULE_CASES(block_dispatch, walks, n, g, beg_pos, csr, a, s, blocks, plan, ps, status, stream)
   return cudaErrorInvalidValue;
 }
 
@@ -427,9 +510,9 @@ static int elementwise_grid(uint64_t n) {
 }
 
 cudaError_t launch_unpack_words(const uint64_t* words, const uint32_t* ids, uint64_t n,
-                                uint32_t block_base, gw_walk_rec* out, cudaStream_t stream) {
+                                uint32_t block_base, gw_walk_rec* out, cudaStream_t stream, uint32_t* minhop) {
   if (n == 0) return cudaSuccess;
-  unpack_words_kernel<<<elementwise_grid(n), 256, 0, stream>>>(words, ids, n, block_base, out);
+  unpack_words_kernel<<<elementwise_grid(n), 256, 0, stream>>>(words, ids, n, block_base, out, minhop);
   return cudaGetLastError();
 }
 

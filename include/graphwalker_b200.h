@@ -404,7 +404,7 @@ gw_status gw_simrank_batch(gw_ctx *ctx, const gw_walk_params *params, const uint
    order, group d starting at d_offsets[d] (nblocks + 1 entries, the last =
    walks moved); d_minhop[d] = lowest hop moved into block d (0xffffffff if
    none).  All scratch comes from one fixed device array of the library
-   (about 12 MiB per GPU that loads it, held until exit): at most 1,048,576
+   (about 8 MiB per GPU that loads it, held until exit): at most 1,048,576
    walks and 256 blocks per call, else GW_E_INVALID.  The first call on a
    device (and the first after that device's context was recreated, e.g. by
    cudaDeviceReset) looks up that array's address, so make it before any
