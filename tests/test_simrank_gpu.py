@@ -109,3 +109,41 @@ def test_simrank_batch_matches_oracle(cuda_device, oracle):
         assert np.array_equal(meet[q], ref_meet), q
         assert scores[q] == pytest.approx(gw.simrank_estimate(ref_meet, R), rel=1e-12)
     assert np.all(meet[:5, 0] >= R)  # every walk meets itself at its source
+
+
+@pytest.mark.parametrize("R,L,vertices", [(511, 520, 5000), (512, 513, 3), (3650, 11, 5000), (4097, 9, 1),
+                                          (2049, 40, 900), (2020, 33, 100_000)])
+def test_meet_counts_at_join_tile_edges(cuda_device, oracle, R, L, vertices):
+    """Past 2^27 comparisons the walks are joined, in tiles of 256 here (one
+    query) and of 512 below: one short of and exactly a tile, one past, rows of
+    one to 44 staged pieces of 12 positions; sparse meetings, long chains and
+    every pair meeting at once; vertex ids that share few hash slots."""
+    assert R * R * L >= 1 << 27
+    g = load_golden("hand")
+    rng = np.random.default_rng(R + L)
+    ids = (np.arange(vertices, dtype=np.uint64) * (1 << 21) % 0xFFFFFFFB).astype(np.uint32)
+    pa, pb = ids[rng.integers(0, vertices, (R, L))], ids[rng.integers(0, vertices, (R, L))]
+    pa[rng.random((R, L)) < 0.05] = 0xFFFFFFFF
+    _, ref_meet = oracle.simrank(pa, pb, R, L)
+    with _graph(g) as G:
+        assert np.array_equal(G.simrank_meet(_dev(pa), _dev(pb), R, L), ref_meet)
+
+
+@pytest.mark.parametrize("nq,R", [(300, 513), (80, 512)])
+def test_simrank_batch_joined_in_both_tiles(cuda_device, oracle, nq, R):
+    """Batches past the comparison limit: 592 tiles of 512 walks or more, and
+    fewer (tiles of 256).  Counts equal the oracle's."""
+    import graphwalker_b200 as gw
+    rp, ci = oracle.rmat_csr(12, 8, seed=4)
+    L, rng = 8, np.random.default_rng(nq)
+    assert nq * R * R * L >= 1 << 27 and (nq * (-(-R // 512)) ** 2 >= 592) == (nq == 300)
+    a, b = rng.integers(0, len(rp) - 1, (2, nq)).astype(np.uint32)
+    b[:3] = a[:3]
+    with gw.Graph.from_csr(rp, ci, oracle.compute_blocks(rp, 64)) as G:
+        _, meet = G.simrank_batch(a, b, R, L, seed=9)
+    for q in range(0, nq, 7):
+        pa, pb = (oracle.run_walks(rp, ci, np.full(R, v, np.uint32), ids=np.full(R, v, np.uint32),
+                                   src=np.full(R, v, np.uint32), hop0=(np.arange(R) * L).astype(np.uint32), rule=3, L=L,
+                                   seed=9, stride=L, counts=False)["paths"] for v in (int(a[q]), int(b[q])))
+        _, ref_meet = oracle.simrank(pa, pb, R, L)
+        assert np.array_equal(meet[q], ref_meet), q
