@@ -11,7 +11,18 @@
 // rules, L-1 per restart segment, until the mass vanishes for the uncapped
 // rule).  The neighbour choice is taken as exactly uniform; the walks'
 // r % deg has a bias below deg / 2^31.
-#include <vector>
+//
+// A hop is two kernels.  The vertex kernel finishes x (the pushes plus what the
+// last hop's else-branches owe the source and all vertices), adds it to the
+// visits, leaves each vertex's share per out-edge and sums the new debts.  The
+// edge kernel adds the shares at the targets: warps take equal runs of edges,
+// whatever their sources' degrees, so no warp is left with a hub: 154 us a hop
+// for 16.8 M edges at R-MAT scale 20, where a warp per vertex took 355.  What
+// bounds it is the L2's FP64 atomic rate, 109 G updates/s (32-bit ones: 190).
+// It is not the hottest target's address: pushes spread over 2 or 4 copies of
+// the targets gained 5 % and lost 11 %, and at scale 22, where the copies
+// outgrow the L2, cost 1.3 and 2.1 times.
+#include <algorithm>
 
 #include "gw_ctx.h"
 
@@ -19,54 +30,123 @@ namespace gw {
 namespace {
 
 constexpr int kExactThreads = 256;
+constexpr int kSums = 4;  // debt sets: the last hop's, this one's, and one cleared ahead
 
-// one warp per vertex: lanes stride over its out-edges
+struct Debt {
+  double to_src, to_uniform, mass;
+};
+
+__device__ __forceinline__ double block_sum(double v, double* warp_sums) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kExactThreads / 32; ++w) v += warp_sums[w];
+  __syncthreads();
+  return v;  // in thread 0
+}
+
+// x (in acc) of this hop; acc is left zero for the edge kernel's pushes.
 __global__ void __launch_bounds__(kExactThreads)
-    exact_hop_kernel(const double* __restrict__ x, double* __restrict__ y, double* __restrict__ visits,
-                     double* __restrict__ sums, GraphView g, double q, int rule, bool capped_jump_to_src) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    exact_vertex_kernel(double* __restrict__ acc, double* __restrict__ share, double* __restrict__ visits,
+                        Debt* __restrict__ debts, uint32_t hop, const unsigned long long* __restrict__ rowptr,
+                        uint32_t nv, uint32_t src, uint32_t njump, double q, int rule) {
+  __shared__ double warp_sums[kExactThreads / 32];
+  const Debt last = debts[(hop + kSums - 1) % kSums];  // zero before the first hop
+  if (blockIdx.x == 0 && threadIdx.x == 0) debts[(hop + 1) % kSums] = Debt{0.0, 0.0, 0.0};
+  const double uniform = last.to_uniform / (double)njump;
   double to_src = 0.0, to_uniform = 0.0, mass = 0.0;
-  for (uint64_t v = warp; v < g.nv; v += nwarps) {
-    const double xv = x[v];
-    if (xv == 0.0) continue;
-    if (lane == 0) {
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x) {
+    double add = v < njump ? uniform : 0.0;
+    if (v == src) add += last.to_src;
+    const double xv = acc[v] + add;
+    double sh = 0.0;
+    if (xv != 0.0) {
+      const unsigned long long deg = rowptr[v + 1] - rowptr[v];
       visits[v] += xv;
       mass += xv;
-    }
-    const unsigned long long b = g.rowptr[v], deg = g.rowptr[v + 1] - b;
-    double fail;
-    if (deg > 0) {
-      const double share = xv * q / (double)deg;
-      for (unsigned long long e = lane; e < deg; e += 32) atomicAdd(y + g.colidx[b + e], share);
-      fail = xv * (1.0 - q);
-    } else {
-      fail = xv;
-    }
-    if (lane == 0) {
-      if (rule == GW_RULE_RESTART) to_src += fail;
-      else if (rule == GW_RULE_PPR && deg == 0) to_src += fail;
+      double fail = xv;
+      if (deg > 0) {
+        sh = xv * q / (double)deg;
+        fail = xv * (1.0 - q);
+      }
+      if (rule == GW_RULE_RESTART || (rule == GW_RULE_PPR && deg == 0)) to_src += fail;
       else if (rule == GW_RULE_JUMP) to_uniform += fail;
     }
+    share[v] = sh;
+    acc[v] = 0.0;
   }
-  (void)capped_jump_to_src;
-  if (lane == 0) {
-    if (to_src != 0.0) atomicAdd(sums + 0, to_src);
-    if (to_uniform != 0.0) atomicAdd(sums + 1, to_uniform);
-    if (mass != 0.0) atomicAdd(sums + 2, mass);
+  to_src = block_sum(to_src, warp_sums);
+  to_uniform = block_sum(to_uniform, warp_sums);
+  mass = block_sum(mass, warp_sums);
+  if (threadIdx.x == 0) {
+    Debt* d = debts + hop % kSums;
+    if (to_src != 0.0) atomicAdd(&d->to_src, to_src);
+    if (to_uniform != 0.0) atomicAdd(&d->to_uniform, to_uniform);
+    if (mass != 0.0) atomicAdd(&d->mass, mass);
   }
 }
 
-// y[src] += to_src; y[v] += to_uniform / njump for v < njump; x := 0
-__global__ void exact_fold_kernel(double* __restrict__ y, double* __restrict__ x, const double* __restrict__ sums,
-                                  uint32_t nv, uint32_t src, uint32_t njump) {
-  const double u = sums[1] / (double)njump;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x) {
-    double add = (v < njump) ? u : 0.0;
-    if (v == src) add += sums[0];
-    if (add != 0.0) y[v] += add;
-    x[v] = 0.0;
+// first[c]: the source of edge c * run (the last vertex whose row starts at or
+// before it and is not empty).
+__global__ void exact_runs_kernel(const unsigned long long* __restrict__ rowptr, uint32_t nv, uint64_t nruns,
+                                  uint32_t run, uint32_t* __restrict__ first) {
+  for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nruns; c += (uint64_t)gridDim.x * blockDim.x) {
+    const unsigned long long e = c * run;
+    uint32_t lo = 0, hi = nv;  // first v with rowptr[v + 1] > e
+    while (lo < hi) {
+      const uint32_t mid = lo + (hi - lo) / 2;
+      if (rowptr[mid + 1] > e) hi = mid;
+      else lo = mid + 1;
+    }
+    first[c] = lo;
+  }
+}
+
+// One warp per run of edges.  The lanes hold the row ends and shares of 32
+// consecutive vertices; a lane finds its edge's source among them by bisection.
+__global__ void __launch_bounds__(kExactThreads)
+    exact_edge_kernel(const double* __restrict__ share, double* __restrict__ acc,
+                      const unsigned long long* __restrict__ rowptr, const uint32_t* __restrict__ colidx, uint32_t nv,
+                      uint64_t ne, uint64_t nruns, uint32_t run, const uint32_t* __restrict__ first) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nruns) return;
+  const uint64_t e0 = c * run;
+  const uint32_t n = (uint32_t)(ne - e0 < run ? ne - e0 : run);  // positions below are relative to e0
+  uint32_t v = __ldg(first + c);
+  for (uint32_t done = 0; done < n; v += 32) {
+    const uint32_t mine = v + lane;
+    uint32_t end = n;  // of vertex `mine`, at most n
+    double sh = 0.0;
+    if (mine < nv) {
+      const unsigned long long x = __ldg(rowptr + mine + 1) - e0;
+      end = x < n ? (uint32_t)x : n;
+      sh = __ldg(share + mine);
+    }
+    const uint32_t last = __shfl_sync(~0u, end, 31);  // edges these vertices reach to
+    const bool any = __any_sync(~0u, sh != 0.0);
+    for (; any && done < last; done += 128) {
+      uint32_t to[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t e = done + u * 32 + lane;
+        to[u] = e < last ? __ldg(colidx + e0 + e) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t e = done + u * 32 + lane;
+        uint32_t at = 0;  // lanes whose row ends at or before e
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(~0u, end, at + step - 1) <= e) at += step;
+        const double s = __shfl_sync(~0u, sh, at);
+        if (e < last && s != 0.0) atomicAdd(acc + to[u], s);
+      }
+    }
+    done = last;
   }
 }
 
@@ -87,39 +167,60 @@ extern "C" gw_status gw_expected_visits(gw_ctx* ctx, const gw_walk_params* param
   else if (rule == GW_RULE_PROB) hops = a.max_hops;
   else hops = params->L;
   const size_t nv = ctx->nv;
-  gw_devbuf bx, by, bvis, bsum;
-  GW_CUDA(ctx, bx.ensure(nv * 8), "alloc");
-  GW_CUDA(ctx, by.ensure(nv * 8), "alloc");
-  GW_CUDA(ctx, bvis.ensure(nv * 8), "alloc");
-  GW_CUDA(ctx, bsum.ensure(3 * 8), "alloc");
+  GW_CUDA(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  // Edges per warp: enough warps to fill the SMs, at most 1024 edges each.
+  const uint64_t ne = ctx->ne;
+  const uint32_t run = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(ne / ((uint64_t)sms * 64) / 128 * 128, 128), 1024);
+  const uint64_t nruns = (ne + run - 1) / run;
+  // One workspace: pushes, shares and visits (8 bytes a vertex each), the debt
+  // sets, and the runs' first vertices.  Kept in the context while it is small.
+  constexpr size_t kKeptBytes = 256ull << 20;
+  const size_t debts_at = 3 * nv * 8, first_at = debts_at + gw::kSums * sizeof(gw::Debt);
+  const size_t bytes = first_at + nruns * 4;
+  GW_CUDA(ctx, ctx->d_exact.ensure(bytes), "alloc");
+  struct Release {
+    gw_ctx* ctx;
+    ~Release() {
+      if (ctx->d_exact.bytes > kKeptBytes) ctx->d_exact.release();
+    }
+  } release{ctx};
   cudaStream_t st = ctx->stream;
-  double* x = bx.as<double>();
-  double* y = by.as<double>();
-  GW_CUDA(ctx, cudaMemsetAsync(x, 0, nv * 8, st), "clear");
-  GW_CUDA(ctx, cudaMemsetAsync(y, 0, nv * 8, st), "clear");
-  GW_CUDA(ctx, cudaMemsetAsync(bvis.p, 0, nv * 8, st), "clear");
+  double* acc = ctx->d_exact.as<double>();
+  double *share = acc + nv, *visits = share + nv;
+  gw::Debt* debts = reinterpret_cast<gw::Debt*>(ctx->d_exact.as<char>() + debts_at);
+  uint32_t* first = reinterpret_cast<uint32_t*>(ctx->d_exact.as<char>() + first_at);
+  GW_CUDA(ctx, cudaMemsetAsync(acc, 0, nv * 8, st), "clear");
+  GW_CUDA(ctx, cudaMemsetAsync(visits, 0, nv * 8 + gw::kSums * sizeof(gw::Debt), st), "clear");  // and the debts
   const double one = 1.0;
-  GW_CUDA(ctx, cudaMemcpyAsync(x + source, &one, 8, cudaMemcpyHostToDevice, st), "seed");
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = sms * 8;
-  double sums[3];
+  GW_CUDA(ctx, cudaMemcpyAsync(acc + source, &one, 8, cudaMemcpyHostToDevice, st), "seed");
+  const unsigned long long* rowptr = ctx->d_rowptr.as<unsigned long long>();
+  if (nruns) {
+    gw::exact_runs_kernel<<<(unsigned)std::min<uint64_t>((nruns + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(
+        rowptr, ctx->nv, nruns, run, first);
+    GW_CUDA(ctx, cudaGetLastError(), "edge runs");
+  }
+  const unsigned vgrid = (unsigned)std::min<uint64_t>((nv + gw::kExactThreads - 1) / gw::kExactThreads, (uint64_t)sms * 8);
+  const unsigned egrid = (unsigned)((nruns * 32 + gw::kExactThreads - 1) / gw::kExactThreads);
   for (uint32_t h = 0; h < hops; ++h) {
-    GW_CUDA(ctx, cudaMemsetAsync(bsum.p, 0, 3 * 8, st), "clear");
-    gw::exact_hop_kernel<<<grid, gw::kExactThreads, 0, st>>>(x, y, bvis.as<double>(), bsum.as<double>(), ctx->view(),
-                                                             q, rule, false);
-    GW_CUDA(ctx, cudaGetLastError(), "exact hop");
-    gw::exact_fold_kernel<<<grid, 256, 0, st>>>(y, x, bsum.as<double>(), ctx->nv, source, a.njump);
-    GW_CUDA(ctx, cudaGetLastError(), "exact fold");
-    std::swap(x, y);
+    gw::exact_vertex_kernel<<<vgrid, gw::kExactThreads, 0, st>>>(acc, share, visits, debts, h, rowptr, ctx->nv, source,
+                                                                 a.njump, q, rule);
+    GW_CUDA(ctx, cudaGetLastError(), "exact vertices");
+    if (h + 1 == hops) break;  // the last hop's moves are not visited
+    if (nruns) {
+      gw::exact_edge_kernel<<<egrid, gw::kExactThreads, 0, st>>>(share, acc, rowptr, ctx->d_colidx.as<uint32_t>(),
+                                                                 ctx->nv, ne, nruns, run, first);
+      GW_CUDA(ctx, cudaGetLastError(), "exact edges");
+    }
     if (rule == GW_RULE_PROB && (h & 15) == 15) {  // the uncapped rule stops when the mass is gone
-      GW_CUDA(ctx, cudaMemcpyAsync(sums, bsum.p, 3 * 8, cudaMemcpyDeviceToHost, st), "mass");
+      double mass = 0.0;
+      GW_CUDA(ctx, cudaMemcpyAsync(&mass, &debts[h % gw::kSums].mass, 8, cudaMemcpyDeviceToHost, st), "mass");
       GW_CUDA(ctx, cudaStreamSynchronize(st), "sync");
-      if (sums[2] < 1e-16) break;
+      if (mass < 1e-16) break;
     }
   }
-  GW_CUDA(ctx, cudaMemcpyAsync(out, bvis.p, nv * 8, cudaMemcpyDeviceToHost, st), "visits out");
+  GW_CUDA(ctx, cudaMemcpyAsync(out, visits, nv * 8, cudaMemcpyDeviceToHost, st), "visits out");
   GW_CUDA(ctx, cudaStreamSynchronize(st), "sync");
   return GW_OK;
 }

@@ -185,3 +185,31 @@ def test_expected_visits_kernel_matches_fp64_oracle(cuda_device, oracle, rule, L
         got = G.expected_visits(gw.params(rule, gw.SINK_NONE, L), src)
     ref = oracle.expected_visits(rp, ci, src, rule, L)
     assert np.allclose(got, ref, rtol=1e-9, atol=1e-13)
+
+
+@pytest.mark.parametrize("edges", ["none", "one", "hub", "runs"])
+@pytest.mark.parametrize("rule,L", [(0, 6), (1, 1), (3, 7), (4, 9)])
+def test_expected_visits_edge_runs(cuda_device, oracle, edges, rule, L):
+    """The edge kernel's runs at their edges: no edges at all, one edge, a hub
+    whose row fills many runs between long stretches of empty rows, and rows of
+    127, 128 and 129 edges.  All terms are positive, so the relative error of a
+    sum of k of them is below k times 2^-53; k is at most every edge and every
+    vertex, in each of L hops."""
+    import graphwalker_b200 as gw
+    nv, r = 2000, np.random.default_rng(3)
+    deg = np.zeros(nv, np.int64)
+    if edges == "one":
+        deg[700] = 1
+    elif edges == "hub":
+        deg[700], deg[1500], deg[nv - 1] = 50_001, 3, 7
+    elif edges == "runs":
+        deg[700:1300:2] = r.choice([127, 128, 129], 300)
+    rp = np.r_[0, np.cumsum(deg)].astype(np.uint64)
+    ci = r.integers(0, nv, int(rp[-1])).astype(np.uint32)
+    ci[:: max(1, len(ci) // 8)] = 700  # some walks come back to a vertex with edges
+    with gw.Graph.from_csr(rp, ci, np.array([0, nv], np.uint32)) as G:
+        for src in (700, 701):
+            for _ in range(2):  # again, in the workspace the first call left
+                got = G.expected_visits(gw.params(rule, gw.SINK_NONE, L), src)
+            ref = oracle.expected_visits(rp, ci, src, rule, L)
+            assert np.allclose(got, ref, rtol=L * (len(ci) + nv) * 2.0 ** -53, atol=0), (src, np.abs(got - ref).max())
