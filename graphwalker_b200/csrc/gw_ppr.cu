@@ -18,12 +18,14 @@
 // of consecutive batch positions from a global cursor, so the walks in flight
 // belong to a narrow window of queries whose tables stay in L2.
 //
-// Top-k: a CTA scans a table (or a segment of one) and keeps a candidate
-// buffer of keys (count << 32 | ~vertex): whenever the buffer could overflow
-// it is sorted and cut to the best k, and the k-th key becomes the admission
+// Top-k: a CTA ranks a table (or a segment of one) by keys count << 32 |
+// ~vertex.  Up to a few thousand slots it holds them in registers and selects
+// by radix; more stream through a candidate buffer: whenever the buffer could
+// overflow it is cut to the best k, and the k-th key becomes the admission
 // threshold.  Large tables are split into segments ranked by separate CTAs,
-// whose lists a second kernel merges.  The result is the exact top k by
-// count, ties broken by the smaller vertex id.
+// whose lists a second kernel (or, for a few queries, each query's last CTA)
+// merges.  The result is the exact top k by count, ties broken by the smaller
+// vertex id.
 #include "gw_ppr.h"
 
 namespace gw {
@@ -277,27 +279,6 @@ __global__ void __launch_bounds__(kPprThreads)
   }
 }
 
-// Sorts keys[0, n) in shared memory, largest first (bitonic; n a power of two).
-__device__ void block_sort_desc(unsigned long long* keys, uint32_t n) {
-  for (uint32_t size = 2; size <= n; size <<= 1) {
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      __syncthreads();
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t partner = i ^ stride;
-        if (partner > i) {
-          const bool desc = (i & size) == 0;
-          const unsigned long long x = keys[i], y = keys[partner];
-          if (desc ? x < y : x > y) {
-            keys[i] = y;
-            keys[partner] = x;
-          }
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-
 // Cuts cand[0, nc) (distinct nonzero keys, nc > k) to its k largest, in any
 // order, at cand[0, *kept), and returns the smallest of them.  The k-th
 // largest key is found by an MSB-first radix select on 8-bit digits (a
@@ -382,15 +363,15 @@ __device__ unsigned long long cut_to_k(unsigned long long* cand, uint32_t nc, ui
   return t;
 }
 
-// The best k keys of n (key i = src.key(src.fetch(i)); 0 = no key) into
-// cand[0, k), largest first.  kTopkUnroll values per thread are fetched
+// The best k keys of n (key i = src.key(src.fetch(i)); 0 = no key) into cand,
+// in any order; returns how many there are.  kTopkUnroll values per thread are fetched
 // before any is converted (the loads issue back to back, so a large table is
 // read with that many loads in flight per thread), then filtered one step of
 // blockDim.x keys at a time into the candidate buffer; whenever the buffer
 // could overflow it is cut to the best k (cut_to_k), and the k-th key
-// becomes the admission threshold.  Only the final k are sorted.
+// becomes the admission threshold.
 template <typename Src>
-__device__ void block_best(Src src, uint32_t n, uint32_t k, unsigned long long* cand, uint32_t& ncand,
+__device__ uint32_t block_best(Src src, uint32_t n, uint32_t k, unsigned long long* cand, uint32_t& ncand,
                            unsigned long long& thresh) {
   if (threadIdx.x == 0) {
     ncand = 0;
@@ -432,10 +413,145 @@ __device__ void block_best(Src src, uint32_t n, uint32_t k, unsigned long long* 
     cut_to_k(cand, nc, k, &kept);
     nc = kept;
   }
-  uint32_t m = 1;
-  while (m < k) m <<= 1;
-  for (uint32_t x = nc + threadIdx.x; x < m; x += blockDim.x) cand[x] = 0;
-  block_sort_desc(cand, m);
+  return nc;
+}
+
+// The best k keys of n <= U * THREADS into cand (at least k entries), in any
+// order; returns how many there are.  Every thread holds U keys in registers
+// and the k-th largest is found by an MSB-first radix select over them, on
+// 11-bit digits of the bits in which the keys differ (equal bits, such as the
+// high bits of the counts and of the complemented vertex ids, cost no pass),
+// which stops when the wanted keys fill their bucket.  Three barriers per
+// digit, whatever n is, where block_best pays one for every blockDim.x keys
+// and three per 8-bit digit of each cut.
+struct SelectSmem {
+  uint32_t hist[2][kSelectBins];  // one digit's counts, and the next one's, cleared meanwhile
+  unsigned long long differ_or, differ_and;
+  uint32_t warp_sum[32];
+  uint32_t sel[3];  // chosen digit, rank left inside it, keys in its bucket
+  uint32_t kept;
+};
+
+// Inclusive scan over the lanes of a warp.
+__device__ __forceinline__ uint32_t warp_scan(uint32_t x, uint32_t lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(~0u, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  return x;
+}
+
+template <int THREADS, int U, typename Src>
+__device__ uint32_t block_select(Src src, uint32_t n, uint32_t k, unsigned long long* cand, SelectSmem& sm) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long key[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t i = u * THREADS + threadIdx.x;
+    key[u] = i < n ? src.fetch(i) : Src::kNone;
+  }
+  if (threadIdx.x == 0) {
+    sm.differ_or = 0;
+    sm.differ_and = ~0ull;
+    sm.kept = 0;
+  }
+  for (uint32_t b = threadIdx.x; b < kSelectBins; b += THREADS) sm.hist[0][b] = 0;
+  unsigned long long any = 0, all = ~0ull;
+  uint32_t mine = 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (u * THREADS >= n) break;
+    key[u] = src.key(key[u]);
+    if (key[u]) {
+      any |= key[u];
+      all &= key[u];
+      ++mine;
+    }
+  }
+  any = (unsigned long long)__reduce_or_sync(~0u, (uint32_t)(any >> 32)) << 32 | __reduce_or_sync(~0u, (uint32_t)any);
+  all = (unsigned long long)__reduce_and_sync(~0u, (uint32_t)(all >> 32)) << 32 | __reduce_and_sync(~0u, (uint32_t)all);
+  mine = __reduce_add_sync(~0u, mine);
+  __syncthreads();
+  if (lane == 0) {
+    sm.warp_sum[warp] = mine;
+    if (mine) {
+      atomicOr(&sm.differ_or, any);
+      atomicAnd(&sm.differ_and, all);
+    }
+  }
+  __syncthreads();
+  const uint32_t m = __reduce_add_sync(~0u, lane < THREADS / 32 ? sm.warp_sum[lane] : 0u);
+  unsigned long long prefix = 0, pmask = 0;  // keys >= prefix are kept (all, when m <= k)
+  if (m > k) {
+    const unsigned long long ones = sm.differ_or, differ = ones ^ sm.differ_and;
+    unsigned long long left = differ;  // differing bits not looked at yet
+    uint32_t need = k;                 // rank (1 = largest) of the wanted key among those matching prefix
+    bool whole = false;
+    for (uint32_t t = 0; left && !whole; t ^= 1) {
+      const int top = 64 - __clzll((long long)left);
+      const int shift = top < kSelectBits ? 0 : top - kSelectBits;
+      const uint32_t dmask = (1u << (top - shift)) - 1u;
+      // the equal bits above the digit belong to the prefix
+      const unsigned long long above = top < 64 ? ~0ull << top : 0ull;
+      prefix |= ones & above & ~pmask;
+      pmask |= above;
+      uint32_t* const hist = sm.hist[t];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (u * THREADS >= n) break;
+        const bool in = key[u] && (key[u] & pmask) == prefix;
+        const uint32_t digit = (uint32_t)(key[u] >> shift) & dmask;
+        const uint32_t zeros = __ballot_sync(~0u, in && digit == 0);  // the common digit: one update per warp
+        if (lane == 0 && zeros) atomicAdd(&hist[0], (uint32_t)__popc(zeros));
+        if (in && digit) atomicAdd(&hist[digit], 1u);
+      }
+      __syncthreads();
+      // thread x holds the bins from the top: kSelectBins - 1 - kPer * x down
+      constexpr uint32_t kPer = kSelectBins / THREADS;
+      const uint32_t first = kSelectBins - 1 - kPer * threadIdx.x;
+      uint32_t sum = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < kPer; ++i) {
+        sum += hist[first - i];
+        sm.hist[t ^ 1][first - i] = 0;
+      }
+      const uint32_t incl = warp_scan(sum, lane);
+      if (lane == 31) sm.warp_sum[warp] = incl;
+      __syncthreads();
+      const uint32_t warps = warp_scan(lane < THREADS / 32 ? sm.warp_sum[lane] : 0u, lane);
+      const uint32_t below = __shfl_sync(~0u, warps, warp ? warp - 1 : 0);
+      const uint32_t upto = incl + (warp ? below : 0u);
+      uint32_t c = upto - sum;
+      if (c < need && need <= upto) {
+        for (uint32_t i = 0; i < kPer; ++i) {
+          const uint32_t h = hist[first - i];
+          if (c + h >= need) {
+            sm.sel[0] = first - i;
+            sm.sel[1] = need - c;
+            sm.sel[2] = h;
+            break;
+          }
+          c += h;
+        }
+      }
+      __syncthreads();
+      prefix |= (unsigned long long)sm.sel[0] << shift;
+      pmask |= (unsigned long long)dmask << shift;
+      need = sm.sel[1];
+      whole = sm.sel[2] == need;  // the bucket's keys are all wanted
+      left &= (1ull << shift) - 1ull;
+    }
+    // every bit below was equal or is all wanted: the prefix is the bound
+    if (!whole) prefix |= ones & ~pmask;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (u * THREADS >= n) break;
+    if (key[u] && key[u] >= prefix) cand[atomicAdd(&sm.kept, 1u)] = key[u];
+  }
+  __syncthreads();
+  return sm.kept;
 }
 
 // Key of a table slot: count << 32 | ~vertex (larger = more visits, then the
@@ -455,17 +571,47 @@ struct SlotKey {
 struct CandKey {  // candidate lists hold keys already (0 = none)
   static constexpr unsigned long long kNone = 0ull;
   const unsigned long long* c;
-  __device__ unsigned long long fetch(uint32_t i) const { return c[i]; }
+  __device__ unsigned long long fetch(uint32_t i) const { return __ldcg(c + i); }  // other CTAs' lists
   __device__ static unsigned long long key(unsigned long long v) { return v; }
 };
 
-__device__ void write_topk(const unsigned long long* cand, uint32_t q, uint32_t k, uint32_t* out_ids,
+// Row q of the result: the n <= k distinct keys of cand by rank, largest
+// first, a key per thread counting the larger ones; then empty entries.
+__device__ void write_topk(const unsigned long long* cand, uint32_t n, uint32_t q, uint32_t k, uint32_t* out_ids,
                            uint32_t* out_counts) {
+  out_ids += (unsigned long long)q * k;
+  out_counts += (unsigned long long)q * k;
   for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) {
-    const unsigned long long key = cand[r];
-    out_ids[(unsigned long long)q * k + r] = key ? ~(uint32_t)key : 0xffffffffu;
-    out_counts[(unsigned long long)q * k + r] = (uint32_t)(key >> 32);
+    const unsigned long long key = r < n ? cand[r] : 0ull;
+    uint32_t rank = r;
+    if (r < n) {
+      rank = 0;
+      for (uint32_t j = 0; j < n; ++j) rank += cand[j] > key ? 1u : 0u;
+    }
+    out_ids[rank] = key ? ~(uint32_t)key : 0xffffffffu;
+    out_counts[rank] = (uint32_t)(key >> 32);
   }
+}
+
+// Shared memory of a ranking CTA.
+struct TopkSmem {
+  unsigned long long cand[kTopkBuffer];
+  SelectSmem select;
+  uint32_t ncand;
+  unsigned long long thresh;
+};
+
+// Small tables are ranked from registers: 8 slots per thread, so that the
+// streaming of the large ones keeps its three CTAs per SM.
+constexpr int kSmallUnroll = 8;
+
+__device__ uint32_t best_slots(const SlotKey& src, uint32_t n, uint32_t k, TopkSmem& sm) {
+  return n <= kSmallUnroll * kTopkThreads ? block_select<kTopkThreads, kSmallUnroll>(src, n, k, sm.cand, sm.select)
+                                          : block_best(src, n, k, sm.cand, sm.ncand, sm.thresh);
+}
+
+__device__ __forceinline__ SlotKey table_slots(const QueryView& qv, uint32_t q, uint32_t first) {
+  return SlotKey{qv.tables + qv.table_off[q] + first, l2_policy(true, false), qv.tag, qv.tag_mask};
 }
 
 // One CTA per query over its whole table; CTA i takes query q_begin +
@@ -473,13 +619,21 @@ __device__ void write_topk(const unsigned long long* cand, uint32_t q, uint32_t 
 __global__ void __launch_bounds__(kTopkThreads, 3)
     topk_kernel(QueryView qv, uint32_t q_begin, uint32_t k, const uint32_t* __restrict__ order,
                 uint32_t* __restrict__ out_ids, uint32_t* __restrict__ out_counts) {
-  __shared__ unsigned long long cand[kTopkBuffer];
-  __shared__ uint32_t ncand;
-  __shared__ unsigned long long thresh;
+  __shared__ TopkSmem sm;
   const uint32_t q = q_begin + (order ? __ldg(order + blockIdx.x) : blockIdx.x);
-  block_best(SlotKey{qv.tables + qv.table_off[q], l2_policy(true, false), qv.tag, qv.tag_mask}, qv.table_mask[q] + 1,
-             k, cand, ncand, thresh);
-  write_topk(cand, q, k, out_ids, out_counts);
+  const uint32_t n = best_slots(table_slots(qv, q, 0), qv.table_mask[q] + 1, k, sm);
+  write_topk(sm.cand, n, q, k, out_ids, out_counts);
+}
+
+// The query holding segment g.
+__device__ __forceinline__ uint32_t segment_query(const unsigned long long* __restrict__ seg_first, uint32_t lo,
+                                                  uint32_t hi, unsigned long long g) {
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (seg_first[mid] <= g) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
 }
 
 // One CTA per table segment of seg_slots slots (CTA i takes segment
@@ -491,27 +645,17 @@ __global__ void __launch_bounds__(kTopkThreads, 3)
                         const unsigned long long* __restrict__ seg_first, const uint32_t* __restrict__ order,
                         unsigned long long* __restrict__ seg_cand, uint32_t* __restrict__ out_ids,
                         uint32_t* __restrict__ out_counts) {
-  __shared__ unsigned long long cand[kTopkBuffer];
-  __shared__ uint32_t ncand;
-  __shared__ unsigned long long thresh;
+  __shared__ TopkSmem sm;
   const unsigned long long g = seg_first[q_begin] + (order ? __ldg(order + blockIdx.x) : blockIdx.x);
-  uint32_t lo = q_begin, hi = q_begin + q_count - 1;  // the query holding segment g
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (seg_first[mid] <= g) lo = mid;
-    else hi = mid - 1;
-  }
-  const uint32_t q = lo;
+  const uint32_t q = segment_query(seg_first, q_begin, q_begin + q_count - 1, g);
   const unsigned long long nseg = seg_first[q + 1] - seg_first[q];
   const uint32_t cap = qv.table_mask[q] + 1;
   const uint32_t first = (uint32_t)(g - seg_first[q]) * seg_slots;
-  const uint32_t n = cap - first < seg_slots ? cap - first : seg_slots;
-  block_best(SlotKey{qv.tables + qv.table_off[q] + first, l2_policy(true, false), qv.tag, qv.tag_mask}, n, k, cand,
-             ncand, thresh);
+  const uint32_t n = best_slots(table_slots(qv, q, first), cap - first < seg_slots ? cap - first : seg_slots, k, sm);
   if (nseg == 1) {
-    write_topk(cand, q, k, out_ids, out_counts);
+    write_topk(sm.cand, n, q, k, out_ids, out_counts);
   } else {
-    for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) seg_cand[g * k + r] = cand[r];
+    for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) seg_cand[g * k + r] = r < n ? sm.cand[r] : 0ull;
   }
 }
 
@@ -520,14 +664,54 @@ __global__ void __launch_bounds__(kTopkThreads, 3)
     topk_merge_kernel(uint32_t q_begin, uint32_t k, const unsigned long long* __restrict__ seg_first,
                       const unsigned long long* __restrict__ seg_cand, uint32_t* __restrict__ out_ids,
                       uint32_t* __restrict__ out_counts) {
-  __shared__ unsigned long long cand[kTopkBuffer];
-  __shared__ uint32_t ncand;
-  __shared__ unsigned long long thresh;
+  __shared__ TopkSmem sm;
   const uint32_t q = q_begin + blockIdx.x;
   const unsigned long long s0 = seg_first[q], nseg = seg_first[q + 1] - s0;
   if (nseg < 2) return;
-  block_best(CandKey{seg_cand + s0 * k}, (uint32_t)(nseg * k), k, cand, ncand, thresh);
-  write_topk(cand, q, k, out_ids, out_counts);
+  const CandKey src{seg_cand + s0 * k};
+  const uint32_t keys = (uint32_t)(nseg * k);
+  const uint32_t n = keys <= kSmallUnroll * kTopkThreads
+                         ? block_select<kTopkThreads, kSmallUnroll>(src, keys, k, sm.cand, sm.select)
+                         : block_best(src, keys, k, sm.cand, sm.ncand, sm.thresh);
+  write_topk(sm.cand, n, q, k, out_ids, out_counts);
+}
+
+// A few queries: segments of kTopkFewSlots slots, ranked from registers, and
+// the CTA that finishes a query's last segment merges its lists (at most
+// kTopkFewKeys keys), so a query costs one launch.  seg_done: per query,
+// segments finished (zero; left zero).
+//
+// One query of 100,000 walks (a million slots) took 26 us in 64 streaming CTAs
+// and 22 us in the merge's one, most of it barriers; here 26 together (ncu, cold L2).
+__global__ void __launch_bounds__(kTopkFewThreads, 1)
+    topk_few_kernel(QueryView qv, uint32_t q_begin, uint32_t q_count, uint32_t k,
+                    const unsigned long long* __restrict__ seg_first, unsigned long long* seg_cand,
+                    uint32_t* __restrict__ seg_done, uint32_t* __restrict__ out_ids,
+                    uint32_t* __restrict__ out_counts) {
+  __shared__ unsigned long long cand[kTopkMaxK];
+  __shared__ SelectSmem select;
+  __shared__ bool last;
+  const unsigned long long g = seg_first[q_begin] + blockIdx.x;
+  const uint32_t q = segment_query(seg_first, q_begin, q_begin + q_count - 1, g);
+  const uint32_t nseg = (uint32_t)(seg_first[q + 1] - seg_first[q]);
+  const uint32_t cap = qv.table_mask[q] + 1, first = (uint32_t)(g - seg_first[q]) * kTopkFewSlots;
+  uint32_t n = block_select<kTopkFewThreads, kTopkFewSlots / kTopkFewThreads>(
+      table_slots(qv, q, first), cap - first < kTopkFewSlots ? cap - first : kTopkFewSlots, k, cand, select);
+  if (nseg > 1) {
+    for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) seg_cand[g * k + r] = r < n ? cand[r] : 0ull;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      last = atomicAdd(seg_done + q, 1u) + 1 == nseg;
+      if (last) seg_done[q] = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    n = block_select<kTopkFewThreads, kTopkFewKeys / kTopkFewThreads>(CandKey{seg_cand + seg_first[q] * k}, nseg * k, k,
+                                                                      cand, select);
+  }
+  write_topk(cand, n, q, k, out_ids, out_counts);
 }
 
 __global__ void clear_tables_kernel(ulonglong2* __restrict__ t, unsigned long long n2) {
@@ -535,6 +719,17 @@ __global__ void clear_tables_kernel(ulonglong2* __restrict__ t, unsigned long lo
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n2;
        i += (unsigned long long)gridDim.x * blockDim.x)
     t[i] = empty;
+}
+
+// One CTA per piece of a query's table (tables are powers of two of at least
+// 256 slots).
+__global__ void __launch_bounds__(256)
+    clear_queries_kernel(QueryView qv, const unsigned long long* __restrict__ piece_first) {
+  const uint32_t q = segment_query(piece_first, 0, qv.nq - 1, blockIdx.x);
+  const uint32_t slots = qv.table_mask[q] + 1, first = (uint32_t)(blockIdx.x - piece_first[q]) * kClearSlots;
+  const uint32_t n2 = (slots - first < kClearSlots ? slots - first : kClearSlots) / 2;
+  ulonglong2* const t = reinterpret_cast<ulonglong2*>(qv.tables + qv.table_off[q] + first);
+  for (uint32_t i = threadIdx.x; i < n2; i += 256) t[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
 }
 
 int sm_count() {
@@ -600,10 +795,30 @@ cudaError_t launch_clear_tables(unsigned long long* tables, unsigned long long n
   return cudaGetLastError();
 }
 
-uint32_t topk_segment_slots(uint32_t nq) {
+cudaError_t launch_clear_queries(const QueryView& qv, const unsigned long long* d_piece_first, uint64_t npieces,
+                                 cudaStream_t stream) {
+  if (npieces == 0) return cudaSuccess;
+  if (npieces > 0x7fffffffull) return cudaErrorInvalidValue;
+  clear_queries_kernel<<<(unsigned)npieces, 256, 0, stream>>>(qv, d_piece_first);
+  return cudaGetLastError();
+}
+
+uint32_t topk_segment_slots(const uint32_t* table_mask, uint32_t nq) {
+  uint64_t few = 0;
+  for (uint32_t q = 0; q < nq && few <= kTopkFewSegments; ++q) few += table_mask[q] / kTopkFewSlots + 1;
+  if (few <= kTopkFewSegments) return kTopkFewSlots;
   uint64_t s = kTopkSegment;
   while (s < (1ull << 30) && s / kTopkSegment * 64 < nq) s <<= 1;  // 64 queries per doubling
   return (uint32_t)s;
+}
+
+bool topk_is_few(const unsigned long long* seg_first, uint32_t nq, uint32_t seg_slots, uint32_t k) {
+  // the register path pays while its CTAs (one per SM) make few waves, and one
+  // CTA must be able to hold a query's lists
+  if (seg_slots != kTopkFewSlots || seg_first[nq] - seg_first[0] > kTopkFewSegments) return false;
+  for (uint32_t q = 0; q < nq; ++q)
+    if ((seg_first[q + 1] - seg_first[q]) * k > kTopkFewKeys) return false;
+  return true;
 }
 
 void topk_segment_prefix(const uint32_t* table_mask, uint32_t nq, uint32_t seg_slots, unsigned long long* seg_first) {
@@ -633,11 +848,17 @@ void topk_segment_order(const uint32_t* table_mask, uint32_t nq, uint32_t seg_sl
 cudaError_t launch_topk_segmented(const QueryView& qv, uint32_t q_begin, uint32_t q_count, uint32_t k,
                                   uint32_t* out_ids, uint32_t* out_counts, const unsigned long long* d_seg_first,
                                   const unsigned long long* h_seg_first, uint32_t seg_slots,
-                                  unsigned long long* d_seg_cand, const uint32_t* d_order, cudaStream_t stream) {
+                                  unsigned long long* d_seg_cand, uint32_t* d_seg_done, const uint32_t* d_order,
+                                  cudaStream_t stream) {
   if (q_count == 0) return cudaSuccess;
   if (k == 0 || k > kTopkMaxK) return cudaErrorInvalidValue;
   const unsigned long long nseg = h_seg_first[q_begin + q_count] - h_seg_first[q_begin];
   if (nseg == 0 || nseg > 0x7fffffffull) return cudaErrorInvalidValue;
+  if (topk_is_few(h_seg_first + q_begin, q_count, seg_slots, k)) {
+    topk_few_kernel<<<(unsigned)nseg, kTopkFewThreads, 0, stream>>>(qv, q_begin, q_count, k, d_seg_first, d_seg_cand,
+                                                                  d_seg_done, out_ids, out_counts);
+    return cudaGetLastError();
+  }
   if (nseg == q_count) {  // no table is split: one CTA per query
     topk_kernel<<<q_count, kTopkThreads, 0, stream>>>(qv, q_begin, k, d_order, out_ids, out_counts);
     return cudaGetLastError();
@@ -650,14 +871,6 @@ cudaError_t launch_topk_segmented(const QueryView& qv, uint32_t q_begin, uint32_
     e = cudaGetLastError();
   }
   return e;
-}
-
-cudaError_t launch_topk(const QueryView& qv, uint32_t q_begin, uint32_t q_count, uint32_t k, uint32_t* out_ids,
-                        uint32_t* out_counts, cudaStream_t stream) {
-  if (q_count == 0) return cudaSuccess;
-  if (k == 0 || k > kTopkMaxK) return cudaErrorInvalidValue;
-  topk_kernel<<<q_count, kTopkThreads, 0, stream>>>(qv, q_begin, k, nullptr, out_ids, out_counts);
-  return cudaGetLastError();
 }
 
 }  // namespace gw

@@ -89,7 +89,7 @@ gw_status plan_set(gw_ctx* ctx, const uint32_t* sources, const uint32_t* budgets
 
 // batched: the top-k segments grow with the set (64 queries per doubling),
 // so one launch ranks the whole set; one query at a time (plain), every table
-// splits into kTopkSegment-slot segments, so a large table is ranked by many
+// splits into kTopkFewSlots-slot segments, so a large table is ranked by many
 // CTAs instead of one.
 gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool batched) {
   const uint32_t n = (uint32_t)s->qmap.size();
@@ -102,12 +102,12 @@ gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool
   const size_t table_bytes0 = s->d_tables->bytes;
   GW_CUDA(ctx, s->d_tables->ensure(s->slots * 8), "query tables alloc");
   s->fresh_tables = s->d_tables->p != tables0 || s->d_tables->bytes != table_bytes0;
-  GW_CUDA(ctx, s->d_full->ensure(n * 4), "query alloc");
+  GW_CUDA(ctx, s->d_full->ensure(2 * (size_t)n * 4), "query alloc");  // table-full flags, segments ranked
   GW_CUDA(ctx, s->d_ids->ensure((uint64_t)n * k * 4), "top-k alloc");
   GW_CUDA(ctx, s->d_cnt->ensure((uint64_t)n * k * 4), "top-k alloc");
   GW_CUDA(ctx, s->d_cursor->ensure(sizeof(unsigned long long)), "query alloc");
   s->seg_first.resize(n + 1);
-  s->seg_slots = batched ? gw::topk_segment_slots(n) : gw::kTopkSegment;
+  s->seg_slots = batched ? gw::topk_segment_slots(s->tmask.data(), n) : gw::kTopkFewSlots;
   gw::topk_segment_prefix(s->tmask.data(), n, s->seg_slots, s->seg_first.data());
   s->seg_order.resize(s->seg_first[n]);
   gw::topk_segment_order(s->tmask.data(), n, s->seg_slots, s->seg_first.data(), s->seg_order.data());
@@ -122,7 +122,7 @@ gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool
   GW_CUDA(ctx, cudaMemcpyAsync(s->d_id_base->p, s->id_base.data(), n * 8, cudaMemcpyHostToDevice, st), "copy");
   GW_CUDA(ctx, cudaMemcpyAsync(s->d_toff->p, s->toff.data(), n * 8, cudaMemcpyHostToDevice, st), "copy");
   GW_CUDA(ctx, cudaMemcpyAsync(s->d_tmask->p, s->tmask.data(), n * 4, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemsetAsync(s->d_full->p, 0, n * 4, st), "clear flags");
+  GW_CUDA(ctx, cudaMemsetAsync(s->d_full->p, 0, 2 * (size_t)n * 4, st), "clear flags");
   s->qv.sources = s->d_sources->as<uint32_t>();
   s->qv.walk_prefix = s->d_prefix->as<unsigned long long>();
   s->qv.id_base = s->d_id_base->as<unsigned long long>();
@@ -191,10 +191,10 @@ cudaError_t run_set(gw_ctx* ctx, const gw_walk_params* p, const gw::WalkArgs& a,
     if (e == cudaSuccess)
       e = gw::launch_topk_segmented(s->qv, 0, n, k, s->d_ids->as<uint32_t>(), s->d_cnt->as<uint32_t>(),
                                     s->d_segs->as<unsigned long long>(), s->seg_first.data(), s->seg_slots,
-                                    s->d_cand->as<unsigned long long>(),
+                                    s->d_cand->as<unsigned long long>(), s->qv.full + n,
                                     reinterpret_cast<const uint32_t*>(s->d_segs->as<unsigned long long>() + n + 1), st);
     cudaEventRecord(ev[3], st);
-    *launches += (s->seg_first[n] > n ? 3 : 2) + (cleared ? 1 : 0);
+    *launches += (s->seg_first[n] > n && !gw::topk_is_few(s->seg_first.data(), n, s->seg_slots, k) ? 3 : 2) + (cleared ? 1 : 0);
   } else {
     cudaEventRecord(ev[1], st);
     *launches += cleared ? 1 : 0;
@@ -206,8 +206,8 @@ cudaError_t run_set(gw_ctx* ctx, const gw_walk_params* p, const gw::WalkArgs& a,
       if (e == cudaSuccess)
         e = gw::launch_topk_segmented(s->qv, q, 1, k, s->d_ids->as<uint32_t>(), s->d_cnt->as<uint32_t>(),
                                       s->d_segs->as<unsigned long long>(), s->seg_first.data(), s->seg_slots,
-                                      s->d_cand->as<unsigned long long>(), nullptr, st);
-      *launches += s->seg_first[q + 1] - s->seg_first[q] > 1 ? 1 : 0;
+                                      s->d_cand->as<unsigned long long>(), s->qv.full + n, nullptr, st);
+      if (s->seg_first[q + 1] - s->seg_first[q] > 1 && !gw::topk_is_few(&s->seg_first[q], 1, s->seg_slots, k)) ++*launches;
     }
     cudaEventRecord(ev[2], st);
     cudaEventRecord(ev[3], st);

@@ -4,7 +4,8 @@
 // scheduler thread repeats supersteps:
 //   1. admit arrived queries in FIFO order while their visit table fits in the
 //      arena (a query that does not fit waits until completed queries free
-//      space), clearing each new table;
+//      space); one launch clears the tables of the queries that start now (one
+//      launch each took 590 us for a burst of 256);
 //   2. launch one walk kernel over a mix of walk chunks: every admitted query
 //      with walks left contributes up to `quantum` of them (the plain mode
 //      takes one whole query per superstep instead);
@@ -124,49 +125,54 @@ struct gw_server {
   gw_hostbuf h_stage;
   gw_devbuf d_stage;
   uint32_t stage_cap = 0;
-  gw_devbuf d_topk_segs, d_topk_cand;  // segmented top-k of large finishing tables
+  gw_devbuf d_topk_cand;  // segmented top-k of large finishing tables
 };
 
 namespace {
 
 // Staging layout for up to n queries in one superstep: the launch's chunk
-// cursor; the per-query inputs (copied up); then the results, one contiguous
-// range copied back: the launch's status word, the table-full flags and the
-// top-k lists.  The status word and the flags are also copied up, as zeros.
+// cursor; the per-query inputs (copied up), with the pieces of the tables to
+// clear and the top-k segments; then the results, one contiguous range copied
+// back: the launch's status word, the table-full flags and the top-k lists.
+// The segment counters, the status word and the flags are also copied up, as
+// zeros.
 struct Stage {
-  unsigned long long *cursor, *prefix, *id_base, *toff;
-  uint32_t *sources, *tmask, *stream, *status, *full, *ids, *counts;
+  unsigned long long *cursor, *prefix, *id_base, *toff, *clear_first, *seg_first;
+  uint32_t *sources, *tmask, *stream, *seg_done, *status, *full, *ids, *counts;
 };
 
 size_t stage_bytes(uint32_t n, uint32_t k) {
-  return 8 + (size_t)(n + 1) * 8 + 2 * (size_t)n * 8 + 3 * (size_t)n * 4 + 4 + (size_t)n * 4 +
+  return 8 + 3 * (size_t)(n + 1) * 8 + 2 * (size_t)n * 8 + 4 * (size_t)n * 4 + 4 + (size_t)n * 4 +
          2 * (size_t)n * k * 4;
 }
 
 Stage carve(void* base, uint32_t n, uint32_t k) {
   Stage s;
   char* p = static_cast<char*>(base);
-  s.cursor = reinterpret_cast<unsigned long long*>(p);
-  p += 8;
-  s.prefix = reinterpret_cast<unsigned long long*>(p);
-  p += (size_t)(n + 1) * 8;
-  s.id_base = reinterpret_cast<unsigned long long*>(p);
-  p += (size_t)n * 8;
-  s.toff = reinterpret_cast<unsigned long long*>(p);
-  p += (size_t)n * 8;
-  s.sources = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)n * 4;
-  s.tmask = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)n * 4;
-  s.stream = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)n * 4;
-  s.status = reinterpret_cast<uint32_t*>(p);
-  p += 4;
-  s.full = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)n * 4;
-  s.ids = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)n * k * 4;
-  s.counts = reinterpret_cast<uint32_t*>(p);
+  auto u64s = [&](size_t count) {
+    unsigned long long* x = reinterpret_cast<unsigned long long*>(p);
+    p += count * 8;
+    return x;
+  };
+  auto u32s = [&](size_t count) {
+    uint32_t* x = reinterpret_cast<uint32_t*>(p);
+    p += count * 4;
+    return x;
+  };
+  s.cursor = u64s(1);
+  s.prefix = u64s((size_t)n + 1);
+  s.clear_first = u64s((size_t)n + 1);
+  s.seg_first = u64s((size_t)n + 1);
+  s.id_base = u64s(n);
+  s.toff = u64s(n);
+  s.sources = u32s(n);
+  s.tmask = u32s(n);
+  s.stream = u32s(n);
+  s.seg_done = u32s(n);
+  s.status = u32s(1);
+  s.full = u32s(n);
+  s.ids = u32s((size_t)n * k);
+  s.counts = u32s((size_t)n * k);
   return s;
 }
 
@@ -192,7 +198,7 @@ bool superstep(gw_server* srv) {
   const uint32_t k = srv->cfg.k;
   // Queries are reached through pointers taken under the lock: map nodes do
   // not move, and only this thread changes an admitted query's fields.
-  std::vector<Query*> admitted, cq;
+  std::vector<Query*> cq;
   std::vector<uint64_t> chosen;
   std::vector<uint32_t> take;
   {
@@ -208,7 +214,6 @@ bool superstep(gw_server* srv) {
       q.table_slots = slots;
       q.admit_ns = t;
       srv->active.push_back(srv->pending.front());
-      admitted.push_back(&q);
       srv->pending.pop_front();
     }
     // the walk chunks of this superstep; queries that finish in it go first
@@ -239,8 +244,6 @@ bool superstep(gw_server* srv) {
     take.insert(take.end(), later_take.begin(), later_take.end());
     for (uint64_t tk : chosen) cq.push_back(&srv->queries[tk]);
   }
-  for (Query* q : admitted)
-    gw::launch_clear_tables(srv->tables.as<unsigned long long>() + q->table_off, q->table_slots, st);
   if (chosen.empty()) return true;
   const uint32_t n = (uint32_t)chosen.size();
   if (n > srv->stage_cap) {
@@ -252,7 +255,7 @@ bool superstep(gw_server* srv) {
     srv->stage_cap = n;
   }
   Stage h = carve(srv->h_stage.p, n, k), d = carve(srv->d_stage.p, n, k);
-  unsigned long long acc = 0;
+  unsigned long long acc = 0, pieces = 0;  // pieces: of the tables of queries whose first walks run now
   uint32_t nfin = 0;  // leading queries whose last walks run now
   for (uint32_t i = 0; i < n; ++i) {
     const Query& q = *cq[i];
@@ -263,36 +266,32 @@ bool superstep(gw_server* srv) {
     h.sources[i] = q.source;
     h.tmask[i] = (uint32_t)(q.table_slots - 1);
     h.full[i] = 0;
+    h.seg_done[i] = 0;
     h.stream[i] = q.stream;
+    h.clear_first[i] = pieces;
+    if (q.issued == 0) pieces += (q.table_slots + gw::kClearSlots - 1) / gw::kClearSlots;
     acc += take[i];
   }
   h.prefix[n] = acc;
+  h.clear_first[n] = pieces;
+  // queries whose last walks are in this superstep get their top-k after them;
+  // a large table is ranked by several CTAs (segmented top-k)
+  const uint32_t seg_slots = gw::topk_segment_slots(h.tmask, nfin);
+  gw::topk_segment_prefix(h.tmask, nfin, seg_slots, h.seg_first);
   h.status[0] = 0;
   const size_t head = stage_bytes(n, k) - 8 - 2 * (size_t)n * k * 4;  // prefix .. full
   cudaError_t e = cudaMemcpyAsync(d.prefix, h.prefix, head, cudaMemcpyHostToDevice, st);
   gw::QueryView qv = make_view(d, srv->tables.as<unsigned long long>(), n);
   qv.chunk = ctx->ppr_chunk;
+  if (e == cudaSuccess) e = gw::launch_clear_queries(qv, d.clear_first, pieces, st);
   if (e == cudaSuccess)
     e = gw::launch_walk_queries((int)srv->params.rule, qv, 0, acc, ctx->view(), srv->args, d.status,
                                 ctx->ppr_threads_per_sm, st);
-  // queries whose last walks are in this superstep get their top-k now; a
-  // large table is ranked by several CTAs (segmented top-k)
   if (e == cudaSuccess && nfin) {
-    const uint32_t seg_slots = gw::topk_segment_slots(nfin);
-    std::vector<unsigned long long> sf(nfin + 1);
-    gw::topk_segment_prefix(h.tmask, nfin, seg_slots, sf.data());
-    if (sf[nfin] == nfin) {
-      e = gw::launch_topk(qv, 0, nfin, k, d.ids, d.counts, st);
-    } else {
-      e = srv->d_topk_segs.ensure((nfin + 1) * 8);
-      if (e == cudaSuccess) e = srv->d_topk_cand.ensure(sf[nfin] * k * 8);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(srv->d_topk_segs.p, sf.data(), (nfin + 1) * 8, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess)
-        e = gw::launch_topk_segmented(qv, 0, nfin, k, d.ids, d.counts, srv->d_topk_segs.as<unsigned long long>(),
-                                      sf.data(), seg_slots, srv->d_topk_cand.as<unsigned long long>(), nullptr, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // sf is read by the copy above
-    }
+    e = srv->d_topk_cand.ensure(h.seg_first[nfin] * k * 8);
+    if (e == cudaSuccess)
+      e = gw::launch_topk_segmented(qv, 0, nfin, k, d.ids, d.counts, d.seg_first, h.seg_first, seg_slots,
+                                    srv->d_topk_cand.as<unsigned long long>(), d.seg_done, nullptr, st);
   }
   // status, flags and lists come back in one copy, then one synchronisation
   if (e == cudaSuccess)
@@ -328,8 +327,7 @@ bool superstep(gw_server* srv) {
       if (srv->arena.alloc(slots, &off)) {
         q.table_off = off;
         q.table_slots = slots;
-        srv->active.push_back(chosen[i]);
-        gw::launch_clear_tables(srv->tables.as<unsigned long long>() + off, slots, st);
+        srv->active.push_back(chosen[i]);  // its table is cleared with its first walks
       } else {
         srv->pending.push_front(chosen[i]);  // waits at the head of the queue for space
       }
@@ -515,7 +513,6 @@ gw_status gw_serve_close(gw_server* srv) {
   srv->tables.release();
   srv->h_stage.release();
   srv->d_stage.release();
-  srv->d_topk_segs.release();
   srv->d_topk_cand.release();
   const gw_status s = srv->fatal;
   delete srv;

@@ -213,3 +213,35 @@ def test_expected_visits_edge_runs(cuda_device, oracle, edges, rule, L):
                 got = G.expected_visits(gw.params(rule, gw.SINK_NONE, L), src)
             ref = oracle.expected_visits(rp, ci, src, rule, L)
             assert np.allclose(got, ref, rtol=L * (len(ci) + nv) * 2.0 ** -53, atol=0), (src, np.abs(got - ref).max())
+
+
+@pytest.mark.parametrize("budgets", [[1], [32], [512], [513], [2048], [2049], [30_000], [40, 5000, 0, 20_000],
+                                     [300] * 150 + [9000] * 150],
+                         ids=lambda b: "x".join(map(str, (len(b), max(b)))))
+@pytest.mark.parametrize("k", [1, 100, 512])
+def test_topk_at_table_sizes(cuda_device, oracle, budgets, k):
+    """Tables of 256 slots (one walk) up to 16 segments of 16384; exactly the
+    4096 slots a batch ranks from registers (512 walks) and twice that; exactly
+    one segment (2048 walks) and two; merges of up to 8192 keys (k = 512); a
+    batch too wide for the register path.  Ties by the thousand: most vertices
+    of a walk from a low-degree source are visited once."""
+    import graphwalker_b200 as gw
+    rp, ci = oracle.rmat_csr(15, 8, seed=8)
+    deg = np.diff(rp.astype(np.int64))
+    rng = np.random.default_rng(k)
+    sources = rng.choice(np.nonzero(deg)[0], len(budgets)).astype(np.uint32)
+    b = np.array(budgets, np.uint32)
+    with gw.Graph.from_csr(rp, ci, oracle.compute_blocks(rp, 256)) as G:
+        p = gw.params(gw.RULE_PPR, gw.SINK_NONE, 10, seed=3)
+        got = [G.ppr(p, sources, b, k=k, batched=x)[:2] for x in (True, False, True)]
+    for ids, cnt in got[1:]:
+        assert np.array_equal(ids, got[0][0]) and np.array_equal(cnt, got[0][1])
+    check = range(len(b)) if len(b) < 10 else (0, 149, 150, 299)
+    prefix = np.r_[0, np.cumsum(b.astype(np.int64))]
+    for q in check:
+        cur = np.full(b[q], sources[q], np.uint32)
+        r = oracle.run_walks(rp, ci, cur, ids=np.arange(prefix[q], prefix[q + 1], dtype=np.uint32), src=cur,
+                             rule=gw.RULE_PPR, L=10, seed=3)
+        v = np.nonzero(r["counts"])[0] if b[q] else np.zeros(0, np.int64)
+        want = _topk_ref(dict(zip(v.tolist(), r["counts"][v].tolist())), k)
+        assert np.array_equal(got[0][0][q], want[0]) and np.array_equal(got[0][1][q], want[1]), q
