@@ -477,10 +477,8 @@ gw_status gw_close(gw_ctx* ctx) {
                        &ctx->d_status,
                        &ctx->d_walks, &ctx->d_words, &ctx->d_ids, &ctx->d_counts, &ctx->d_paths,
                        &ctx->d_plen, &ctx->d_closure, &ctx->d_pool_offsets, &ctx->d_dest,
-                       &ctx->d_tile_hist, &ctx->d_minhop, &ctx->d_pool_table, &ctx->d_q_sources,
-                       &ctx->d_q_prefix, &ctx->d_q_idbase, &ctx->d_q_toff, &ctx->d_q_tmask, &ctx->d_q_tables,
-                       &ctx->d_q_full, &ctx->d_q_ids, &ctx->d_q_counts, &ctx->d_q_visits,
-                       &ctx->d_q_cursor, &ctx->d_q_segs, &ctx->d_q_cand})
+                       &ctx->d_tile_hist, &ctx->d_minhop, &ctx->d_pool_table, &ctx->d_q_stage, &ctx->d_q_tables,
+                       &ctx->d_q_cand})
     b->release();
   ctx->release_pools();
   ctx->h_rowptr.release();
@@ -488,6 +486,9 @@ gw_status gw_close(gw_ctx* ctx) {
   ctx->h_status.release();
   ctx->pool_arena.release();
   ctx->h_xfer.release();
+  ctx->h_q_stage.release();
+  for (cudaEvent_t ev : ctx->q_events)
+    if (ev) cudaEventDestroy(ev);
   ctx->slots.release();
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);

@@ -772,8 +772,6 @@ cudaError_t launch_walk_queries(int rule, const QueryView& qv, unsigned long lon
                                 uint32_t* status, int threads_per_sm, cudaStream_t stream) {
   if (w_end <= w_begin || qv.nq == 0) return cudaSuccess;
   if (!qv.cursor) return cudaErrorInvalidValue;
-  const cudaError_t e = cudaMemsetAsync(qv.cursor, 0, sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
   switch (rule) {
     case GW_RULE_JUMP: return query_dispatch<GW_RULE_JUMP>(qv, w_begin, w_end, g, a, status, threads_per_sm, stream);
     case GW_RULE_STOP: return query_dispatch<GW_RULE_STOP>(qv, w_begin, w_end, g, a, status, threads_per_sm, stream);

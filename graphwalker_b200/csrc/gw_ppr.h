@@ -35,7 +35,7 @@ struct QueryView {
   uint32_t* full;                          // nq: set to 1 when query q's table filled up
   const uint32_t* stream;                  // nq: Philox stream word of query q (NULL = 0)
   unsigned long long* visits;              // total visits counter (may be NULL)
-  unsigned long long* cursor;              // batch positions handed out (zeroed by the launcher)
+  unsigned long long* cursor;              // batch positions handed out (zero before the launch)
   uint32_t chunk;                          // walks per cursor grab (0 = kWarpChunk)
   uint32_t nq;
   // Batch tag: the high bits of a slot's vertex word (tag_mask) hold the tag

@@ -15,6 +15,7 @@
 // large enough table would have given.
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "gw_ctx.h"
@@ -30,36 +31,48 @@ uint64_t next_pow2(uint64_t x) {
   return p;
 }
 
-// A set of queries laid out for one launch.  Its device buffers are the
-// context's (kept across calls) for the first round, its own for retries.
+// A set of queries laid out for one launch.  Everything a launch needs besides
+// the tables lies in one staging range, written in pinned host memory and
+// copied up at once, and everything it returns behind it, copied back at once:
+// a query of a few hundred walks spent more time on fifteen small copies than
+// on its walks.  Its device buffers are the context's (kept across calls) for
+// the first round, its own for retries.
 struct QuerySet {
-  std::vector<uint32_t> sources, qmap;  // qmap: index in the caller's query list
+  std::vector<uint32_t> qmap;  // index in the caller's query list
   std::vector<unsigned long long> prefix, id_base, toff;
-  std::vector<uint32_t> tmask;
+  std::vector<uint32_t> sources, tmask;
   std::vector<unsigned long long> seg_first;  // top-k segments per query (prefix)
-  std::vector<uint32_t> seg_order;            // top-k segments in launch order, largest first
-  uint32_t seg_slots = gw::kTopkSegment;
+  uint32_t seg_slots = 0;
   uint64_t walks = 0, slots = 0;
   bool shared = false;        // the context's buffers (tagged), or this set's own (cleared, untagged)
   bool fresh_tables = false;  // d_tables was (re)allocated by upload_set: its content is undefined
-  gw_devbuf own[12];
-  gw_devbuf *d_sources, *d_prefix, *d_id_base, *d_toff, *d_tmask, *d_tables, *d_full, *d_ids, *d_cnt, *d_cursor,
-      *d_segs, *d_cand;
+  gw_devbuf own[3];
+  gw_devbuf *d_stage, *d_tables, *d_cand;
+  size_t back_at = 0, head_bytes = 0;  // the staging range: where the results start, and how much is copied up
   gw::QueryView qv{};
+  unsigned long long* d_seg_first = nullptr;
+  uint32_t *seg_done = nullptr, *seg_order = nullptr, *status = nullptr, *ids = nullptr, *cnt = nullptr;  // device
 
   QuerySet(gw_ctx* ctx, bool use_ctx_buffers) {
-    gw_devbuf* b[12] = {&ctx->d_q_sources, &ctx->d_q_prefix, &ctx->d_q_idbase, &ctx->d_q_toff,
-                        &ctx->d_q_tmask,   &ctx->d_q_tables, &ctx->d_q_full,   &ctx->d_q_ids,
-                        &ctx->d_q_counts,  &ctx->d_q_cursor, &ctx->d_q_segs,   &ctx->d_q_cand};
-    gw_devbuf** d[12] = {&d_sources, &d_prefix, &d_id_base, &d_toff, &d_tmask, &d_tables,
-                         &d_full,    &d_ids,    &d_cnt,     &d_cursor, &d_segs, &d_cand};
-    for (int i = 0; i < 12; ++i) *d[i] = use_ctx_buffers ? b[i] : &own[i];
+    gw_devbuf* b[3] = {&ctx->d_q_stage, &ctx->d_q_tables, &ctx->d_q_cand};
+    gw_devbuf** d[3] = {&d_stage, &d_tables, &d_cand};
+    for (int i = 0; i < 3; ++i) *d[i] = use_ctx_buffers ? b[i] : &own[i];
     shared = use_ctx_buffers;
   }
   ~QuerySet() {
     for (auto& b : own) b.release();
   }
 };
+
+// The results, as they lie behind the inputs: total visits, the status word
+// (and padding), the table-full flags, then the lists.
+struct Results {
+  unsigned long long visits;
+  uint32_t status, unused;
+};
+// Lists up to this size come back through the pinned staging; larger ones go
+// straight to the caller's arrays.
+constexpr size_t kStagedListBytes = 1u << 20;
 
 gw_status plan_set(gw_ctx* ctx, const uint32_t* sources, const uint32_t* budgets, const unsigned long long* ids,
                    const std::vector<uint32_t>& which, uint64_t factor, QuerySet* s) {
@@ -92,46 +105,54 @@ gw_status plan_set(gw_ctx* ctx, const uint32_t* sources, const uint32_t* budgets
 // splits into kTopkFewSlots-slot segments, so a large table is ranked by many
 // CTAs instead of one.
 gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool batched) {
-  const uint32_t n = (uint32_t)s->qmap.size();
-  GW_CUDA(ctx, s->d_sources->ensure(n * 4), "query alloc");
-  GW_CUDA(ctx, s->d_prefix->ensure((n + 1) * 8), "query alloc");
-  GW_CUDA(ctx, s->d_id_base->ensure(n * 8), "query alloc");
-  GW_CUDA(ctx, s->d_toff->ensure(n * 8), "query alloc");
-  GW_CUDA(ctx, s->d_tmask->ensure(n * 4), "query alloc");
+  const size_t n = s->qmap.size();
   const void* tables0 = s->d_tables->p;
   const size_t table_bytes0 = s->d_tables->bytes;
   GW_CUDA(ctx, s->d_tables->ensure(s->slots * 8), "query tables alloc");
   s->fresh_tables = s->d_tables->p != tables0 || s->d_tables->bytes != table_bytes0;
-  GW_CUDA(ctx, s->d_full->ensure(2 * (size_t)n * 4), "query alloc");  // table-full flags, segments ranked
-  GW_CUDA(ctx, s->d_ids->ensure((uint64_t)n * k * 4), "top-k alloc");
-  GW_CUDA(ctx, s->d_cnt->ensure((uint64_t)n * k * 4), "top-k alloc");
-  GW_CUDA(ctx, s->d_cursor->ensure(sizeof(unsigned long long)), "query alloc");
   s->seg_first.resize(n + 1);
-  s->seg_slots = batched ? gw::topk_segment_slots(s->tmask.data(), n) : gw::kTopkFewSlots;
-  gw::topk_segment_prefix(s->tmask.data(), n, s->seg_slots, s->seg_first.data());
-  s->seg_order.resize(s->seg_first[n]);
-  gw::topk_segment_order(s->tmask.data(), n, s->seg_slots, s->seg_first.data(), s->seg_order.data());
-  // d_segs: seg_first (n + 1 u64), then seg_order (u32 per segment)
-  GW_CUDA(ctx, s->d_segs->ensure((n + 1) * 8 + s->seg_first[n] * 4), "top-k segments");
-  GW_CUDA(ctx, s->d_cand->ensure(s->seg_first[n] * k * 8 + 8), "top-k candidates");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_segs->p, s->seg_first.data(), (n + 1) * 8, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_segs->as<unsigned long long>() + n + 1, s->seg_order.data(), s->seg_first[n] * 4,
-                               cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_sources->p, s->sources.data(), n * 4, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_prefix->p, s->prefix.data(), (n + 1) * 8, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_id_base->p, s->id_base.data(), n * 8, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_toff->p, s->toff.data(), n * 8, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemcpyAsync(s->d_tmask->p, s->tmask.data(), n * 4, cudaMemcpyHostToDevice, st), "copy");
-  GW_CUDA(ctx, cudaMemsetAsync(s->d_full->p, 0, 2 * (size_t)n * 4, st), "clear flags");
-  s->qv.sources = s->d_sources->as<uint32_t>();
-  s->qv.walk_prefix = s->d_prefix->as<unsigned long long>();
-  s->qv.id_base = s->d_id_base->as<unsigned long long>();
-  s->qv.table_off = s->d_toff->as<unsigned long long>();
-  s->qv.table_mask = s->d_tmask->as<uint32_t>();
+  s->seg_slots = batched ? gw::topk_segment_slots(s->tmask.data(), (uint32_t)n) : gw::kTopkFewSlots;
+  gw::topk_segment_prefix(s->tmask.data(), (uint32_t)n, s->seg_slots, s->seg_first.data());
+  const size_t nseg = s->seg_first[n];
+  GW_CUDA(ctx, s->d_cand->ensure(nseg * k * 8 + 8), "top-k candidates");
+  // 64-bit arrays first: prefix, seg_first (n + 1 each), id_base, toff, cursors
+  // (n each); then sources, tmask, segment counters, segment order; then the results
+  const size_t u64s = 2 * (n + 1) + 3 * n, u32s = 3 * n + nseg;
+  s->back_at = (u64s * 8 + u32s * 4 + 7) / 8 * 8;
+  s->head_bytes = s->back_at + sizeof(Results) + n * 4;
+  GW_CUDA(ctx, s->d_stage->ensure(s->head_bytes + 2 * n * k * 4), "query alloc");
+  GW_CUDA(ctx, ctx->h_q_stage.ensure(s->head_bytes + std::min(2 * n * k * 4, kStagedListBytes)), "query staging");
+  char* const h = ctx->h_q_stage.as<char>();
+  char* const d = s->d_stage->as<char>();
+  memset(h, 0, s->head_bytes);  // cursors, segment counters, results start at zero
+  size_t at = 0;
+  auto put = [&](const void* src, size_t count, size_t width) {  // returns the array's place on the device
+    if (src) memcpy(h + at, src, count * width);
+    char* const where = d + at;
+    at += count * width;
+    return where;
+  };
+  s->qv.walk_prefix = reinterpret_cast<unsigned long long*>(put(s->prefix.data(), n + 1, 8));
+  auto* seg_first = reinterpret_cast<unsigned long long*>(put(s->seg_first.data(), n + 1, 8));
+  s->qv.id_base = reinterpret_cast<unsigned long long*>(put(s->id_base.data(), n, 8));
+  s->qv.table_off = reinterpret_cast<unsigned long long*>(put(s->toff.data(), n, 8));
+  s->qv.cursor = reinterpret_cast<unsigned long long*>(put(nullptr, n, 8));
+  s->qv.sources = reinterpret_cast<uint32_t*>(put(s->sources.data(), n, 4));
+  s->qv.table_mask = reinterpret_cast<uint32_t*>(put(s->tmask.data(), n, 4));
+  s->seg_done = reinterpret_cast<uint32_t*>(put(nullptr, n, 4));
+  s->seg_order = reinterpret_cast<uint32_t*>(d + at);
+  gw::topk_segment_order(s->tmask.data(), (uint32_t)n, s->seg_slots, s->seg_first.data(),
+                         reinterpret_cast<uint32_t*>(h + at));
+  Results* const r = reinterpret_cast<Results*>(d + s->back_at);
+  s->qv.visits = &r->visits;
+  s->status = &r->status;
+  s->qv.full = reinterpret_cast<uint32_t*>(r + 1);
+  s->ids = s->qv.full + n;
+  s->cnt = s->ids + n * k;
   s->qv.tables = s->d_tables->as<unsigned long long>();
-  s->qv.full = s->d_full->as<uint32_t>();
-  s->qv.cursor = s->d_cursor->as<unsigned long long>();
-  s->qv.nq = n;
+  s->qv.nq = (uint32_t)n;
+  s->d_seg_first = seg_first;
+  GW_CUDA(ctx, cudaMemcpyAsync(d, h, s->head_bytes, cudaMemcpyHostToDevice, st), "query copy");
   return GW_OK;
 }
 
@@ -185,14 +206,11 @@ cudaError_t run_set(gw_ctx* ctx, const gw_walk_params* p, const gw::WalkArgs& a,
   if (batched) {
     cudaEventRecord(ev[1], st);
     if (e == cudaSuccess)
-      e = gw::launch_walk_queries((int)p->rule, s->qv, 0, s->walks, ctx->view(), a, ctx->d_status.as<uint32_t>(),
-                                  threads_per_sm, st);
+      e = gw::launch_walk_queries((int)p->rule, s->qv, 0, s->walks, ctx->view(), a, s->status, threads_per_sm, st);
     cudaEventRecord(ev[2], st);
     if (e == cudaSuccess)
-      e = gw::launch_topk_segmented(s->qv, 0, n, k, s->d_ids->as<uint32_t>(), s->d_cnt->as<uint32_t>(),
-                                    s->d_segs->as<unsigned long long>(), s->seg_first.data(), s->seg_slots,
-                                    s->d_cand->as<unsigned long long>(), s->qv.full + n,
-                                    reinterpret_cast<const uint32_t*>(s->d_segs->as<unsigned long long>() + n + 1), st);
+      e = gw::launch_topk_segmented(s->qv, 0, n, k, s->ids, s->cnt, s->d_seg_first, s->seg_first.data(), s->seg_slots,
+                                    s->d_cand->as<unsigned long long>(), s->seg_done, s->seg_order, st);
     cudaEventRecord(ev[3], st);
     *launches += (s->seg_first[n] > n && !gw::topk_is_few(s->seg_first.data(), n, s->seg_slots, k) ? 3 : 2) + (cleared ? 1 : 0);
   } else {
@@ -200,13 +218,13 @@ cudaError_t run_set(gw_ctx* ctx, const gw_walk_params* p, const gw::WalkArgs& a,
     *launches += cleared ? 1 : 0;
     for (uint32_t q = 0; q < n && e == cudaSuccess; ++q) {
       e = gw::launch_clear_tables(s->qv.tables + s->toff[q], (uint64_t)s->tmask[q] + 1, st);
+      gw::QueryView one = s->qv;
+      one.cursor += q;
       if (e == cudaSuccess)
-        e = gw::launch_walk_queries((int)p->rule, s->qv, s->prefix[q], s->prefix[q + 1], ctx->view(), a,
-                                    ctx->d_status.as<uint32_t>(), 0, st);
+        e = gw::launch_walk_queries((int)p->rule, one, s->prefix[q], s->prefix[q + 1], ctx->view(), a, s->status, 0, st);
       if (e == cudaSuccess)
-        e = gw::launch_topk_segmented(s->qv, q, 1, k, s->d_ids->as<uint32_t>(), s->d_cnt->as<uint32_t>(),
-                                      s->d_segs->as<unsigned long long>(), s->seg_first.data(), s->seg_slots,
-                                      s->d_cand->as<unsigned long long>(), s->qv.full + n, nullptr, st);
+        e = gw::launch_topk_segmented(s->qv, q, 1, k, s->ids, s->cnt, s->d_seg_first, s->seg_first.data(), s->seg_slots,
+                                      s->d_cand->as<unsigned long long>(), s->seg_done, nullptr, st);
       if (s->seg_first[q + 1] - s->seg_first[q] > 1 && !gw::topk_is_few(&s->seg_first[q], 1, s->seg_slots, k)) ++*launches;
     }
     cudaEventRecord(ev[2], st);
@@ -240,42 +258,52 @@ extern "C" gw_status gw_ppr_run(gw_ctx* ctx, const gw_walk_params* params, const
   for (uint32_t q = 0; q < nq; ++q) which[q] = q;
   uint64_t factor = params->table_factor ? params->table_factor : 8;
   cudaStream_t st = ctx->stream;
-  GW_CUDA(ctx, ctx->d_q_visits.ensure(8), "visit counter");
-  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_q_visits.p, 0, 8, st), "visit counter");
-  cudaEvent_t ev[4];
-  for (auto& e : ev) cudaEventCreate(&e);
+  cudaEvent_t* const ev = ctx->q_events;
+  for (int i = 0; i < 4; ++i)
+    if (!ev[i]) GW_CUDA(ctx, cudaEventCreate(&ev[i]), "event");
   gw_ppr_stats local{};
   local.walks = total;
-  std::vector<uint32_t> full, hid, hcnt;
+  std::vector<uint32_t> lists;
   for (int round = 0; round <= kMaxRetries && !which.empty(); ++round) {
     QuerySet set(ctx, round == 0);
     s = plan_set(ctx, sources, budgets, ids.data(), which, factor, &set);
     const bool b = batched || round > 0;
     if (s == GW_OK) s = upload_set(ctx, &set, k, st, b);
     if (s != GW_OK) break;
-    set.qv.visits = ctx->d_q_visits.as<unsigned long long>();
     set.qv.chunk = ctx->ppr_chunk;
     cudaError_t e = run_set(ctx, params, a, &set, k, b, b ? ctx->ppr_threads_per_sm : 0, st, ev, &local.launches);
     const uint32_t n = (uint32_t)which.size();
-    // The first round holds every query in the caller's order: its lists go
+    const size_t nk = (size_t)n * k;
+    // The first round holds every query in the caller's order: long lists go
     // straight into the caller's arrays (a rerun query's rows are overwritten
-    // later); a rerun's lists go through host staging to their rows.
-    const bool direct = round == 0;
-    full.resize(n);
-    if (!direct) {
-      hid.resize((size_t)n * k);
-      hcnt.resize((size_t)n * k);
+    // later); short ones and a rerun's go through host memory to their rows.
+    const bool staged = 2 * nk * 4 <= kStagedListBytes, direct = round == 0 && !staged;
+    char* const back = ctx->h_q_stage.as<char>() + set.back_at;
+    const size_t head = sizeof(Results) + (size_t)n * 4;
+    uint32_t* hid = topk_ids;
+    uint32_t* hcnt = topk_counts;
+    if (staged) {
+      hid = reinterpret_cast<uint32_t*>(back + head);
+      hcnt = hid + nk;
+    } else if (!direct) {
+      lists.resize(2 * nk);
+      hid = lists.data();
+      hcnt = hid + nk;
     }
-    uint32_t* ids_out = direct ? topk_ids : hid.data();
-    uint32_t* cnt_out = direct ? topk_counts : hcnt.data();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(full.data(), set.d_full->p, n * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ids_out, set.d_ids->p, (size_t)n * k * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt_out, set.d_cnt->p, (size_t)n * k * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(back, set.d_stage->as<char>() + set.back_at, head + (staged ? 2 * nk * 4 : 0),
+                          cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && !staged) e = cudaMemcpyAsync(hid, set.ids, nk * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && !staged) e = cudaMemcpyAsync(hcnt, set.cnt, nk * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
       s = ctx->cuda_fail(e, "gw_ppr_run");
       break;
     }
-    s = gw::take_status(ctx, st);
+    const Results* const res = reinterpret_cast<const Results*>(back);
+    const uint32_t* const full = reinterpret_cast<const uint32_t*>(res + 1);
+    local.visits += res->visits;
+    s = gw::status_of(ctx, res->status);
     if (s != GW_OK) break;
     if (round == 0 && b) {
       local.ms_clear = elapsed(ev[0], ev[1]);
@@ -292,15 +320,12 @@ extern "C" gw_status gw_ppr_run(gw_ctx* ctx, const gw_walk_params* params, const
         continue;
       }
       if (direct) continue;
-      std::copy(hid.begin() + (size_t)i * k, hid.begin() + (size_t)(i + 1) * k, topk_ids + (size_t)q * k);
-      std::copy(hcnt.begin() + (size_t)i * k, hcnt.begin() + (size_t)(i + 1) * k, topk_counts + (size_t)q * k);
+      std::copy(hid + (size_t)i * k, hid + (size_t)(i + 1) * k, topk_ids + (size_t)q * k);
+      std::copy(hcnt + (size_t)i * k, hcnt + (size_t)(i + 1) * k, topk_counts + (size_t)q * k);
     }
     which.swap(again);
     factor *= 4;
   }
-  for (auto& x : ev) cudaEventDestroy(x);
-  unsigned long long nvis = 0;
-  if (cudaMemcpy(&nvis, ctx->d_q_visits.p, 8, cudaMemcpyDeviceToHost) == cudaSuccess) local.visits = nvis;
   if (s == GW_OK && !which.empty())
     s = ctx->fail(GW_E_OVERFLOW, "%zu queries still filled their visit tables after %d retries",
                   which.size(), kMaxRetries);
@@ -355,6 +380,7 @@ extern "C" gw_status gw_ppr_autotune(gw_ctx* ctx, const gw_walk_params* params, 
       for (int rep = 0; rep < 3; ++rep) {
         bool cleared = false;
         if (assign_tag(ctx, &set, st, &cleared) != cudaSuccess) break;
+        cudaMemsetAsync(set.qv.cursor, 0, sizeof(unsigned long long), st);
         cudaEventRecord(e0, st);
         gw::launch_walk_queries((int)params->rule, set.qv, 0, set.walks, ctx->view(), a,
                                 ctx->d_status.as<uint32_t>(), c, st);

@@ -131,7 +131,7 @@ struct gw_server {
 namespace {
 
 // Staging layout for up to n queries in one superstep: the launch's chunk
-// cursor; the per-query inputs (copied up), with the pieces of the tables to
+// cursor and the per-query inputs (copied up), with the pieces of the tables to
 // clear and the top-k segments; then the results, one contiguous range copied
 // back: the launch's status word, the table-full flags and the top-k lists.
 // The segment counters, the status word and the flags are also copied up, as
@@ -279,8 +279,9 @@ bool superstep(gw_server* srv) {
   const uint32_t seg_slots = gw::topk_segment_slots(h.tmask, nfin);
   gw::topk_segment_prefix(h.tmask, nfin, seg_slots, h.seg_first);
   h.status[0] = 0;
-  const size_t head = stage_bytes(n, k) - 8 - 2 * (size_t)n * k * 4;  // prefix .. full
-  cudaError_t e = cudaMemcpyAsync(d.prefix, h.prefix, head, cudaMemcpyHostToDevice, st);
+  *h.cursor = 0;
+  const size_t head = stage_bytes(n, k) - 2 * (size_t)n * k * 4;  // cursor .. full
+  cudaError_t e = cudaMemcpyAsync(d.cursor, h.cursor, head, cudaMemcpyHostToDevice, st);
   gw::QueryView qv = make_view(d, srv->tables.as<unsigned long long>(), n);
   qv.chunk = ctx->ppr_chunk;
   if (e == cudaSuccess) e = gw::launch_clear_queries(qv, d.clear_first, pieces, st);
