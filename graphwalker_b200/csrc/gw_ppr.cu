@@ -50,12 +50,13 @@ __device__ __forceinline__ uint32_t slot_hash(uint32_t v) {  // MurmurHash3 fmix
   return v;
 }
 
-// Slot operations.  The add carries an L2 eviction policy (the tables of the
-// queries in flight should stay in L2 while the graph streams through it);
-// the compare-and-swap form of atom takes none, so a slot's line is first
-// touched by a prefetch marked evict_last (prefetch_slot).
-__device__ __forceinline__ void prefetch_slot(const unsigned long long* a) {
-  asm volatile("prefetch.global.L2::evict_last [%0];" ::"l"(a));
+// Slot operations.  The load and the add carry an L2 eviction policy: the
+// tables of the queries in flight should stay in L2 while the graph streams
+// through it (the compare-and-swap form of atom takes none).
+__device__ __forceinline__ unsigned long long load_slot(const unsigned long long* a, uint64_t pol) {
+  unsigned long long r;
+  asm volatile("ld.relaxed.gpu.global.L2::cache_hint.b64 %0, [%1], %2;" : "=l"(r) : "l"(a), "l"(pol) : "memory");
+  return r;
 }
 
 __device__ __forceinline__ unsigned long long cas_u64(unsigned long long* a, unsigned long long cmp,
@@ -76,43 +77,64 @@ __device__ __forceinline__ bool slot_free(unsigned long long old, uint32_t tag, 
   return old == kEmptySlot || ((uint32_t)(old >> 32) & tag_mask) != tag;
 }
 
-// Completes a table update of n visits under key = tag | v whose first probe
-// (a CAS of the empty pattern at slot s) returned `old`: nothing to do if the
-// CAS claimed the slot, an add if the slot holds the key; a slot left by an
-// earlier batch is claimed by a second CAS against its content (within a
-// batch only current keys are written, so a slot is resolved in at most two
-// CAS); otherwise linear probing from s + 1.  False when the table is full
-// (no free slot or slot holding the key within kMaxProbes of s).
-__device__ __forceinline__ bool table_finish(unsigned long long* __restrict__ t, uint32_t mask, uint32_t s,
-                                             unsigned long long old, uint32_t key, uint32_t n, uint64_t pol,
-                                             uint32_t tag_mask) {
-  const unsigned long long val = ((unsigned long long)key << 32) | n;
-  unsigned long long cmp = kEmptySlot;
-  const uint32_t last = probe_limit(mask);
-  for (uint32_t probe = 0;;) {
-    if (old == cmp) return true;
-    if ((uint32_t)(old >> 32) == key) {
-      red_add_u64(t + s, n, pol);
-      return true;
-    }
-    if (slot_free(old, key & tag_mask, tag_mask)) {
-      cmp = old;
-      old = cas_u64(t + s, cmp, val);
-      continue;
-    }
-    if (++probe > last) return false;
-    s = (s + 1) & mask;
-    cmp = kEmptySlot;
-    old = cas_u64(t + s, cmp, val);
-  }
+// Where v's probes in query q's table start.
+__device__ __forceinline__ unsigned long long* first_slot(const QueryView& qv, uint32_t q, uint32_t v) {
+  return qv.tables + __ldg(qv.table_off + q) + (slot_hash(v) & __ldg(qv.table_mask + q));
 }
 
-// Adds n visits under key = tag | v to a table; false when the table is full.
-__device__ __forceinline__ bool table_add(unsigned long long* __restrict__ t, uint32_t mask, uint32_t key,
-                                          uint32_t n, uint64_t pol, uint32_t tag_mask) {
-  const uint32_t s = slot_hash(key & ~tag_mask) & mask;
-  return table_finish(t, mask, s, cas_u64(t + s, kEmptySlot, ((unsigned long long)key << 32) | n), key, n, pol,
-                      tag_mask);
+// R table updates per lane, side by side: update r adds n[r] visits (0: none)
+// under tag | v[r] to query q[r]'s table, whose first slot was loaded as
+// seen[r].  Every round acts on each update's slot as it was last seen: an add
+// if it holds the key (keys stay once written), a CAS of the seen content if it
+// is free or left by an earlier batch, else the next slot is loaded (linear
+// probing); the rounds of the R updates overlap.  Loading a slot first costs an
+// atomic only where the slot changes: a CAS of the empty pattern as the first
+// probe failed on every known key and every earlier batch's slot, so nearly
+// every visit took two atomics.  A table without a free slot or the key within
+// kMaxProbes is reported full.
+template <int R>
+__device__ __forceinline__ void table_updates(const QueryView& qv, const uint32_t (&q)[R], const uint32_t (&v)[R],
+                                              uint32_t (&n)[R], unsigned long long (&seen)[R], uint64_t pol) {
+  unsigned long long* at[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) at[r] = n[r] ? first_slot(qv, q[r], v[r]) : nullptr;
+  for (;;) {
+    unsigned long long got[R];
+    bool tried[R];  // a CAS was issued
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      tried[r] = false;
+      got[r] = 0;
+      if (n[r]) {
+        const uint32_t key = qv.tag | v[r];
+        if ((uint32_t)(seen[r] >> 32) == key) {
+          red_add_u64(at[r], n[r], pol);
+          n[r] = 0;
+        } else if (slot_free(seen[r], qv.tag, qv.tag_mask)) {
+          tried[r] = true;
+          got[r] = cas_u64(at[r], seen[r], ((unsigned long long)key << 32) | n[r]);
+        } else {
+          unsigned long long* const t = qv.tables + __ldg(qv.table_off + q[r]);
+          const uint32_t mask = __ldg(qv.table_mask + q[r]), slot = (uint32_t)(at[r] - t);
+          if (((slot - slot_hash(v[r])) & mask) >= probe_limit(mask)) {
+            qv.full[q[r]] = 1u;
+            n[r] = 0;
+          } else {
+            at[r] = t + ((slot + 1) & mask);
+            got[r] = load_slot(at[r], pol);
+          }
+        }
+      }
+    }
+    uint32_t left = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (tried[r] && got[r] == seen[r]) n[r] = 0;
+      seen[r] = got[r];  // another lane's claim, or the next slot
+      left |= n[r];
+    }
+    if (!left) break;
+  }
 }
 
 __device__ __forceinline__ uint32_t query_of(const unsigned long long* __restrict__ prefix, uint32_t nq,
@@ -126,12 +148,36 @@ __device__ __forceinline__ uint32_t query_of(const unsigned long long* __restric
   return lo;
 }
 
-template <int RULE, bool ER>
-__global__ void __launch_bounds__(kPprThreads)
+// One walk per lane.  A visit's table update is a chain of its own (the slot,
+// then a CAS or more probes), and in a warp of 32 visits some lane always has a
+// long one, so the hop does not wait for it:
+//
+//  * SMALL = false, launches that fill the GPU, which the random line fills and
+//    the tables' requests bound: the slot is loaded at a visit and acted on at
+//    the lane's next one, behind that visit's gather.
+//  * SMALL = true, launches of few walks, which the chain of hops bounds: visits
+//    go to a queue in shared memory, worked off kFlush at a time, kPerLane per
+//    lane side by side, behind a gather; the draws of the next hop are computed
+//    while this one's gather is in flight, so a hop's own chain is the gather,
+//    a modulo and the next address.  (It holds visits back, so the tables of
+//    more queries are open at once: 16.5 ms where the other takes 11.6 on 4096
+//    queries.)
+//
+// Measured on B200 (walk kernel alone): 4096 queries, 59 M walks, R-MAT scale
+// 24: 14.0 ms when a CAS was the first probe and the hop waited for it, 11.6
+// now (33 G visits/s); one query of 100,000 walks at scale 20: 65 -> 60 us; one
+// of 300 walks at scale 22: 55 -> 33 us (42 with SMALL = false).
+template <int RULE, bool ER, bool SMALL>
+__global__ void __launch_bounds__(kPprThreads, SMALL ? 4 : 1)
     walk_query_kernel(QueryView qv, unsigned long long w_begin, unsigned long long w_end, GraphView g,
                       WalkArgs a, uint32_t* __restrict__ status) {
+  constexpr int kPerLane = 2;
+  constexpr uint32_t kFlush = 32 * kPerLane;
+  __shared__ uint2 queues[SMALL ? kPprThreads / 32 : 1][kFlush + 32];  // (query, vertex)
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1u;  // lanes under this one
+  uint2* const queue = queues[SMALL ? threadIdx.x >> 5 : 0];
+  uint32_t queued = 0;  // warp-uniform
   const unsigned long long total = w_end - w_begin;
   const unsigned long long chunk = qv.chunk ? qv.chunk : kWarpChunk;
   const L2Hints hp = make_hints(a.hints);
@@ -145,8 +191,33 @@ __global__ void __launch_bounds__(kPprThreads)
   unsigned long long j = 0, id_shift = 0, q_lo = 1, q_hi = 0;
   unsigned long long cur_rec = 0, src_rec = 0;  // edge-record mode: records of v and of the source
   uint32_t q = 0, src = 0, sid = 0, v = 0, hop = 0, st = 0, nvisit = 0;
+  Draws dr{0, 0};
   DrawCache dc;
   dc.reset();
+  // The queue's last `count` entries; equal (query, vertex) of a row of 32
+  // fold into one update.
+  auto flush = [&](uint32_t count) {
+    __syncwarp();
+    uint32_t fq[kPerLane], fv[kPerLane], fn[kPerLane];
+    unsigned long long seen[kPerLane];
+#pragma unroll
+    for (int r = 0; r < kPerLane; ++r) {
+      const uint32_t x = r * 32 + lane;
+      const bool in = x < count;
+      const uint2 e = in ? queue[queued - count + x] : make_uint2(0xffffffffu, lane);
+      fq[r] = e.x;
+      fv[r] = e.y;
+      const uint32_t peers = __match_any_sync(~0u, ((unsigned long long)e.x << 32) | e.y);
+      fn[r] = in && (peers & below) == 0 ? (uint32_t)__popc(peers) : 0u;
+      seen[r] = fn[r] ? load_slot(first_slot(qv, fq[r], fv[r]), hp.cnt) : 0ull;
+    }
+    queued -= count;
+    table_updates<kPerLane>(qv, fq, fv, fn, seen, hp.cnt);
+    __syncwarp();
+  };
+  // The lane's update in flight (SMALL = false).
+  uint32_t p_q[1] = {0}, p_v[1] = {0}, p_n[1] = {0};
+  unsigned long long p_seen[1] = {0};
   for (;;) {
     // Idle lanes take the next walks of the warp's chunk, in lane order.
     uint32_t idle = __ballot_sync(~0u, !busy);
@@ -177,62 +248,57 @@ __global__ void __launch_bounds__(kPprThreads)
           if (ER) src_rec = vertex_rec(g, hp, src);
         }
         const unsigned long long lo = q_lo > w_begin ? q_lo : w_begin, hi = q_hi < w_end ? q_hi : w_end;
-        if (visits_source && j == lo && src < g.nv &&
-            !table_add(qv.tables + __ldg(qv.table_off + q), __ldg(qv.table_mask + q), qv.tag | src,
-                       (uint32_t)(hi - lo), hp.cnt, qv.tag_mask))
-          qv.full[q] = 1u;
+        if (visits_source && j == lo && src < g.nv) {
+          const uint32_t uq[1] = {q}, uv[1] = {src};
+          uint32_t un[1] = {(uint32_t)(hi - lo)};
+          unsigned long long seen[1] = {load_slot(first_slot(qv, q, src), hp.cnt)};
+          table_updates<1>(qv, uq, uv, un, seen, hp.cnt);
+        }
         v = src;
         cur_rec = src_rec;
         hop = 0;
         dc.reset();
+        if (SMALL) dr = hop_draws(a, (uint32_t)(j + id_shift), 0u, sid, dc);
       }
       const uint32_t n_idle = __popc(idle);
       c_next += n_idle < avail ? n_idle : avail;
       idle = __ballot_sync(~0u, !busy);
     }
     if (!__any_sync(~0u, busy)) break;
-    if (!busy) continue;
-    bool end;
-    if (rule_capped<RULE>() && hop >= a.L) {
-      end = true;
-    } else if (RULE == GW_RULE_PROB && hop >= a.max_hops) {
-      st |= kStHops;
-      end = true;
-    } else if (v >= g.nv) {
-      st |= kStBounds;
-      end = true;
-    } else {
-      // the move after a walk's last visit is never observed: skipped
-      const bool last = last_visit<RULE>(a, hop);
-      const unsigned long long rec = (ER || last) ? cur_rec : ld_nc_u64(g.vrec + v, hp.rec);
+    bool visits = false, end = true;
+    if (busy) {
+      if (rule_capped<RULE>() && hop >= a.L) {
+      } else if (RULE == GW_RULE_PROB && hop >= a.max_hops) {
+        st |= kStHops;
+      } else if (v >= g.nv) {
+        st |= kStBounds;
+      } else {
+        visits = true;
+      }
+    }
+    const uint32_t pushes = SMALL ? __ballot_sync(~0u, visits && hop > 0) : 0u;
+    if (visits) {
       ++nvisit;
-      // Table update for hops >= 1: lanes visiting the same (query, vertex)
-      // fold into one; its first probe (a CAS) is issued now and resolved
-      // only after this hop's column load is in flight.
-      bool leader = false;
-      uint32_t n = 0, s0 = 0, mask = 0;
-      unsigned long long old = kEmptySlot, *t = nullptr;
-      if (hop > 0) {
-        const unsigned active = __activemask();
-        const unsigned peers = __match_any_sync(active, ((unsigned long long)q << 32) | v);
-        leader = lane == (uint32_t)__ffs(peers) - 1;
-        if (leader) {
-          n = (uint32_t)__popc(peers);
-          t = qv.tables + __ldg(qv.table_off + q);
-          mask = __ldg(qv.table_mask + q);
-          s0 = slot_hash(v) & mask;
-          prefetch_slot(t + s0);  // keeps the table's lines in L2 ahead of the graph's (walk phase -34 %)
-          old = cas_u64(t + s0, kEmptySlot, ((unsigned long long)(qv.tag | v) << 32) | n);
+      uint32_t u_n = 0;  // SMALL = false: this visit's update, if the lane makes it
+      const uint32_t u_v = v;
+      unsigned long long u_seen = 0;
+      if (SMALL) {
+        if (hop > 0) queue[queued + __popc(pushes & below)] = make_uint2(q, v);
+      } else if (hop > 0) {
+        // lanes visiting the same (query, vertex) fold into one
+        const uint32_t peers = __match_any_sync(__activemask(), ((unsigned long long)q << 32) | v);
+        if ((peers & below) == 0) {
+          u_n = (uint32_t)__popc(peers);
+          u_seen = load_slot(first_slot(qv, q, v), hp.cnt);
         }
       }
-      // the hop itself: hop_advance_rec's draws and choices, written out so
-      // the table update above can complete after the column load is issued
-      uint32_t next = v;
-      unsigned long long next_rec = 0;
-      bool moved = !last;
-      if (!last) {
-        const Draws dr = hop_draws(a, (uint32_t)(j + id_shift), hop, sid, dc);
+      // the move after a walk's last visit is never observed: skipped
+      if (!last_visit<RULE>(a, hop)) {
+        // hop_advance_rec's choices on this hop's draws
+        const unsigned long long rec = ER ? cur_rec : ld_nc_u64(g.vrec + v, hp.rec);
+        if (!SMALL) dr = hop_draws(a, (uint32_t)(j + id_shift), hop, sid, dc);
         const uint32_t d0 = dr.d0, d1 = dr.d1;
+        bool moved = true;
         unsigned long long off = rec >> kDegBits, deg = rec & kDegEscape;
         if (deg == kDegEscape) {
           off = __ldg(g.rowptr + v);
@@ -243,35 +309,45 @@ __global__ void __launch_bounds__(kPprThreads)
               deg > 0x7fffffffull ? (unsigned long long)d1 : (unsigned long long)(d1 % (uint32_t)deg);
           if (ER) {
             const ulonglong2 e = ld_nc_u64x2(g.erec + off + r, hp.col);
-            next = (uint32_t)e.y;
-            next_rec = e.x;
+            v = (uint32_t)e.y;
+            cur_rec = e.x;
           } else {
-            next = ld_nc_u32(g.colidx + off + r, hp.col);
+            v = ld_nc_u32(g.colidx + off + r, hp.col);
           }
         } else {
           const uint32_t dj = deg > 0 ? d1 : d0;
           if (RULE == GW_RULE_JUMP) {
-            next = dj % a.njump;
-            if (ER) next_rec = jump_rec(g, hp, next);
+            v = dj % a.njump;
+            if (ER) cur_rec = jump_rec(g, hp, v);
           } else if (RULE == GW_RULE_RESTART || (RULE == GW_RULE_PPR && deg == 0)) {
-            next = src;
-            next_rec = src_rec;
+            v = src;
+            cur_rec = src_rec;
           } else {
             moved = false;
           }
         }
+        if (moved) {
+          ++hop;
+          end = RULE == GW_RULE_RESTART && hop % a.L == a.L - 1;
+          if (SMALL && !end && !last_visit<RULE>(a, hop)) dr = hop_draws(a, (uint32_t)(j + id_shift), hop, sid, dc);
+        }
       }
-      if (leader && !table_finish(t, mask, s0, old, qv.tag | v, n, hp.cnt, qv.tag_mask)) qv.full[q] = 1u;
-      end = !moved;
-      if (moved) {
-        v = next;
-        cur_rec = next_rec;
-        ++hop;
-        if (RULE == GW_RULE_RESTART && hop % a.L == a.L - 1) end = true;
+      if (!SMALL) {
+        if (p_n[0]) table_updates<1>(qv, p_q, p_v, p_n, p_seen, hp.cnt);
+        p_q[0] = q;
+        p_v[0] = u_v;
+        p_n[0] = u_n;
+        p_seen[0] = u_seen;
       }
     }
     if (end) busy = false;
+    if (SMALL) {
+      queued += __popc(pushes);
+      if (queued >= kFlush) flush(kFlush);
+    }
   }
+  if (SMALL && queued) flush(queued);
+  if (!SMALL && p_n[0]) table_updates<1>(qv, p_q, p_v, p_n, p_seen, hp.cnt);
   if (st) atomicOr(status, st);
   if (qv.visits) {
     const unsigned long long w = __reduce_add_sync(~0u, nvisit);
@@ -739,17 +815,24 @@ int sm_count() {
   return sms;
 }
 
+// Launches up to this many walks run the SMALL kernel: one CTA per SM.  Scales
+// 20 and 22, one query: 3000 walks 41 us against 49, 20,000 42.5 against 46.5,
+// 37,000 45 against 48, 60,000 54 against 53, 100,000 76 against 60.
+constexpr unsigned long long kSmallLaunch = 148 * kPprThreads;
+
 template <int RULE>
 cudaError_t query_dispatch(const QueryView& qv, unsigned long long w_begin, unsigned long long w_end,
                            const GraphView& g, const WalkArgs& a, uint32_t* status, int threads_per_sm,
                            cudaStream_t stream) {
-  auto kern = g.erec ? walk_query_kernel<RULE, true> : walk_query_kernel<RULE, false>;
+  const unsigned long long n = w_end - w_begin;
+  const bool small = n <= kSmallLaunch;
+  auto kern = g.erec ? (small ? walk_query_kernel<RULE, true, true> : walk_query_kernel<RULE, true, false>)
+                     : (small ? walk_query_kernel<RULE, false, true> : walk_query_kernel<RULE, false, false>);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPprThreads, 0);
   const int sms = sm_count();
   if (per_sm <= 0) per_sm = 1;
   if (threads_per_sm > 0) per_sm = std::max(1, std::min(per_sm, threads_per_sm / kPprThreads));
-  const unsigned long long n = w_end - w_begin;
   const unsigned long long need = (n + kPprThreads - 1) / kPprThreads;
   const unsigned long long full = (unsigned long long)sms * per_sm;
   const int grid = (int)(need < full ? (need ? need : 1) : full);

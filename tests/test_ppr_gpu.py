@@ -245,3 +245,32 @@ def test_topk_at_table_sizes(cuda_device, oracle, budgets, k):
         v = np.nonzero(r["counts"])[0] if b[q] else np.zeros(0, np.int64)
         want = _topk_ref(dict(zip(v.tolist(), r["counts"][v].tolist())), k)
         assert np.array_equal(got[0][0][q], want[0]) and np.array_equal(got[0][1][q], want[1]), q
+
+
+@pytest.mark.parametrize("walks", [37_887, 37_888, 37_889, 120_000])
+@pytest.mark.parametrize("rule,layout", [(4, 1), (0, 1), (3, 0)])
+def test_walk_launches_around_the_small_limit(cuda_device, oracle, walks, rule, layout):
+    """One query and several whose walks sum to one short of, exactly and past
+    the launch size (148 x 256) up to which visits are queued in shared memory;
+    all lists equal the oracle's counts.  Sources of low degree make their
+    first visits collide."""
+    import graphwalker_b200 as gw
+    rp, ci = oracle.rmat_csr(14, 8, seed=2)
+    deg = np.diff(rp.astype(np.int64))
+    few = np.nonzero((deg > 0) & (deg < 4))[0]
+    L, k = 7, 100
+    with gw.Graph.from_csr(rp, ci, oracle.compute_blocks(rp, 256)) as G:
+        G.set_edge_records(layout)
+        p = gw.params(rule, gw.SINK_NONE, L, seed=6)
+        for budgets in ([walks], [5, walks - 1005, 1000]):
+            src = few[: len(budgets)].astype(np.uint32)
+            ids, cnt, st = G.ppr(p, src, np.array(budgets, np.uint32), k=k)
+            first = 0
+            for q, b in enumerate(budgets):
+                cur = np.full(b, src[q], np.uint32)
+                r = oracle.run_walks(rp, ci, cur, ids=np.arange(first, first + b, dtype=np.uint32), src=cur, rule=rule,
+                                     L=L, seed=6)
+                v = np.nonzero(r["counts"])[0]
+                want = _topk_ref(dict(zip(v.tolist(), r["counts"][v].tolist())), k)
+                assert np.array_equal(ids[q], want[0]) and np.array_equal(cnt[q], want[1]), (q, b)
+                first += b
