@@ -70,6 +70,8 @@ gw_status init_ctx(gw_ctx* ctx, int device) {
   GW_CUDA(ctx, cudaMemsetAsync(ctx->d_status.p, 0, sizeof(uint32_t), ctx->stream), "memset");
   const char* env = getenv("GW_EDGE_RECORDS");
   ctx->erec_mode = env && strcmp(env, "0") == 0 ? GW_EDGE_RECORDS_OFF : GW_EDGE_RECORDS_AUTO;
+  // GW_CSR_WALK_BYTES: tests run the edge-record kernels on small graphs with 0
+  if (const char* limit = getenv("GW_CSR_WALK_BYTES")) ctx->csr_walk_limit = strtoull(limit, nullptr, 10);
   return GW_OK;
 }
 
@@ -234,7 +236,7 @@ bool fault_now(uint32_t kind) {
 gw_status thread_error(gw_status code, const std::string& msg) { return set_thread_error(code, msg); }
 
 // Grid of a resident walk launch over n walks: the autotuned CTAs per SM
-// (gw_walk_autotune), or 0 for the kernel's full occupancy.
+// (gw_walk_autotune), or 0 for the launch's default shape.
 int resident_grid(gw_ctx* ctx, uint64_t n) {
   if (ctx->walk_ctas_per_sm <= 0) return 0;
   int sms = 148;
@@ -1026,7 +1028,7 @@ gw_status gw_walk_autotune(gw_ctx* ctx, const gw_walk_params* params, const gw_w
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  ctx->walk_ctas_per_sm = best == max_per_sm ? 0 : best;  // full occupancy is the default shape
+  ctx->walk_ctas_per_sm = best;
   if (ctas_per_sm) *ctas_per_sm = (uint32_t)best;
   return gw::take_status(ctx, st);
 }

@@ -91,6 +91,9 @@ struct gw_ctx {
   gw_devbuf d_exact;                    // gw_expected_visits' workspace
   gw_devbuf d_meet, d_sr_rows;          // SimRank meeting counts, per-query path rows
   uint32_t erec_mode = GW_EDGE_RECORDS_AUTO;
+  // Resident walks read the plain CSR, not the edge records, while it is at
+  // most this large, or half of it (gw_walk.cu: walks_use_records).
+  uint64_t csr_walk_limit = 640ull << 20;
   gw_hostbuf h_rowptr, h_colidx;  // pinned copy (streaming residency)
 
   // device status word (+ pinned mirror)
@@ -223,6 +226,8 @@ struct gw_ctx {
     g.colidx = d_colidx.as<const uint32_t>();
     g.erec = d_erec.p && d_erec.bytes >= ne * sizeof(ulonglong2) ? d_erec.as<const ulonglong2>() : nullptr;
     g.out_bits = d_vrec.p && d_vrec.bytes >= gw::vrec_bytes(nv) ? reinterpret_cast<const uint32_t*>(g.vrec + nv) : nullptr;
+    g.csr_bytes = ne * sizeof(uint32_t) + (uint64_t)nv * 8;
+    g.csr_limit = csr_walk_limit;
     g.nv = nv;
     return g;
   }

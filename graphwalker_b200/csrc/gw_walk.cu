@@ -10,7 +10,11 @@
 // one 8-byte packed vertex record load, one 4-byte column load, one Philox
 // block computed while the record load is in flight, and one visit atomic.
 // With edge records (ER) the record of the current vertex is carried from the
-// previous hop, so a hop along an edge is a single 16-byte gather.
+// previous hop, so a hop along an edge is a single 16-byte gather; graphs of a
+// few L2 sizes are walked over the plain layout all the same
+// (walks_use_records).
+#include <algorithm>
+
 #include "gw_internal.h"
 
 namespace gw {
@@ -401,21 +405,67 @@ int num_sms() {
 }
 
 template <typename K>
-int occupancy_grid(K kernel, uint64_t n) {
+int ctas_per_sm(K kernel) {
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWalkThreads, 0);
-  if (per_sm <= 0) per_sm = 1;
+  return per_sm > 0 ? per_sm : 1;
+}
+
+int grid_of(int per_sm, uint64_t n) {
   const uint64_t full = (uint64_t)num_sms() * per_sm;
   const uint64_t need = (n + kWalkThreads - 1) / kWalkThreads;
   return (int)(need < full ? (need > 0 ? need : 1) : full);
+}
+
+// Whether n resident walks over g read its edge records.  A move along an edge
+// record is one gather where the CSR takes two, but the records are four times
+// the columns, and a jump over them waits for a bitmap word, the target's
+// record and its edge in turn, in a warp whose other lanes wait for theirs.  So
+// jumping walks on graphs of a few L2 sizes read the CSR, and so do large sets
+// of the rules that end at a failed test (records / CSR, us, warm, random
+// starts, edge factor 16):
+//   jump: 4099 walks at scale 14 17.4 / 11.3 a call; 1 M at 20 169 / 147, at 21
+//     199 / 145; 4 M at 22 850 / 702 and at 23 (603 MB) 911 / 904, recording
+//     paths 819 / 793; one walk per vertex at 24 3742 / 4222;
+//   stop, uncapped: 1 M at 21 86 / 72 and 85 / 80; 4 M at 22 (301 MB) 357 / 323
+//     and 468 / 411, at 23 379 / 377 and 471 / 486; few walks 11.3 / 12.7 (8310
+//     at 18), 48.5 / 53.7 (39 k at 21): a chain of hops with two gathers each;
+//   PPR, restart: their walks go back to a source whose record they hold (PPR:
+//     1 M at 20 148 / 162, 4 M at 22 560 / 656; restart: 127 / 122, 513 / 534).
+template <int RULE>
+bool walks_use_records(const GraphView& g, uint64_t n) {
+  if (!g.erec) return false;
+  if (RULE == GW_RULE_JUMP) return g.csr_bytes > g.csr_limit;
+  return rule_returns<RULE>() || n < 1u << 19 || g.csr_bytes > g.csr_limit / 2;
+}
+
+// CTAs per SM of a resident launch that no autotuner shaped: all that fit,
+// except where fewer requests in flight queue less at the DRAM: jumps over
+// edge records (one walk per vertex at scale 24: 8 CTAs 4.02 ms, 6 3.81, 5 3.74,
+// 4 3.80; at 23 1749, 1684, 1684, 1714 us), and restarting walks that record
+// paths beyond a third of the L2, whose rows then fill before they are written
+// out (3 M at 22, 11 visits: 8 CTAs 352 us, 6 332; 2 M at 21, 20 visits: 1.08
+// times; under 40 MB 0.94 to 1.04 times).  The PPR rule, whose walks end early,
+// wants them all (24: 2.21 ms with 8, 2.83 with 5).
+template <int RULE, int SINK>
+int default_ctas_per_sm(bool records, uint64_t n, uint32_t path_stride) {
+  if (RULE == GW_RULE_JUMP && records) return 5;
+  if (RULE == GW_RULE_RESTART && SINK == GW_SINK_PATH_RECORD && n * path_stride * 4 >= 40u << 20) return 6;
+  return 1 << 16;
 }
 
 template <int RULE, int SINK, bool AGG>
 cudaError_t resident_dispatch(const gw_walk_rec* walks, uint64_t n, const GraphView& g,
                               const WalkArgs& a, const SinkView& s, uint32_t* status, int grid,
                               cudaStream_t stream, const cudaAccessPolicyWindow* window) {
-  auto k = g.erec ? walk_resident_kernel<RULE, SINK, AGG, true> : walk_resident_kernel<RULE, SINK, AGG, false>;
-  if (grid <= 0) grid = occupancy_grid(k, n);
+  const bool records = walks_use_records<RULE>(g, n);
+  auto k = records ? walk_resident_kernel<RULE, SINK, AGG, true> : walk_resident_kernel<RULE, SINK, AGG, false>;
+  if (grid <= 0) {
+    // a kernel's occupancy is asked for once: the call takes as long as a short launch
+    static const int fit[2] = {ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, false>),
+                               ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, true>)};
+    grid = grid_of(std::min(fit[records], default_ctas_per_sm<RULE, SINK>(records, n, a.path_stride)), n);
+  }
   if (!window) {
     k<<<grid, kWalkThreads, 0, stream>>>(walks, n, g, a, s, status);
     return cudaGetLastError();
@@ -435,9 +485,9 @@ cudaError_t resident_dispatch(const gw_walk_rec* walks, uint64_t n, const GraphV
 template <int RULE, int SINK, bool AGG>
 int resident_grid(uint64_t n) {
   // both variants have the same block shape; the larger register count bounds the grid
-  const int a = occupancy_grid(walk_resident_kernel<RULE, SINK, AGG, false>, n);
-  const int b = occupancy_grid(walk_resident_kernel<RULE, SINK, AGG, true>, n);
-  return a < b ? a : b;
+  return grid_of(std::min(ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, false>),
+                          ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, true>)),
+                 n);
 }
 
 template <int RULE, int SINK, bool AGG>
