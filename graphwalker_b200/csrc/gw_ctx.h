@@ -256,8 +256,8 @@ void pipe_release(gw_ctx* ctx);
 // the walk words cross the host link faster than their walks run, so the
 // chunks start small (the first kernel waits only for a short copy) and grow
 // by 7/4 each time, which keeps each copy shorter than the kernel it hides
-// behind (gw_run_pools, gw_run_pools_submit).
-std::vector<uint64_t> chunk_bounds(uint64_t n);
+// behind, up to `most` walks (gw_run_pools, gw_run_pools_submit).
+std::vector<uint64_t> chunk_bounds(uint64_t n, uint64_t most);
 }  // namespace gw
 
 #define GW_CUDA(ctx, expr, what)                    \

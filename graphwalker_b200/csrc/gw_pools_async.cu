@@ -36,9 +36,11 @@ cudaError_t pipe_init(gw_ctx* ctx) {
 
 }  // namespace
 
-std::vector<uint64_t> chunk_bounds(uint64_t n) {
+std::vector<uint64_t> chunk_bounds(uint64_t n, uint64_t most) {
   std::vector<uint64_t> lo{0};
-  for (uint64_t m = 1ull << 17; lo.back() < n; m += m * 3 / 4) lo.push_back(std::min(n, lo.back() + m));
+  most = std::max<uint64_t>(most, 1ull << 17);
+  for (uint64_t m = 1ull << 17; lo.back() < n; m = std::min(most, m + m * 3 / 4))
+    lo.push_back(std::min(n, lo.back() + m));
   return lo;
 }
 
@@ -90,7 +92,7 @@ extern "C" gw_status gw_run_pools_submit(gw_ctx* ctx, const gw_walk_params* para
   GW_CUDA(ctx, P.counts[s].ensure((size_t)ctx->nv * 4), "counts alloc");
   GW_CUDA(ctx, P.status[s].ensure(sizeof(uint32_t)), "status alloc");
 
-  const std::vector<uint64_t> lo = gw::chunk_bounds(n);
+  const std::vector<uint64_t> lo = gw::chunk_bounds(n, n);  // the next run's copies follow: no kernel is left alone
   const uint64_t nchunks = lo.size() - 1;
   cudaStream_t cs = ctx->stream, as = ctx->aux_stream, xs = ctx->copy_stream, rs = P.readback;
   uint32_t* d_counts = P.counts[s].as<uint32_t>();
