@@ -12,16 +12,20 @@
 // rule).  The neighbour choice is taken as exactly uniform; the walks'
 // r % deg has a bias below deg / 2^31.
 //
-// A hop is two kernels.  The vertex kernel finishes x (the pushes plus what the
-// last hop's else-branches owe the source and all vertices), adds it to the
-// visits, leaves each vertex's share per out-edge and sums the new debts.  The
-// edge kernel adds the shares at the targets: warps take equal runs of edges,
-// whatever their sources' degrees, so no warp is left with a hub: 154 us a hop
-// for 16.8 M edges at R-MAT scale 20, where a warp per vertex took 355.  What
-// bounds it is the L2's FP64 atomic rate, 109 G updates/s (32-bit ones: 190).
-// It is not the hottest target's address: pushes spread over 2 or 4 copies of
-// the targets gained 5 % and lost 11 %, and at scale 22, where the copies
-// outgrow the L2, cost 1.3 and 2.1 times.
+// A hop is two kernels.  The vertex kernel finishes x (what arrived over edges
+// plus what the last hop's else-branches owe the source and all vertices), adds
+// it to the visits, leaves each vertex's share per out-edge and sums the new
+// debts.  The edge kernel carries the shares to the targets, warps taking equal
+// runs of edges whatever their vertices' degrees, so no warp is left with a
+// hub: a warp per vertex took 355 us a hop at R-MAT scale 20 (16.8 M edges).
+//
+//  * Push: an FP64 atomic per edge, 154 us a hop there, the L2's rate of them
+//    (109 G/s; 32-bit ones: 190).  It is not the hottest target's address:
+//    pushes spread over 2 or 4 copies of the targets gained 5 % and lost 11 %.
+//  * Pull: over in-edges, so an edge is a gather (284 G/s from the L2) and only
+//    the end of a vertex's run of edges an atomic: 85 us a hop, after 385 us of
+//    turning the graph around, a counting sort by target.  Taken from kPullHops
+//    hops on (six pushes cost 924 us, six pulls 895).
 #include <algorithm>
 
 #include "gw_ctx.h"
@@ -105,12 +109,27 @@ __global__ void exact_runs_kernel(const unsigned long long* __restrict__ rowptr,
   }
 }
 
-// One warp per run of edges.  The lanes hold the row ends and shares of 32
-// consecutive vertices; a lane finds its edge's source among them by bisection.
+// The lane whose row holds edge e, when lane i's row ends at `end` (in lane
+// order) and e lies in one of them: the number of rows that end at or before e.
+__device__ __forceinline__ uint32_t row_of(uint32_t end, uint32_t e) {
+  uint32_t at = 0;
+#pragma unroll
+  for (uint32_t step = 16; step > 0; step >>= 1)
+    if (__shfl_sync(~0u, end, at + step - 1) <= e) at += step;
+  return at;
+}
+
+// One warp per run of edges of the rows `rowptr`, which are sources; the lanes
+// hold the row ends of 32 consecutive ones.  Push: a row's share is added at
+// each of its targets.  Turn: a row's source is written into each target's row
+// of the turned graph, whose next free place is place[target].  An edge to a
+// vertex past the last carries nothing.
+template <bool TURN>
 __global__ void __launch_bounds__(kExactThreads)
     exact_edge_kernel(const double* __restrict__ share, double* __restrict__ acc,
                       const unsigned long long* __restrict__ rowptr, const uint32_t* __restrict__ colidx, uint32_t nv,
-                      uint64_t ne, uint64_t nruns, uint32_t run, const uint32_t* __restrict__ first) {
+                      uint64_t ne, uint64_t nruns, uint32_t run, const uint32_t* __restrict__ first,
+                      uint32_t* __restrict__ place, uint32_t* __restrict__ turned) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= nruns) return;
@@ -124,29 +143,161 @@ __global__ void __launch_bounds__(kExactThreads)
     if (mine < nv) {
       const unsigned long long x = __ldg(rowptr + mine + 1) - e0;
       end = x < n ? (uint32_t)x : n;
-      sh = __ldg(share + mine);
+      if (!TURN) sh = __ldg(share + mine);
     }
     const uint32_t last = __shfl_sync(~0u, end, 31);  // edges these vertices reach to
-    const bool any = __any_sync(~0u, sh != 0.0);
+    const bool any = TURN || __any_sync(~0u, sh != 0.0);
     for (; any && done < last; done += 128) {
       uint32_t to[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t e = done + u * 32 + lane;
-        to[u] = e < last ? __ldg(colidx + e0 + e) : 0u;
+        to[u] = e < last ? __ldg(colidx + e0 + e) : nv;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const uint32_t e = done + u * 32 + lane;
-        uint32_t at = 0;  // lanes whose row ends at or before e
-#pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1)
-          if (__shfl_sync(~0u, end, at + step - 1) <= e) at += step;
-        const double s = __shfl_sync(~0u, sh, at);
-        if (e < last && s != 0.0) atomicAdd(acc + to[u], s);
+        const uint32_t at = row_of(end, done + u * 32 + lane);
+        const double s = TURN ? 0.0 : __shfl_sync(~0u, sh, at);
+        if (to[u] >= nv) continue;
+        if (TURN) turned[atomicAdd(place + to[u], 1u)] = v + at;
+        else if (s != 0.0) atomicAdd(acc + to[u], s);
       }
     }
     done = last;
+  }
+}
+
+// The same over the turned graph: rows are targets, turned[e] the source of
+// in-edge e.  A lane sums four consecutive edges; where they span rows it adds
+// all but the last row's part by itself, and the last parts of the lanes of one
+// row are summed in the warp and added by its first lane.
+__global__ void __launch_bounds__(kExactThreads)
+    exact_pull_kernel(const double* __restrict__ share, double* __restrict__ acc,
+                      const unsigned long long* __restrict__ rows, const uint32_t* __restrict__ turned, uint32_t nv,
+                      uint64_t ne, uint64_t nruns, uint32_t run, const uint32_t* __restrict__ first) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nruns) return;
+  const uint64_t e0 = c * run;
+  const uint32_t n = (uint32_t)(ne - e0 < run ? ne - e0 : run);
+  uint32_t v = __ldg(first + c);
+  for (uint32_t done = 0; done < n && v < nv; v += 32) {
+    const uint32_t mine = v + lane;
+    uint32_t end = n;
+    if (mine < nv) {
+      const unsigned long long x = __ldg(rows + mine + 1) - e0;
+      end = x < n ? (uint32_t)x : n;
+    }
+    const uint32_t last = __shfl_sync(~0u, end, 31);
+    for (; done < last; done += 128) {
+      const uint32_t e = done + lane * 4;
+      uint32_t src[4], at[4];
+      double got[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) src[u] = e + u < last ? __ldg(turned + e0 + e + u) : nv;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) got[u] = src[u] < nv ? __ldg(share + src[u]) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) at[u] = row_of(end, e + u);
+      double s = got[0];
+#pragma unroll
+      for (int u = 1; u < 4; ++u) {
+        if (at[u] != at[u - 1]) {
+          if (s != 0.0 && v + at[u - 1] < nv) atomicAdd(acc + v + at[u - 1], s);
+          s = 0.0;
+        }
+        s += got[u];
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_down_sync(~0u, s, o);
+        const uint32_t row = __shfl_down_sync(~0u, at[3], o);
+        if (lane + o < 32 && row == at[3]) s += x;
+      }
+      const uint32_t before = __shfl_up_sync(~0u, at[3], 1);
+      if ((lane == 0 || before != at[3]) && s != 0.0 && v + at[3] < nv) atomicAdd(acc + v + at[3], s);
+    }
+    done = last;
+  }
+}
+
+// In-degrees of the turned graph.
+__global__ void in_degree_kernel(const uint32_t* __restrict__ colidx, uint64_t ne, uint32_t nv,
+                                 uint32_t* __restrict__ deg) {
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (uint64_t)gridDim.x * blockDim.x)
+    if (const uint32_t to = __ldg(colidx + e); to < nv) atomicAdd(deg + to, 1u);
+}
+
+// Exclusive scan of the in-degrees, in three launches: every block's sum; the
+// sums, in one block; then rows[v] (where v's in-edges start) and place[v] (the
+// same, advanced by the turn; it holds the in-degrees before).
+constexpr uint32_t kScanItems = 4, kScanBlock = kExactThreads * kScanItems;
+
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long x, unsigned long long* warp_sums,
+                                                         unsigned long long* total) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long incl = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(~0u, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  unsigned long long below = 0, all = 0;
+  for (uint32_t w = 0; w < kExactThreads / 32; ++w) {
+    if (w < warp) below += warp_sums[w];
+    all += warp_sums[w];
+  }
+  __syncthreads();  // warp_sums may be written again
+  *total = all;
+  return below + incl - x;
+}
+
+__global__ void __launch_bounds__(kExactThreads)
+    scan_sums_kernel(const uint32_t* __restrict__ deg, uint32_t nv, unsigned long long* __restrict__ sums) {
+  __shared__ unsigned long long warp_sums[kExactThreads / 32];
+  const uint64_t v0 = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+  unsigned long long x = 0, all = 0;
+  for (uint32_t i = 0; i < kScanItems; ++i)
+    if (v0 + i < nv) x += deg[v0 + i];
+  block_scan(x, warp_sums, &all);
+  if (threadIdx.x == 0) sums[blockIdx.x] = all;
+}
+
+__global__ void __launch_bounds__(kExactThreads) scan_blocks_kernel(unsigned long long* __restrict__ sums, uint32_t n) {
+  __shared__ unsigned long long warp_sums[kExactThreads / 32];
+  unsigned long long carry = 0;
+  for (uint32_t b = 0; b < n; b += kExactThreads) {
+    const uint32_t i = b + threadIdx.x;
+    const unsigned long long x = i < n ? sums[i] : 0ull;
+    unsigned long long all = 0;
+    const unsigned long long before = block_scan(x, warp_sums, &all);
+    if (i < n) sums[i] = carry + before;
+    carry += all;
+  }
+}
+
+__global__ void __launch_bounds__(kExactThreads)
+    scan_rows_kernel(uint32_t* __restrict__ place, uint32_t nv, const unsigned long long* __restrict__ sums,
+                     unsigned long long* __restrict__ rows) {
+  __shared__ unsigned long long warp_sums[kExactThreads / 32];
+  const uint64_t v0 = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+  uint32_t d[kScanItems];
+  unsigned long long x = 0, all = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < kScanItems; ++i) {
+    d[i] = v0 + i < nv ? place[v0 + i] : 0u;
+    x += d[i];
+  }
+  unsigned long long at = sums[blockIdx.x] + block_scan(x, warp_sums, &all);
+#pragma unroll
+  for (uint32_t i = 0; i < kScanItems; ++i) {
+    if (v0 + i >= nv) break;
+    rows[v0 + i] = at;
+    place[v0 + i] = (uint32_t)at;
+    at += d[i];
+    if (v0 + i + 1 == nv) rows[nv] = at;
   }
 }
 
@@ -174,12 +325,27 @@ extern "C" gw_status gw_expected_visits(gw_ctx* ctx, const gw_walk_params* param
   const uint64_t ne = ctx->ne;
   const uint32_t run = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(ne / ((uint64_t)sms * 64) / 128 * 128, 128), 1024);
   const uint64_t nruns = (ne + run - 1) / run;
-  // One workspace: pushes, shares and visits (8 bytes a vertex each), the debt
-  // sets, and the runs' first vertices.  Kept in the context while it is small.
+  // One workspace: arrivals, shares and visits (8 bytes a vertex each), the debt
+  // sets, the turned graph's rows (8 bytes a vertex) and block sums, the runs'
+  // first vertices, and the turned graph's places (4 bytes a vertex) and sources
+  // (4 bytes an edge).  Kept in the context while it is small.
   constexpr size_t kKeptBytes = 256ull << 20;
-  const size_t debts_at = 3 * nv * 8, first_at = debts_at + gw::kSums * sizeof(gw::Debt);
-  const size_t bytes = first_at + nruns * 4;
-  GW_CUDA(ctx, ctx->d_exact.ensure(bytes), "alloc");
+  constexpr uint32_t kPullHops = 7;
+  bool pull = hops >= kPullHops && ne > 0 && ne < (1ull << 32);
+  const uint32_t nscan = (uint32_t)((nv + gw::kScanBlock - 1) / gw::kScanBlock);
+  const size_t debts_at = 3 * nv * 8, rows_at = debts_at + gw::kSums * sizeof(gw::Debt);
+  size_t first_at = 0, place_at = 0, turned_at = 0;
+  auto lay_out = [&] {
+    first_at = rows_at + (pull ? (nv + 1 + nscan) * 8 : 0);
+    place_at = first_at + nruns * 4;
+    turned_at = place_at + (pull ? nv * 4 : 0);
+    return turned_at + (pull ? ne * 4 : 0);
+  };
+  if (pull && ctx->d_exact.ensure(lay_out()) != cudaSuccess) {
+    cudaGetLastError();  // no room to turn the graph around: push
+    pull = false;
+  }
+  GW_CUDA(ctx, ctx->d_exact.ensure(lay_out()), "alloc");
   struct Release {
     gw_ctx* ctx;
     ~Release() {
@@ -196,21 +362,42 @@ extern "C" gw_status gw_expected_visits(gw_ctx* ctx, const gw_walk_params* param
   const double one = 1.0;
   GW_CUDA(ctx, cudaMemcpyAsync(acc + source, &one, 8, cudaMemcpyHostToDevice, st), "seed");
   const unsigned long long* rowptr = ctx->d_rowptr.as<unsigned long long>();
+  const uint32_t* const colidx = ctx->d_colidx.as<uint32_t>();
+  const unsigned egrid = (unsigned)((nruns * 32 + gw::kExactThreads - 1) / gw::kExactThreads);
+  const unsigned rgrid = (unsigned)std::min<uint64_t>((nruns + 255) / 256, (uint64_t)sms * 8);
+  auto* rows = reinterpret_cast<unsigned long long*>(ctx->d_exact.as<char>() + rows_at);
+  uint32_t* const turned = reinterpret_cast<uint32_t*>(ctx->d_exact.as<char>() + turned_at);
   if (nruns) {
-    gw::exact_runs_kernel<<<(unsigned)std::min<uint64_t>((nruns + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(
-        rowptr, ctx->nv, nruns, run, first);
+    gw::exact_runs_kernel<<<rgrid, 256, 0, st>>>(rowptr, ctx->nv, nruns, run, first);
     GW_CUDA(ctx, cudaGetLastError(), "edge runs");
   }
+  if (pull) {
+    unsigned long long* const sums = rows + nv + 1;
+    uint32_t* const place = reinterpret_cast<uint32_t*>(ctx->d_exact.as<char>() + place_at);
+    GW_CUDA(ctx, cudaMemsetAsync(place, 0, nv * 4, st), "clear");
+    gw::in_degree_kernel<<<(unsigned)std::min<uint64_t>((ne + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(
+        colidx, ne, ctx->nv, place);
+    gw::scan_sums_kernel<<<nscan, gw::kExactThreads, 0, st>>>(place, ctx->nv, sums);
+    gw::scan_blocks_kernel<<<1, gw::kExactThreads, 0, st>>>(sums, nscan);
+    gw::scan_rows_kernel<<<nscan, gw::kExactThreads, 0, st>>>(place, ctx->nv, sums, rows);
+    gw::exact_edge_kernel<true><<<egrid, gw::kExactThreads, 0, st>>>(nullptr, nullptr, rowptr, colidx, ctx->nv, ne,
+                                                                         nruns, run, first, place, turned);
+    gw::exact_runs_kernel<<<rgrid, 256, 0, st>>>(rows, ctx->nv, nruns, run, first);
+    GW_CUDA(ctx, cudaGetLastError(), "turn");
+  }
   const unsigned vgrid = (unsigned)std::min<uint64_t>((nv + gw::kExactThreads - 1) / gw::kExactThreads, (uint64_t)sms * 8);
-  const unsigned egrid = (unsigned)((nruns * 32 + gw::kExactThreads - 1) / gw::kExactThreads);
   for (uint32_t h = 0; h < hops; ++h) {
     gw::exact_vertex_kernel<<<vgrid, gw::kExactThreads, 0, st>>>(acc, share, visits, debts, h, rowptr, ctx->nv, source,
                                                                  a.njump, q, rule);
     GW_CUDA(ctx, cudaGetLastError(), "exact vertices");
     if (h + 1 == hops) break;  // the last hop's moves are not visited
     if (nruns) {
-      gw::exact_edge_kernel<<<egrid, gw::kExactThreads, 0, st>>>(share, acc, rowptr, ctx->d_colidx.as<uint32_t>(),
-                                                                 ctx->nv, ne, nruns, run, first);
+      if (pull)
+        gw::exact_pull_kernel<<<egrid, gw::kExactThreads, 0, st>>>(share, acc, rows, turned, ctx->nv, ne, nruns, run,
+                                                                  first);
+      else
+        gw::exact_edge_kernel<false><<<egrid, gw::kExactThreads, 0, st>>>(share, acc, rowptr, colidx, ctx->nv, ne,
+                                                                             nruns, run, first, nullptr, nullptr);
       GW_CUDA(ctx, cudaGetLastError(), "exact edges");
     }
     if (rule == GW_RULE_PROB && (h & 15) == 15) {  // the uncapped rule stops when the mass is gone

@@ -188,9 +188,10 @@ def test_expected_visits_kernel_matches_fp64_oracle(cuda_device, oracle, rule, L
 
 
 @pytest.mark.parametrize("edges", ["none", "one", "hub", "runs"])
-@pytest.mark.parametrize("rule,L", [(0, 6), (1, 1), (3, 7), (4, 9)])
+@pytest.mark.parametrize("rule,L", [(0, 6), (0, 7), (1, 1), (3, 7), (3, 8), (4, 9)])
 def test_expected_visits_edge_runs(cuda_device, oracle, edges, rule, L):
-    """The edge kernel's runs at their edges: no edges at all, one edge, a hub
+    """The edge kernel's runs at their edges, pushed along out-edges (up to six
+    hops) and pulled along in-edges (from seven): no edges at all, one edge, a hub
     whose row fills many runs between long stretches of empty rows, and rows of
     127, 128 and 129 edges.  All terms are positive, so the relative error of a
     sum of k of them is below k times 2^-53; k is at most every edge and every
