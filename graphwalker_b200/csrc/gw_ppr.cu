@@ -148,31 +148,36 @@ __device__ __forceinline__ uint32_t query_of(const unsigned long long* __restric
   return lo;
 }
 
+constexpr int kSmall = 0, kMid = 1, kLarge = 2;
+
 // One walk per lane.  A visit's table update is a chain of its own (the slot,
 // then a CAS or more probes), and in a warp of 32 visits some lane always has a
 // long one, so the hop does not wait for it:
 //
-//  * SMALL = false, launches that fill the GPU, which the random line fills and
+//  * kMid and kLarge, launches that fill the GPU, which the random line fills and
 //    the tables' requests bound: the slot is loaded at a visit and acted on at
 //    the lane's next one, behind that visit's gather.
-//  * SMALL = true, launches of few walks, which the chain of hops bounds: visits
+//  * kSmall, launches of few walks, which the chain of hops bounds: visits
 //    go to a queue in shared memory, worked off kFlush at a time, kPerLane per
 //    lane side by side, behind a gather; the draws of the next hop are computed
 //    while this one's gather is in flight, so a hop's own chain is the gather,
 //    a modulo and the next address.  (It holds visits back, so the tables of
-//    more queries are open at once: 16.5 ms where the other takes 11.6 on 4096
+//    more queries are open at once: 16.5 ms where the others take 11.7 and 10.9 on 4096
 //    queries.)
 //
 // Measured on B200 (walk kernel alone): 4096 queries, 59 M walks, R-MAT scale
-// 24: 14.0 ms when a CAS was the first probe and the hop waited for it, 11.6
-// now (33 G visits/s); one query of 100,000 walks at scale 20: 65 -> 60 us; one
-// of 300 walks at scale 22: 55 -> 33 us (42 with SMALL = false).
-template <int RULE, bool ER, bool SMALL>
-__global__ void __launch_bounds__(kPprThreads, SMALL ? 4 : 1)
+// 24: 14.0 ms when a CAS was the first probe and the hop waited for it, 10.9
+// now (35 G visits/s); one query of 100,000 walks at scale 20: 65 -> 60 us; one
+// of 300 walks at scale 22: 55 -> 33 us (42 with kMid).
+template <int RULE, bool ER, int SHAPE>
+__global__ void __launch_bounds__(kPprThreads, SHAPE == kSmall ? 4 : SHAPE == kLarge ? 5 : 1)
     walk_query_kernel(QueryView qv, unsigned long long w_begin, unsigned long long w_end, GraphView g,
                       WalkArgs a, uint32_t* __restrict__ status) {
+  constexpr bool SMALL = SHAPE == kSmall;
   constexpr int kPerLane = 2;
   constexpr uint32_t kFlush = 32 * kPerLane;
+  let_next_start();
+  wait_for_previous();
   __shared__ uint2 queues[SMALL ? kPprThreads / 32 : 1][kFlush + 32];  // (query, vertex)
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1u;  // lanes under this one
@@ -215,7 +220,7 @@ __global__ void __launch_bounds__(kPprThreads, SMALL ? 4 : 1)
     table_updates<kPerLane>(qv, fq, fv, fn, seen, hp.cnt);
     __syncwarp();
   };
-  // The lane's update in flight (SMALL = false).
+  // The lane's update in flight (not SMALL).
   uint32_t p_q[1] = {0}, p_v[1] = {0}, p_n[1] = {0};
   unsigned long long p_seen[1] = {0};
   for (;;) {
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(kPprThreads, SMALL ? 4 : 1)
     const uint32_t pushes = SMALL ? __ballot_sync(~0u, visits && hop > 0) : 0u;
     if (visits) {
       ++nvisit;
-      uint32_t u_n = 0;  // SMALL = false: this visit's update, if the lane makes it
+      uint32_t u_n = 0;  // not SMALL: this visit's update, if the lane makes it
       const uint32_t u_v = v;
       unsigned long long u_seen = 0;
       if (SMALL) {
@@ -759,6 +764,9 @@ __global__ void __launch_bounds__(kTopkThreads, 3)
 //
 // One query of 100,000 walks (a million slots) took 26 us in 64 streaming CTAs
 // and 22 us in the merge's one, most of it barriers; here 26 together (ncu, cold L2).
+//
+// It is launched to start while the walk kernel drains: what it reads before
+// wait_for_previous() was copied up before that kernel.
 __global__ void __launch_bounds__(kTopkFewThreads, 1)
     topk_few_kernel(QueryView qv, uint32_t q_begin, uint32_t q_count, uint32_t k,
                     const unsigned long long* __restrict__ seg_first, unsigned long long* seg_cand,
@@ -771,6 +779,7 @@ __global__ void __launch_bounds__(kTopkFewThreads, 1)
   const uint32_t q = segment_query(seg_first, q_begin, q_begin + q_count - 1, g);
   const uint32_t nseg = (uint32_t)(seg_first[q + 1] - seg_first[q]);
   const uint32_t cap = qv.table_mask[q] + 1, first = (uint32_t)(g - seg_first[q]) * kTopkFewSlots;
+  wait_for_previous();
   uint32_t n = block_select<kTopkFewThreads, kTopkFewSlots / kTopkFewThreads>(
       table_slots(qv, q, first), cap - first < kTopkFewSlots ? cap - first : kTopkFewSlots, k, cand, select);
   if (nseg > 1) {
@@ -792,6 +801,7 @@ __global__ void __launch_bounds__(kTopkFewThreads, 1)
 
 __global__ void clear_tables_kernel(ulonglong2* __restrict__ t, unsigned long long n2) {
   const ulonglong2 empty = make_ulonglong2(kEmptySlot, kEmptySlot);
+  let_next_start();
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n2;
        i += (unsigned long long)gridDim.x * blockDim.x)
     t[i] = empty;
@@ -801,6 +811,7 @@ __global__ void clear_tables_kernel(ulonglong2* __restrict__ t, unsigned long lo
 // 256 slots).
 __global__ void __launch_bounds__(256)
     clear_queries_kernel(QueryView qv, const unsigned long long* __restrict__ piece_first) {
+  let_next_start();
   const uint32_t q = segment_query(piece_first, 0, qv.nq - 1, blockIdx.x);
   const uint32_t slots = qv.table_mask[q] + 1, first = (uint32_t)(blockIdx.x - piece_first[q]) * kClearSlots;
   const uint32_t n2 = (slots - first < kClearSlots ? slots - first : kClearSlots) / 2;
@@ -815,19 +826,27 @@ int sm_count() {
   return sms;
 }
 
-// Launches up to this many walks run the SMALL kernel: one CTA per SM.  Scales
+// Launches up to this many walks run the kSmall kernel: one CTA per SM.  Scales
 // 20 and 22, one query: 3000 walks 41 us against 49, 20,000 42.5 against 46.5,
 // 37,000 45 against 48, 60,000 54 against 53, 100,000 76 against 60.
 constexpr unsigned long long kSmallLaunch = 148 * kPprThreads;
+// From here on the kLarge kernel: the same in 51 registers, five CTAs per SM
+// instead of four (4096 queries 10.9 ms against 11.7; 4.1 M walks at scale 22
+// 0.80 against 0.85; 600,000 at 23 0.19 against 0.18).
+constexpr unsigned long long kLargeLaunch = 1u << 20;
 
 template <int RULE>
 cudaError_t query_dispatch(const QueryView& qv, unsigned long long w_begin, unsigned long long w_end,
                            const GraphView& g, const WalkArgs& a, uint32_t* status, int threads_per_sm,
                            cudaStream_t stream) {
   const unsigned long long n = w_end - w_begin;
-  const bool small = n <= kSmallLaunch;
-  auto kern = g.erec ? (small ? walk_query_kernel<RULE, true, true> : walk_query_kernel<RULE, true, false>)
-                     : (small ? walk_query_kernel<RULE, false, true> : walk_query_kernel<RULE, false, false>);
+  const int shape = n <= kSmallLaunch ? kSmall : n < kLargeLaunch ? kMid : kLarge;
+  auto kern = g.erec ? (shape == kSmall  ? walk_query_kernel<RULE, true, kSmall>
+                        : shape == kMid ? walk_query_kernel<RULE, true, kMid>
+                                        : walk_query_kernel<RULE, true, kLarge>)
+                     : (shape == kSmall  ? walk_query_kernel<RULE, false, kSmall>
+                        : shape == kMid ? walk_query_kernel<RULE, false, kMid>
+                                        : walk_query_kernel<RULE, false, kLarge>);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPprThreads, 0);
   const int sms = sm_count();
@@ -844,8 +863,7 @@ cudaError_t query_dispatch(const QueryView& qv, unsigned long long w_begin, unsi
   const unsigned long long fair = ((n + warps - 1) / warps + 31) / 32 * 32;
   const unsigned long long chunk = qv.chunk ? qv.chunk : kWarpChunk;
   q.chunk = (uint32_t)(fair < chunk ? fair : chunk);
-  kern<<<grid, kPprThreads, 0, stream>>>(q, w_begin, w_end, g, a, status);
-  return cudaGetLastError();
+  return launch_dependent(kern, grid, kPprThreads, 0, stream, q, w_begin, w_end, g, a, status);
 }
 
 }  // namespace
@@ -936,9 +954,8 @@ cudaError_t launch_topk_segmented(const QueryView& qv, uint32_t q_begin, uint32_
   const unsigned long long nseg = h_seg_first[q_begin + q_count] - h_seg_first[q_begin];
   if (nseg == 0 || nseg > 0x7fffffffull) return cudaErrorInvalidValue;
   if (topk_is_few(h_seg_first + q_begin, q_count, seg_slots, k)) {
-    topk_few_kernel<<<(unsigned)nseg, kTopkFewThreads, 0, stream>>>(qv, q_begin, q_count, k, d_seg_first, d_seg_cand,
-                                                                  d_seg_done, out_ids, out_counts);
-    return cudaGetLastError();
+    return launch_dependent(topk_few_kernel, (unsigned)nseg, kTopkFewThreads, 0, stream, qv, q_begin, q_count, k,
+                            d_seg_first, d_seg_cand, d_seg_done, out_ids, out_counts);
   }
   if (nseg == q_count) {  // no table is split: one CTA per query
     topk_kernel<<<q_count, kTopkThreads, 0, stream>>>(qv, q_begin, k, d_order, out_ids, out_counts);

@@ -21,8 +21,8 @@ constexpr uint32_t kSelectBins = 1u << kSelectBits;
 // Walks a warp takes from the batch cursor at a time, by default: small
 // enough that the walks in flight stay inside a narrow window of the batch
 // (and of its queries, whose tables then stay in L2), large enough that the
-// cursor's atomic is not contended.  R-MAT scale 24, 4096 queries: 13.7 ms
-// with 64, 12.2 with 96, 11.6 with 128, 11.9 with 192 and 13.4 with 256.
+// cursor's atomic is not contended.  R-MAT scale 24, 4096 queries: 12.4 ms
+// with 64, 11.2 with 96, 10.9 with 128, 12.1 with 192.
 // gw_ppr_autotune picks it per context with the launch shape.
 constexpr uint32_t kWarpChunk = 128;
 

@@ -248,12 +248,12 @@ def test_topk_at_table_sizes(cuda_device, oracle, budgets, k):
         assert np.array_equal(got[0][0][q], want[0]) and np.array_equal(got[0][1][q], want[1]), q
 
 
-@pytest.mark.parametrize("walks", [37_887, 37_888, 37_889, 120_000])
+@pytest.mark.parametrize("walks", [37_887, 37_888, 37_889, (1 << 20) - 1, 1 << 20])
 @pytest.mark.parametrize("rule,layout", [(4, 1), (0, 1), (3, 0)])
 def test_walk_launches_around_the_small_limit(cuda_device, oracle, walks, rule, layout):
     """One query and several whose walks sum to one short of, exactly and past
-    the launch size (148 x 256) up to which visits are queued in shared memory;
-    all lists equal the oracle's counts.  Sources of low degree make their
+    the launch size (148 x 256) up to which visits are queued in shared memory,
+    and around the one (2^20) from which five CTAs share an SM; all lists equal the oracle's counts.  Sources of low degree make their
     first visits collide."""
     import graphwalker_b200 as gw
     rp, ci = oracle.rmat_csr(14, 8, seed=2)
