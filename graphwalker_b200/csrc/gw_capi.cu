@@ -880,10 +880,14 @@ gw_status gw_run_pools(gw_ctx* ctx, const gw_walk_params* params, const uint64_t
   // previous kernel's last walks finish instead of after them (the walks of
   // different chunks share only the visit counters, updated atomically).
   // The last chunk's walks run after its copy with nothing to hide behind, so
-  // no chunk holds more than an eighth of them: 4 M walks at R-MAT scale 22
-  // took 1229 us with chunks that kept growing (the last held 43 %), 1089 now
-  // (2^18 and 2^20 walks at most: 1129, 1162); 16.8 M at scale 24 5.22 -> 4.65 ms.
-  const std::vector<uint64_t> chunk_lo = gw::chunk_bounds(n, n / 8);
+  // where walks are of full length no chunk holds more than an eighth of them:
+  // 4 M jumping walks at R-MAT scale 22 took 1229 us with chunks that kept
+  // growing (the last held 43 %), 1089 now (2^18 and 2^20 walks at most: 1129,
+  // 1162); 16.8 M at scale 24 5.22 -> 4.65 ms.  Walks that end early hide in
+  // less, and more copies cost more: 3.1 M with ids at 22 1105 us growing, 1135
+  // in eighths.
+  const bool full_length = params->rule == GW_RULE_JUMP || params->rule == GW_RULE_RESTART;
+  const std::vector<uint64_t> chunk_lo = gw::chunk_bounds(n, full_length ? n / 8 : n);
   const uint64_t nchunks = chunk_lo.size() - 1;
   GW_CUDA(ctx, ctx->d_walks.ensure(n * sizeof(gw_walk_rec)), "walk alloc");
   GW_CUDA(ctx, ctx->d_words.ensure(n * 8), "word alloc");

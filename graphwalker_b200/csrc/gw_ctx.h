@@ -219,8 +219,8 @@ struct gw_ctx {
   gw_status cuda_fail(cudaError_t e, const char* what) {
     return fail(e == cudaErrorMemoryAllocation ? GW_E_NOMEM : GW_E_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
-  gw::GraphView view() const {
-    gw::GraphView g;
+  gw::GraphPlan view() const {
+    gw::GraphPlan g;
     g.vrec = d_vrec.as<const unsigned long long>();
     g.rowptr = d_rowptr.as<const unsigned long long>();
     g.colidx = d_colidx.as<const uint32_t>();

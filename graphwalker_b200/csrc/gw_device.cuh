@@ -133,9 +133,14 @@ struct GraphView {
   // Out-edge bitmap (nv bits, stored right after the packed records; NULL
   // when the records are not built): bit v is set when v has out-edges.
   const uint32_t* __restrict__ out_bits;
+  uint32_t nv;
+};
+
+// The graph as launches see it: the kernels' view, and what the choice of a
+// layout goes by (host only).
+struct GraphPlan : GraphView {
   uint64_t csr_bytes;  // columns and vertex records: what a walk over the plain layout touches
   uint64_t csr_limit;  // resident walks keep to the plain layout up to this many bytes (csr_walk_limit)
-  uint32_t nv;
 };
 
 struct SinkView {

@@ -27,7 +27,7 @@ constexpr uint32_t kDefaultHints = kHintColumnsEvictFirst | kHintCountsEvictLast
 // ---- walk kernels (gw_walk.cu) ----
 // window (may be NULL): an L2 access policy window attached to the launch.
 cudaError_t launch_walk_resident(int rule, int sink, bool agg, const gw_walk_rec* walks, uint64_t n,
-                                 const GraphView& g, const WalkArgs& a, const SinkView& s,
+                                 const GraphPlan& g, const WalkArgs& a, const SinkView& s,
                                  uint32_t* status, int grid, cudaStream_t stream,
                                  const cudaAccessPolicyWindow* window = nullptr);
 int walk_resident_grid(int rule, int sink, bool agg, uint64_t n);

@@ -433,7 +433,7 @@ int grid_of(int per_sm, uint64_t n) {
 //   PPR, restart: their walks go back to a source whose record they hold (PPR:
 //     1 M at 20 148 / 162, 4 M at 22 560 / 656; restart: 127 / 122, 513 / 534).
 template <int RULE>
-bool walks_use_records(const GraphView& g, uint64_t n) {
+bool walks_use_records(const GraphPlan& g, uint64_t n) {
   if (!g.erec) return false;
   if (RULE == GW_RULE_JUMP) return g.csr_bytes > g.csr_limit;
   return rule_returns<RULE>() || n < 1u << 19 || g.csr_bytes > g.csr_limit / 2;
@@ -455,7 +455,7 @@ int default_ctas_per_sm(bool records, uint64_t n, uint32_t path_stride) {
 }
 
 template <int RULE, int SINK, bool AGG>
-cudaError_t resident_dispatch(const gw_walk_rec* walks, uint64_t n, const GraphView& g,
+cudaError_t resident_dispatch(const gw_walk_rec* walks, uint64_t n, const GraphPlan& g,
                               const WalkArgs& a, const SinkView& s, uint32_t* status, int grid,
                               cudaStream_t stream, const cudaAccessPolicyWindow* window) {
   const bool records = walks_use_records<RULE>(g, n);
@@ -529,7 +529,7 @@ cudaError_t block_dispatch(gw_walk_rec* walks, uint64_t n, const GraphView& g,
   }
 
 cudaError_t launch_walk_resident(int rule, int sink, bool agg, const gw_walk_rec* walks, uint64_t n,
-                                 const GraphView& g, const WalkArgs& a, const SinkView& s,
+                                 const GraphPlan& g, const WalkArgs& a, const SinkView& s,
                                  uint32_t* status, int grid, cudaStream_t stream,
                                  const cudaAccessPolicyWindow* window) {
   if (n == 0) return cudaSuccess;
