@@ -13,17 +13,22 @@
 //    in a 16-bit mask.  Integer-ALU bound (87 %): 1647 us for 512 queries of
 //    R = 1000, L = 11 on a scale-20 graph.
 //  * simrank_join_kernel: few pairs ever stand on the same vertex (about 90 of
-//    a million per position there), so a CTA joins a tile of a's walks with a
-//    tile of b's by hashing, O(R) work a position, and only a pair that
-//    matches is checked against its earlier positions.  A pair counts at its
-//    first match only, so the counts are the loop's, whatever the order.
-//    251 us for the same queries; bound by issue slots and the latency of
-//    two barriers and a few shared-memory round trips per position.
+//    a million per position there), so a CTA marks the vertices of a tile of
+//    b's walks in a bitmap and looks a tile of a's walks up in it, O(R) work a
+//    position; only a walk whose bit is set is compared with the whole tile,
+//    by a warp, two such walks at a time.  A bit per pair in shared memory
+//    keeps who has met, as in the pairs kernel, so a matching pair costs one
+//    bit, however many match.  111 us for the same queries (251 with the
+//    walks in hash chains and each match checked against all earlier
+//    positions, which also grew with coinciding walks: 3000 walks x 40 on 100
+//    vertices took 600 us, 120 with every pair compared, 150 so); bound by
+//    issue slots and the latency of two barriers and a few shared-memory
+//    round trips per position.
 //
-// The join has 30 us of such latency even for one query, and its chains grow
-// when walks coincide, so small batches keep comparing pairs (kPairWork).  The
-// grid's z dimension runs over queries: query q compares the R walks at row
-// offset rows[2q] of `a` with those at rows[2q + 1] of `b`.
+// Every position being a round of such latency, small batches keep comparing
+// pairs (kPairWork).  The grid's z dimension runs over queries: query q
+// compares the R walks at row offset rows[2q] of `a` with those at
+// rows[2q + 1] of `b`.
 #include <algorithm>
 
 #include "gw_internal.h"
@@ -85,11 +90,8 @@ __global__ void __launch_bounds__(kPairThreads)
   }
 }
 
-constexpr uint32_t kSrPairs = 512;      // matching pairs listed per position
 constexpr uint32_t kNoVisit = 0xffffffffu;
-constexpr uint32_t kNoWalk = 0xffffffffu;
-
-constexpr uint32_t kSrChunk = 12;  // positions staged at a time
+constexpr uint32_t kSrChunk = 6;  // positions staged at a time (12 leave two CTAs an SM, 4 are read in shorter pieces)
 
 // LOG: a tile is 2^LOG walks of each side, one of each per thread.
 template <int LOG>
@@ -97,52 +99,42 @@ __global__ void __launch_bounds__(1 << LOG)
     simrank_join_kernel(const uint32_t* __restrict__ a0, const uint32_t* __restrict__ b0,
                         const unsigned long long* __restrict__ rows, uint32_t q0, uint32_t R, uint32_t L,
                         unsigned long long* __restrict__ meet0) {
-  constexpr uint32_t kSrTile = 1 << LOG, kSrSlots = 2 * kSrTile;  // tables at most half full
-  auto sr_slot = [](uint32_t v) { return (v * 0x9E3779B1u) >> (31 - LOG); };
-  extern __shared__ uint32_t staged[];
-  uint32_t(*const sa)[kSrTile + 1] = reinterpret_cast<uint32_t(*)[kSrTile + 1]>(staged);
-  uint32_t(*const sb)[kSrTile + 1] = sa + kSrChunk;
-  // Two tables, one cleared while the other is looked up.  A slot holds a
-  // vertex (key; kNoVisit = free) and the walk entered last under it (head);
-  // next[walk] is the walk entered before it.  Half of a position's walks can
-  // stand on one vertex (the source they return to), so heads are exchanged,
-  // which never retries.
-  __shared__ uint32_t key[2][kSrSlots];
-  __shared__ uint32_t head[2][kSrSlots];
-  __shared__ uint32_t next[kSrTile];
-  __shared__ uint32_t pairs[2][kSrPairs];  // a position's matches: walk of a << 16 | walk of b
-  __shared__ uint32_t npairs[2];
-  __shared__ uint32_t met;  // pairs of the tile that have met
-  const uint32_t q = q0 + blockIdx.z, x = threadIdx.x;
+  constexpr uint32_t kSrTile = 1 << LOG, kWarps = kSrTile / 32, kRow = kSrTile + 4, kWords = kSrTile / 32;
+  constexpr uint32_t kBits = 64 * kSrTile;  // a bit per hashed vertex
+  auto bit_of = [](uint32_t v) { return (v * 0x9E3779B1u) >> (26 - LOG); };
+  extern __shared__ __align__(16) uint32_t staged[];
+  uint32_t(*const sa)[kRow] = reinterpret_cast<uint32_t(*)[kRow]>(staged);
+  uint32_t(*const sb)[kRow] = sa + kSrChunk;
+  // a bit per pair that has met, by walk of a
+  uint32_t(*const pairs)[kWords] = reinterpret_cast<uint32_t(*)[kWords]>(staged + 2 * kSrChunk * kRow);
+  __shared__ __align__(16) uint32_t bits[2][kBits / 32];  // one is cleared while the other is read
+  __shared__ uint16_t cand[kSrTile];                       // a's walks whose vertex has its bit set
+  __shared__ uint32_t ncand[2];
+  __shared__ uint32_t found[kSrChunk];  // pairs met at a staged position
+  __shared__ uint32_t met;              // pairs of the tile that have met
+  const uint32_t q = q0 + blockIdx.z, x = threadIdx.x, lane = x & 31, warp = x >> 5;
   const uint32_t i0 = blockIdx.y * kSrTile, j0 = blockIdx.x * kSrTile;
-  const uint32_t na = min(R - i0, (uint32_t)kSrTile), nb = min(R - j0, (uint32_t)kSrTile);
+  const uint32_t na = min(R - i0, kSrTile), nb = min(R - j0, kSrTile);
   const uint32_t* __restrict__ a = a0 + (rows ? rows[2 * (size_t)q] : 0ull) + (size_t)i0 * L;
   const uint32_t* __restrict__ b = b0 + (rows ? rows[2 * (size_t)q + 1] : 0ull) + (size_t)j0 * L;
   unsigned long long* __restrict__ meet = meet0 + (size_t)q * L;
-  for (uint32_t s = x; s < 2 * kSrSlots; s += kSrTile) {
-    key[0][s] = kNoVisit;  // both tables
-    head[0][s] = kNoWalk;
-  }
-  if (x == 0) met = npairs[0] = npairs[1] = 0;
-  uint32_t l0 = 0;  // first position staged
-  // whether walks i and j shared no vertex at a position before l
-  auto first_meeting = [&](uint32_t i, uint32_t j, uint32_t l) {
-    uint32_t k = 0;
-    for (; k < l0 && k < l; ++k) {
-      const uint32_t p = __ldg(a + (size_t)i * L + k);
-      if (p == __ldg(b + (size_t)j * L + k) && p != kNoVisit) return false;
-    }
-    for (; k < l; ++k) {
-      const uint32_t p = sa[k - l0][i];
-      if (p == sb[k - l0][j] && p != kNoVisit) return false;
-    }
-    return true;
+  auto clear = [&](uint32_t t) {
+    for (uint32_t w = x; w < kBits / 128; w += kSrTile) reinterpret_cast<uint4*>(bits[t])[w] = make_uint4(0, 0, 0, 0);
   };
-  uint32_t n = 0;  // pairs this thread found to meet first at the position before
-  for (uint32_t l = 0;; ++l) {
+  clear(0);
+  for (uint32_t w = 0; w < kWords; ++w) pairs[0][w * kSrTile + x] = 0;
+  if (x == 0) met = ncand[0] = ncand[1] = 0;
+  if (x < kSrChunk) found[x] = 0;
+  uint32_t l0 = 0;  // first position staged
+  for (uint32_t l = 0; l < L; ++l) {
     const uint32_t t = l & 1, c = l % kSrChunk;
-    if (c == 0 && l < L) {
-      const uint32_t w = min(L - l, (uint32_t)kSrChunk);  // rows of a tile lie one behind the other
+    if (c == 0) {
+      __syncthreads();  // the candidates before are done with the rows staged before
+      if (x < kSrChunk && found[x]) {
+        atomicAdd(meet + l0 + x, (unsigned long long)found[x]);
+        found[x] = 0;
+      }
+      const uint32_t w = min(L - l, kSrChunk);  // rows of a tile lie one behind the other
       uint32_t r = x / w, z = x - r * w;
       const uint32_t dr = kSrTile / w, dz = kSrTile - dr * w;
       for (uint32_t y = 0; y < w; ++y) {
@@ -158,56 +150,64 @@ __global__ void __launch_bounds__(1 << LOG)
       l0 = l;
       __syncthreads();
     }
-    // enter b's walks of this position; count the matches of the one before
-    if (l < L) {
-      const uint32_t v = sb[c][x];
-      if (v != kNoVisit) {
-        uint32_t s = sr_slot(v);
-        for (;;) {
-          uint32_t k = *reinterpret_cast<volatile uint32_t*>(&key[t][s]);
-          if (k == kNoVisit) k = atomicCAS(&key[t][s], kNoVisit, v);
-          if (k == kNoVisit || k == v) break;
-          s = (s + 1) & (kSrSlots - 1);
+    // mark b's vertices; half of a position's walks can stand on one vertex
+    // (the source they return to), so a bit that is set is left alone
+    const uint32_t u = sb[c][x], h = bit_of(u), m = 1u << (h & 31u);
+    if (u != kNoVisit && !(*reinterpret_cast<volatile uint32_t*>(&bits[t][h >> 5]) & m)) atomicOr(&bits[t][h >> 5], m);
+    __syncthreads();
+    if (met == na * nb) break;  // met changes only after the next barrier
+    // a's walks that may stand on one of them
+    const uint32_t v = sa[c][x], hv = bit_of(v);
+    const bool may = v != kNoVisit && ((bits[t][hv >> 5] >> (hv & 31u)) & 1u);
+    const uint32_t mine = __ballot_sync(~0u, may);
+    if (mine) {
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&ncand[t], (uint32_t)__popc(mine));
+      at = __shfl_sync(~0u, at, 0) + __popc(mine & ((1u << lane) - 1u));
+      if (may) cand[at] = (uint16_t)x;
+    }
+    clear(t ^ 1);
+    if (x == 0) ncand[t ^ 1] = 0;
+    __syncthreads();
+    // a warp per two candidates, its lanes over b's walks
+    uint32_t n = 0;
+    for (uint32_t y = 2 * warp, count = ncand[t]; y < count; y += 2 * kWarps) {
+      const bool two = y + 1 < count;
+      const uint32_t i0 = cand[y], i1 = cand[two ? y + 1 : y], p0 = sa[c][i0], p1 = sa[c][i1];
+      uint32_t now0 = 0, now1 = 0;  // lane w: word w of a walk's matches
+#pragma unroll
+      for (uint32_t k = 0; k < kWords / 4; ++k) {
+        const uint4 w = *reinterpret_cast<const uint4*>(&sb[c][4 * lane + 128 * k]);
+        auto word = [&](uint32_t p) {
+          const uint32_t m0 = __ballot_sync(~0u, w.x == p), m1 = __ballot_sync(~0u, w.y == p);
+          const uint32_t m2 = __ballot_sync(~0u, w.z == p), m3 = __ballot_sync(~0u, w.w == p);
+          return lane & 2 ? (lane & 1 ? m3 : m2) : (lane & 1 ? m1 : m0);
+        };
+        const uint32_t w0 = word(p0), w1 = word(p1);
+        if (lane / 4 == k) {
+          now0 = w0;
+          now1 = w1;
         }
-        next[x] = atomicExch(&head[t][s], x);
+      }
+      if (now0) {
+        const uint32_t old = pairs[i0][lane];
+        n += __popc(now0 & ~old);
+        pairs[i0][lane] = old | now0;
+      }
+      if (two && now1) {
+        const uint32_t old = pairs[i1][lane];
+        n += __popc(now1 & ~old);
+        pairs[i1][lane] = old | now1;
       }
     }
-    if (l > 0) {
-      const uint32_t listed = min(npairs[t ^ 1], kSrPairs);
-      for (uint32_t y = x; y < listed; y += kSrTile) {
-        const uint32_t p = pairs[t ^ 1][y];
-        n += first_meeting(p >> 16, p & 0xffffu, l - 1) ? 1u : 0u;
-      }
-      n = __reduce_add_sync(~0u, n);
-      if ((x & 31) == 0 && n) {
-        atomicAdd(meet + l - 1, (unsigned long long)n);
-        atomicAdd(&met, n);
-      }
-      n = 0;
+    n = __reduce_add_sync(~0u, n);
+    if (lane == 0 && n) {
+      atomicAdd(&found[c], n);
+      atomicAdd(&met, n);
     }
-    __syncthreads();
-    if (l == L || met == na * nb) break;  // met changes only after the next barrier
-    // look a's walks up; clear the other table and the list just counted
-    if (x == 0) npairs[t ^ 1] = 0;
-    const uint32_t v = sa[c][x];
-    if (v != kNoVisit) {
-      uint32_t s = sr_slot(v), k;
-      while ((k = key[t][s]) != v && k != kNoVisit) s = (s + 1) & (kSrSlots - 1);
-      // Matches are listed and checked one per thread: checked here, a lane's
-      // chain would hold its warp for one check after another.  What the list
-      // has no room for is checked here.
-      for (uint32_t j = k == v ? head[t][s] : kNoWalk; j != kNoWalk; j = next[j]) {
-        const uint32_t y = atomicAdd(&npairs[t], 1u);
-        if (y < kSrPairs) pairs[t][y] = x << 16 | j;
-        else n += first_meeting(x, j, l) ? 1u : 0u;
-      }
-    }
-    for (uint32_t s = x; s < kSrSlots; s += kSrTile) {
-      key[t ^ 1][s] = kNoVisit;
-      head[t ^ 1][s] = kNoWalk;
-    }
-    __syncthreads();
   }
+  __syncthreads();
+  if (x < kSrChunk && found[x]) atomicAdd(meet + l0 + x, (unsigned long long)found[x]);
 }
 
 // The app's placement (simrank.cpp:30-57): replica i of vertex v starts at v
@@ -238,20 +238,26 @@ cudaError_t launch_simrank_meet(const uint32_t* a, const uint32_t* b, const unsi
                                 uint32_t R, uint32_t L, unsigned long long* meet, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(meet, 0, (size_t)nq * L * sizeof(unsigned long long), stream);
   if (e != cudaSuccess || R == 0 || L == 0) return e;
-  // Comparisons up to which pairs are compared: 12 queries of R = 1000, L = 11
-  // take about 38 us so, and about 35 us joined; 64 take 205 and 65.  (1000
-  // walks on four vertices, one query: 10 us compared, 370 joined.)
+  // Comparisons up to which pairs are compared.  A call of 8 queries of
+  // R = 1000, L = 11 takes 92 us so and 81 joined, 12 take 106 and 81, 64 take
+  // 283 and 97; 1000 walks on four vertices, one query: 34 us compared, 100
+  // joined (one walk compared at a time).
   constexpr uint64_t kPairWork = 1ull << 27;
   const uint64_t compares = (uint64_t)R * R * L;
   const bool join = compares >= kPairWork / std::max(nq, 1u);
-  // Joined tiles of 512 walks repeat the hashing least (512 queries: 0.57 ms a
-  // call against 0.65 in tiles of 256) but need enough queries to fill the
-  // SMs (64 queries: 0.18 against 0.16).
-  const uint64_t wide = (R + 511) / 512;
-  const uint32_t log = wide * wide * nq >= 592 ? 9 : 8;
+  // Joined tiles of 512 walks repeat the marking least (a call of 512 queries:
+  // 0.30 ms, 0.34 in tiles of 256, 0.44 of 128) but need 592 tiles, four an
+  // SM, to fill the chip (24 queries: 107 us, 85 and 93; one dense query of
+  // 3000 walks x 40: 717, 379 and 270; all with one walk compared at a time).
+  uint32_t log = 9;
+  for (; log > 7; --log) {
+    const uint64_t wide = (R + (1ull << log) - 1) >> log;
+    if (wide * wide * nq >= 592) break;
+  }
   const uint32_t tile = join ? 1u << log : (uint32_t)kPairTile, tiles = (R + tile - 1) / tile;
-  const size_t smem = join ? 2 * kSrChunk * (size_t)(tile + 1) * 4 : 0;
-  auto k = !join ? simrank_pairs_kernel : log == 9 ? simrank_join_kernel<9> : simrank_join_kernel<8>;
+  const size_t smem = join ? (2 * kSrChunk * (size_t)(tile + 4) + tile * tile / 32) * 4 : 0;
+  auto k = !join ? simrank_pairs_kernel
+           : log == 9 ? simrank_join_kernel<9> : log == 8 ? simrank_join_kernel<8> : simrank_join_kernel<7>;
   if (join) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   for (uint32_t q0 = 0; q0 < nq && e == cudaSuccess; q0 += 65535u) {
     const uint32_t nz = nq - q0 < 65535u ? nq - q0 : 65535u;

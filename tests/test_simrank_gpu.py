@@ -111,13 +111,13 @@ def test_simrank_batch_matches_oracle(cuda_device, oracle):
     assert np.all(meet[:5, 0] >= R)  # every walk meets itself at its source
 
 
-@pytest.mark.parametrize("R,L,vertices", [(511, 520, 5000), (512, 513, 3), (3650, 11, 5000), (4097, 9, 1),
+@pytest.mark.parametrize("R,L,vertices", [(511, 520, 5000), (512, 513, 3), (3650, 11, 5000), (4097, 9, 1), (6401, 7, 40),
                                           (2049, 40, 900), (2020, 33, 100_000)])
 def test_meet_counts_at_join_tile_edges(cuda_device, oracle, R, L, vertices):
-    """Past 2^27 comparisons the walks are joined, in tiles of 256 here (one
-    query) and of 512 below: one short of and exactly a tile, one past, rows of
-    one to 44 staged pieces of 12 positions; sparse meetings, long chains and
-    every pair meeting at once; vertex ids that share few hash slots."""
+    """Past 2^27 comparisons the walks are joined, in tiles of 128 (256 from
+    6145 walks a query): one short of and exactly a tile, one past, rows of two
+    to 87 staged pieces of 6 positions; sparse meetings, dense ones and every
+    pair meeting at once; vertex ids that share few hashed bits."""
     assert R * R * L >= 1 << 27
     g = load_golden("hand")
     rng = np.random.default_rng(R + L)
@@ -129,14 +129,15 @@ def test_meet_counts_at_join_tile_edges(cuda_device, oracle, R, L, vertices):
         assert np.array_equal(G.simrank_meet(_dev(pa), _dev(pb), R, L), ref_meet)
 
 
-@pytest.mark.parametrize("nq,R", [(300, 513), (80, 512)])
-def test_simrank_batch_joined_in_both_tiles(cuda_device, oracle, nq, R):
-    """Batches past the comparison limit: 592 tiles of 512 walks or more, and
-    fewer (tiles of 256).  Counts equal the oracle's."""
+@pytest.mark.parametrize("nq,R,side", [(300, 513, 512), (200, 512, 256), (80, 512, 128), (130, 385, 128)])
+def test_simrank_batch_joined_in_each_tile(cuda_device, oracle, nq, R, side):
+    """Batches past the comparison limit: tiles of the largest side that has
+    592 of them, at least 128.  Counts equal the oracle's."""
     import graphwalker_b200 as gw
     rp, ci = oracle.rmat_csr(12, 8, seed=4)
     L, rng = 8, np.random.default_rng(nq)
-    assert nq * R * R * L >= 1 << 27 and (nq * (-(-R // 512)) ** 2 >= 592) == (nq == 300)
+    assert nq * R * R * L >= 1 << 27
+    assert side == next((s for s in (512, 256) if nq * (-(-R // s)) ** 2 >= 592), 128)
     a, b = rng.integers(0, len(rp) - 1, (2, nq)).astype(np.uint32)
     b[:3] = a[:3]
     with gw.Graph.from_csr(rp, ci, oracle.compute_blocks(rp, 64)) as G:
