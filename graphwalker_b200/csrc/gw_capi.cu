@@ -483,6 +483,7 @@ gw_status gw_close(gw_ctx* ctx) {
                        &ctx->d_q_cand})
     b->release();
   ctx->release_pools();
+  ctx->pool_slab.release();
   ctx->h_rowptr.release();
   ctx->h_colidx.release();
   ctx->h_status.release();
