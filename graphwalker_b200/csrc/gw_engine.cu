@@ -256,14 +256,15 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   // pool table, and the superstep clock
   GW_CUDA(ctx, ctx->d_minhop.ensure((size_t)nb * 4), "minhop alloc");
   GW_CUDA(ctx, cudaMemsetAsync(ctx->d_minhop.p, 0xff, (size_t)nb * 4, st), "minhop clear");
-  GW_CUDA(ctx, ctx->d_pool_table.ensure(4 * (size_t)nb * 8 + 8 + 4 * 8), "pool table alloc");
-  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_pool_table.p, 0, 4 * (size_t)nb * 8 + 8 + 4 * 8, st), "pool table clear");
+  const size_t entries = PoolTable::stride(nb), table_bytes = 4 * entries * 8 + 8 + 4 * 8;
+  GW_CUDA(ctx, ctx->d_pool_table.ensure(table_bytes), "pool table alloc");
+  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_pool_table.p, 0, table_bytes, st), "pool table clear");
   PoolTable table;
   table.ptr = ctx->d_pool_table.as<gw_walk_rec*>();
-  table.n = ctx->d_pool_table.as<uint64_t>() + nb;
-  table.cap = table.n + nb;
-  table.place = table.cap + nb;
-  table.full = reinterpret_cast<uint32_t*>(table.place + nb);
+  table.n = ctx->d_pool_table.as<uint64_t>() + entries;
+  table.cap = table.n + entries;
+  table.place = table.cap + entries;
+  table.full = reinterpret_cast<uint32_t*>(table.place + entries);
   PartitionScratch ps{};
   ps.minhop = ctx->d_minhop.as<uint32_t>();
   ps.clock = reinterpret_cast<unsigned long long*>(table.full + 2);

@@ -76,7 +76,10 @@ cudaError_t rmat_build_csr(uint32_t scale, uint64_t nedges_raw, uint64_t seed, u
 // Launches k so that its CTAs may start while the kernel before it on the
 // stream drains (programmatic dependent launch): k must call
 // wait_for_previous() before it touches anything an earlier kernel writes or
-// reads.
+// reads.  What an earlier kernel of the stream writes is read with ordinary,
+// __ldcg or relaxed loads: the read-only path (__ldg, ld.global.nc, and so
+// `const T* __restrict__` parameters) wants data that no one writes from the
+// kernel's start on, and this kernel starts before its predecessors end.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
                              A... args) {
@@ -122,6 +125,9 @@ struct PartitionScratch {
 // scatter then does nothing, and the host grows the pools, uploads the table
 // (launch_fetch_pools) and launches the scatter again.
 struct PoolTable {
+  // Entries from one array to the next: whole 128-byte lines, so that no line
+  // holds both what the scan reads and what it writes for the scatter.
+  static size_t stride(uint32_t nbuckets) { return ((size_t)nbuckets + 15) / 16 * 16; }
   gw_walk_rec** ptr;
   uint64_t* n;      // records held
   uint64_t* cap;    // records the pool has room for

@@ -102,16 +102,15 @@ __global__ void fetch_pools_kernel(const uint64_t* src, PoolTable pools, uint32_
 // One walk per thread: 16 bytes in, 16 out, and 4 bytes of destination; its
 // tile's offset, its pool's pointer and place are cache hits.
 __global__ void __launch_bounds__(256)
-    partition_scatter_kernel(const gw_walk_rec* __restrict__ walks, uint64_t n, PartitionPlan plan,
-                             PartitionScratch ps, gw_walk_rec* const* __restrict__ ptr,
-                             const uint64_t* __restrict__ place, const uint32_t* full) {
+    partition_scatter_kernel(const gw_walk_rec* walks, uint64_t n, PartitionPlan plan, PartitionScratch ps,
+                             gw_walk_rec* const* ptr, const uint64_t* place, const uint32_t* full) {
   wait_for_previous();
   if (full && *full) return;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t x = ps.dest[i];
     if (x == kNoDest) continue;
     const uint32_t d = x & 0xffffu, tile = (uint32_t)(i / plan.tile());
-    const uint4 w = *(reinterpret_cast<const uint4*>(walks) + i);
+    const uint4 w = __ldcg(reinterpret_cast<const uint4*>(walks) + i);
     const uint64_t pos = place[d] + ps.tile_hist[(uint64_t)d * plan.ntiles + tile] + (x >> 16);
     *(reinterpret_cast<uint4*>(ptr[d]) + pos) = w;
   }

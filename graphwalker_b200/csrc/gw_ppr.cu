@@ -642,7 +642,7 @@ struct SlotKey {
   const unsigned long long* t;
   uint64_t pol;
   uint32_t tag, tag_mask;
-  __device__ unsigned long long fetch(uint32_t i) const { return ld_nc_u64(t + i, pol); }
+  __device__ unsigned long long fetch(uint32_t i) const { return load_slot(t + i, pol); }
   __device__ unsigned long long key(unsigned long long e) const {
     return slot_free(e, tag, tag_mask) ? 0ull
                                        : ((e & 0xffffffffull) << 32) | (uint32_t)~((uint32_t)(e >> 32) & ~tag_mask);
