@@ -116,28 +116,113 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   ctx->pool_size.assign(nb, 0);
   ctx->minstep.assign(nb, 0xffff);
   ctx->stats = gw_run_stats{};
-  // Without a budget the pools start as parts of one allocation, each with
-  // room for its walks and an even share of all: one allocation instead of
-  // one per block, and few pools that must grow.  (A budget moves pools out
-  // one by one, so each is then its own.)
+  // What the run needs besides its pools comes first.  Where it does not fit
+  // beside the pools an earlier run left, those go back: their walks are gone,
+  // and in parts of one slab they may hold more than this run will.
+  auto ensure = [&](gw_devbuf& b, size_t bytes) -> cudaError_t {
+    cudaError_t e = b.ensure(bytes);
+    if (e != cudaErrorMemoryAllocation || !ctx->pool_slab.p) return e;
+    cudaGetLastError();
+    ctx->release_pools();
+    return b.ensure(bytes);
+  };
+  uint64_t all = 0, maxpool = 0;
+  for (uint32_t b = 0; b < nb; ++b) {
+    all += ctx->pool_words[b].size();
+    maxpool = std::max<uint64_t>(maxpool, ctx->pool_words[b].size());
+  }
+  GW_CUDA(ctx, ensure(ctx->d_words, maxpool * 8), "word alloc");
+  if (ctx->pools_have_ids) GW_CUDA(ctx, ensure(ctx->d_ids, maxpool * 4), "id alloc");
+
+  // ---- sinks ----
+  SinkView sv{};
+  GW_CUDA(ctx, ensure(ctx->d_counts, (size_t)ctx->nv * 4), "counts alloc");
+  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_counts.p, 0, (size_t)ctx->nv * 4, st), "counts clear");
+  GW_CUDA(ctx, ensure(ctx->d_closure, 8), "closure alloc");
+  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_closure.p, 0, 8, st), "closure clear");
+  sv.counts = ctx->d_counts.as<uint32_t>();
+  sv.closure = ctx->d_closure.as<unsigned long long>();
+
+  // ---- streamed block slots ----
+  // One device slot holds the column slice of one block,
+  //   csr[beg_pos[blocks[b]] .. beg_pos[blocks[b+1]]);
+  // the row pointer of every block stays in HBM.
+  auto& slots = ctx->slots;
+  std::vector<uint32_t> slot_block;  // block held, kNoBlock if empty
+  std::vector<int> slot_of;          // per block: slot index or -1
+  const uint32_t nslots = streaming ? std::max<uint32_t>(2, std::min(ctx->nmblocks, nb)) : 0;
+  uint64_t max_e = 0;
+  if (streaming) {
+    const uint64_t* hr = ctx->h_rowptr.as<uint64_t>();
+    for (uint32_t b = 0; b < nb; ++b) max_e = std::max<uint64_t>(max_e, hr[ctx->blocks[b + 1]] - hr[ctx->blocks[b]]);
+  }
+  struct SlotRelease {  // large slots go back to the device when the run ends
+    gw_ctx* ctx;
+    bool drop;
+    ~SlotRelease() {
+      if (!drop) return;
+      cudaStreamSynchronize(ctx->copy_stream);
+      cudaStreamSynchronize(ctx->stream);
+      ctx->slots.release();
+    }
+  } slot_release{ctx, streaming && nslots * max_e * 4 > gw_ctx::BlockSlots::kKeptSlotBytes};
+  if (streaming) {
+    slot_block.assign(nslots, kNoBlock);
+    slot_of.assign(nb, -1);
+    if (slots.csr.size() != nslots) slots.release();
+    slots.csr.resize(nslots);
+    while (slots.ready.size() < nslots) {
+      cudaEvent_t ev[2] = {};
+      for (auto& x : ev) GW_CUDA(ctx, cudaEventCreateWithFlags(&x, cudaEventDisableTiming), "slot event");
+      slots.ready.push_back(ev[0]);
+      slots.free_ev.push_back(ev[1]);
+    }
+    for (uint32_t i = 0; i < nslots; ++i) {
+      GW_CUDA(ctx, ensure(slots.csr[i], std::max<uint64_t>(max_e, 1) * 4), "slot alloc");
+      cudaEventRecord(slots.free_ev[i], st);
+    }
+  }
+  // Without a budget the pools start as parts of one allocation: one
+  // allocation instead of one per block.  A part holds its walks, or what its
+  // pool held after an earlier run; and, so that few pools must grow, an even
+  // share of all walks more, where the device has room for that whatever the
+  // walks do: every pool growing, one after the other, until it could hold all
+  // of them (twice over, and one being copied).  Elsewhere, as on a device
+  // that the streamed graph's slots fill, the pools take no more than each by
+  // itself would.  Pools that an earlier run grew past their parts leave those
+  // idle, so they are laid out anew.  (A budget moves pools out one by one, so
+  // each is then its own.)
   {
-    uint64_t all = 0, want = 0;
-    bool fits = true;
-    for (uint32_t b = 0; b < nb; ++b) all += ctx->pool_words[b].size();
-    std::vector<uint64_t> room(nb);
+    bool fits = true, idle = false;
+    std::vector<uint64_t> room(nb), roomy(nb);
+    uint64_t want = 0, want_roomy = 0;
     for (uint32_t b = 0; b < nb; ++b) {
       const uint64_t m = ctx->pool_words[b].size(), held = ctx->pools[b].bytes / sizeof(gw_walk_rec);
-      if (held < m) fits = false;
-      room[b] = std::max<uint64_t>(held, m + all / nb + 1024);
+      fits = fits && held >= m;
+      idle = idle || (ctx->pool_slab.p && ctx->pools[b].p && !ctx->in_slab(ctx->pools[b].p));
+      room[b] = std::max(held, m);
+      roomy[b] = std::max<uint64_t>(held, m + all / nb + 1024);
       want += room[b];
+      want_roomy += roomy[b];
     }
     if (ctx->pool_budget) {
       if (ctx->pool_slab.p) ctx->release_pools();
-    } else if (!fits) {
+    } else if (!fits || idle) {
       ctx->release_pools();
-      if (ctx->pool_slab.ensure(want * sizeof(gw_walk_rec)) == cudaSuccess) {
+      const uint64_t most = std::max<uint64_t>(2 * all, 1024);  // what a pool may grow to
+      size_t free_bytes = 0, total_bytes = 0;
+      GW_CUDA(ctx, cudaMemGetInfo(&free_bytes, &total_bytes), "free memory");
+      // beside the pools: 4 bytes a walk of destinations, grown by halves, and the tile counts
+      const double needed = (double)sizeof(gw_walk_rec) * (want_roomy + (double)(nb + 1) * most) + 16.0 * all +
+                            (double)nb * 4 * (1184 + all / (kMaxRows * (uint64_t)kWalkThreads));
+      if (needed <= (double)free_bytes) {
+        room.swap(roomy);
+        want = want_roomy;
+      }
+      if (want && ctx->pool_slab.ensure(want * sizeof(gw_walk_rec)) == cudaSuccess) {
         uint64_t at = 0;
         for (uint32_t b = 0; b < nb; ++b) {
+          if (!room[b]) continue;
           ctx->pools[b].p = ctx->pool_slab.as<gw_walk_rec>() + at;
           ctx->pools[b].bytes = room[b] * sizeof(gw_walk_rec);
           at += room[b];
@@ -164,9 +249,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   constexpr uint64_t kChunk = gw_ctx::kPoolChunk;
   if (ctx->pool_budget) {
     // pinned chunks for every walk of the run, plus a partly filled one per block
-    uint64_t total = 0;
-    for (uint32_t b = 0; b < nb; ++b) total += ctx->pool_words[b].size();
-    const uint64_t nchunks = (total + kChunk - 1) / kChunk + nb;
+    const uint64_t nchunks = (all + kChunk - 1) / kChunk + nb;
     GW_CUDA(ctx, ctx->pool_arena.ensure(nchunks * kChunk * sizeof(gw_walk_rec)), "pool arena");
     ctx->arena_free.resize(nchunks);
     for (uint64_t c = 0; c < nchunks; ++c) ctx->arena_free[c] = (uint32_t)(nchunks - 1 - c);
@@ -233,10 +316,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
     }
     return e;
   };
-  uint64_t walksum = 0, maxpool = 0;
-  for (uint32_t b = 0; b < nb; ++b) maxpool = std::max<uint64_t>(maxpool, ctx->pool_words[b].size());
-  GW_CUDA(ctx, ctx->d_words.ensure(maxpool * 8), "word alloc");
-  if (ctx->pools_have_ids) GW_CUDA(ctx, ctx->d_ids.ensure(maxpool * 4), "id alloc");
+  uint64_t walksum = 0;
   // Mapped pinned memory the host and a superstep's kernels share, reached by
   // the device at its mapped address, so the small transfers of a superstep
   // never wait behind a block copy on the copy engine: what the scan reports
@@ -301,54 +381,6 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   std::vector<uint64_t> own_num;
   std::vector<uint32_t> own_min;
 
-  // ---- sinks ----
-  SinkView sv{};
-  GW_CUDA(ctx, ctx->d_counts.ensure((size_t)ctx->nv * 4), "counts alloc");
-  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_counts.p, 0, (size_t)ctx->nv * 4, st), "counts clear");
-  GW_CUDA(ctx, ctx->d_closure.ensure(8), "closure alloc");
-  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_closure.p, 0, 8, st), "closure clear");
-  sv.counts = ctx->d_counts.as<uint32_t>();
-  sv.closure = ctx->d_closure.as<unsigned long long>();
-
-  // ---- streamed block slots ----
-  // One device slot holds the column slice of one block,
-  //   csr[beg_pos[blocks[b]] .. beg_pos[blocks[b+1]]);
-  // the row pointer of every block stays in HBM.
-  auto& slots = ctx->slots;
-  std::vector<uint32_t> slot_block;  // block held, kNoBlock if empty
-  std::vector<int> slot_of;          // per block: slot index or -1
-  const uint32_t nslots = streaming ? std::max<uint32_t>(2, std::min(ctx->nmblocks, nb)) : 0;
-  uint64_t max_e = 0;
-  if (streaming) {
-    const uint64_t* hr = ctx->h_rowptr.as<uint64_t>();
-    for (uint32_t b = 0; b < nb; ++b) max_e = std::max<uint64_t>(max_e, hr[ctx->blocks[b + 1]] - hr[ctx->blocks[b]]);
-  }
-  struct SlotRelease {  // large slots go back to the device when the run ends
-    gw_ctx* ctx;
-    bool drop;
-    ~SlotRelease() {
-      if (!drop) return;
-      cudaStreamSynchronize(ctx->copy_stream);
-      cudaStreamSynchronize(ctx->stream);
-      ctx->slots.release();
-    }
-  } slot_release{ctx, streaming && nslots * max_e * 4 > gw_ctx::BlockSlots::kKeptSlotBytes};
-  if (streaming) {
-    slot_block.assign(nslots, kNoBlock);
-    slot_of.assign(nb, -1);
-    if (slots.csr.size() != nslots) slots.release();
-    slots.csr.resize(nslots);
-    while (slots.ready.size() < nslots) {
-      cudaEvent_t ev[2] = {};
-      for (auto& x : ev) GW_CUDA(ctx, cudaEventCreateWithFlags(&x, cudaEventDisableTiming), "slot event");
-      slots.ready.push_back(ev[0]);
-      slots.free_ev.push_back(ev[1]);
-    }
-    for (uint32_t i = 0; i < nslots; ++i) {
-      GW_CUDA(ctx, slots.csr[i].ensure(std::max<uint64_t>(max_e, 1) * 4), "slot alloc");
-      cudaEventRecord(slots.free_ev[i], st);
-    }
-  }
   // mapped device address of the pinned host columns (blocks read in place)
   const uint32_t* m_colidx = nullptr;
   if (streaming && ctx->mapped_max_walks) {
