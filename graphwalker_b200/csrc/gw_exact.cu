@@ -119,6 +119,32 @@ __device__ __forceinline__ uint32_t row_of(uint32_t end, uint32_t e) {
   return at;
 }
 
+// The first group of 32 rows, a multiple of 32 past v, that holds an edge past
+// e, or nv: a warp looks at the ends of 32 groups at a time, then of 32 times
+// as many, so a stretch of rows without edges costs its logarithm and not a
+// load for every 32 of them.  A call over a million vertices with 150 edges at
+// either end: three pushes 29.8 ms row group by row group, 1.3 so; nine pulls
+// 86.7 and 1.5.  Not inlined: runs that never need it pay for its code (scale
+// 16, 20 hops: 488 us a call, 527 with it inline).
+__device__ __noinline__ uint32_t next_rows(const unsigned long long* __restrict__ rows, uint32_t nv,
+                                           unsigned long long e, uint32_t v, uint32_t lane) {
+  uint32_t width = 32;  // rows a lane stands for
+  while (v < nv) {
+    const uint64_t row = (uint64_t)v + (uint64_t)(lane + 1) * width - 1;
+    const uint32_t ends = __ballot_sync(~0u, __ldg(rows + (row < nv ? row : nv - 1) + 1) > e);
+    if (ends) {  // inside the first such lane's rows
+      v += (uint32_t)(__ffs(ends) - 1) * width;
+      if (width == 32) return v;
+      width /= 32;
+    } else {
+      if ((uint64_t)v + 32ull * width >= nv) break;
+      v += 32 * width;
+      if (width < 1u << 20) width *= 32;
+    }
+  }
+  return nv;
+}
+
 // One warp per run of edges of the rows `rowptr`, which are sources; the lanes
 // hold the row ends of 32 consecutive ones.  Push: a row's share is added at
 // each of its targets.  Turn: a row's source is written into each target's row
@@ -146,6 +172,10 @@ __global__ void __launch_bounds__(kExactThreads)
       if (!TURN) sh = __ldg(share + mine);
     }
     const uint32_t last = __shfl_sync(~0u, end, 31);  // edges these vertices reach to
+    if (__builtin_expect(last == done, 0)) {
+      v = next_rows(rowptr, nv, e0 + done, v + 32, lane) - 32;
+      continue;
+    }
     const bool any = TURN || __any_sync(~0u, sh != 0.0);
     for (; any && done < last; done += 128) {
       uint32_t to[4];
@@ -189,6 +219,10 @@ __global__ void __launch_bounds__(kExactThreads)
       end = x < n ? (uint32_t)x : n;
     }
     const uint32_t last = __shfl_sync(~0u, end, 31);
+    if (__builtin_expect(last == done, 0)) {
+      v = next_rows(rows, nv, e0 + done, v + 32, lane) - 32;
+      continue;
+    }
     for (; done < last; done += 128) {
       const uint32_t e = done + lane * 4;
       uint32_t src[4], at[4];
