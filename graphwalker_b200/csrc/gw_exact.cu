@@ -24,8 +24,9 @@
 //    pushes spread over 2 or 4 copies of the targets gained 5 % and lost 11 %.
 //  * Pull: over in-edges, so an edge is a gather (284 G/s from the L2) and only
 //    the end of a vertex's run of edges an atomic: 85 us a hop, after 385 us of
-//    turning the graph around, a counting sort by target.  Taken from kPullHops
-//    hops on (six pushes cost 924 us, six pulls 895).
+//    turning the graph around, a counting sort by target.  The first pushes
+//    cost little, as few vertices have been reached: pull_from says from how
+//    many hops on a call pulls.
 #include <algorithm>
 
 #include "gw_ctx.h"
@@ -335,6 +336,28 @@ __global__ void __launch_bounds__(kExactThreads)
   }
 }
 
+// The workspace is kept in the context up to this size.
+constexpr size_t kKeptBytes = 256ull << 20;
+
+// The hops from which a call pulls instead of pushing, with a workspace of
+// `bytes` then.  Turning the graph around costs what 4 to 8 pulls do; a push of
+// a graph of average degree 16 costs about two pulls once all vertices are
+// reached, which takes a few hops, and fewer with a higher degree (calls from
+// the vertex of highest degree, pushed / pulled, us: scale 16, 8 hops 341 / 315;
+// scale 18, 8 hops 788 / 786, 10 hops 922 / 856; scale 20, 8 hops 2127 / 2263,
+// 12 hops 2742 / 2670; scale 19 and degree 48, 8 hops 2122 / 2088; from a vertex
+// of degree 1 pulling pays two hops later).  Below 2^17 edges a call is a chain
+// of launches, and the turn's are six more (scale 12, 20 hops: 258 / 294; the
+// uncapped rule, some hundred: 2588 / 2336).  A workspace too large to keep is allocated by each call, and the turn's
+// scattered writes leave the L2 (scale 24, from a vertex of degree 1, 7 hops: 58 ms
+// with a warp per vertex pushing, 71 pulled; 20 hops from the highest: 113 / 103).
+uint32_t pull_from(uint64_t nv, uint64_t ne, size_t bytes) {
+  if (ne == 0 || ne >= 1ull << 32) return 0xffffffffu;  // never (places are 32 bits)
+  if (ne < 1ull << 17) return 48;
+  if (bytes > kKeptBytes) return 20;
+  return ne < 1ull << 22 || ne >= 32 * nv ? 8 : 12;
+}
+
 }  // namespace
 }  // namespace gw
 
@@ -362,10 +385,8 @@ extern "C" gw_status gw_expected_visits(gw_ctx* ctx, const gw_walk_params* param
   // One workspace: arrivals, shares and visits (8 bytes a vertex each), the debt
   // sets, the turned graph's rows (8 bytes a vertex) and block sums, the runs'
   // first vertices, and the turned graph's places (4 bytes a vertex) and sources
-  // (4 bytes an edge).  Kept in the context while it is small.
-  constexpr size_t kKeptBytes = 256ull << 20;
-  constexpr uint32_t kPullHops = 7;
-  bool pull = hops >= kPullHops && ne > 0 && ne < (1ull << 32);
+  // (4 bytes an edge).
+  bool pull = true;
   const uint32_t nscan = (uint32_t)((nv + gw::kScanBlock - 1) / gw::kScanBlock);
   const size_t debts_at = 3 * nv * 8, rows_at = debts_at + gw::kSums * sizeof(gw::Debt);
   size_t first_at = 0, place_at = 0, turned_at = 0;
@@ -375,6 +396,7 @@ extern "C" gw_status gw_expected_visits(gw_ctx* ctx, const gw_walk_params* param
     turned_at = place_at + (pull ? nv * 4 : 0);
     return turned_at + (pull ? ne * 4 : 0);
   };
+  pull = hops >= gw::pull_from(nv, ne, lay_out());
   if (pull && ctx->d_exact.ensure(lay_out()) != cudaSuccess) {
     cudaGetLastError();  // no room to turn the graph around: push
     pull = false;
@@ -383,7 +405,7 @@ extern "C" gw_status gw_expected_visits(gw_ctx* ctx, const gw_walk_params* param
   struct Release {
     gw_ctx* ctx;
     ~Release() {
-      if (ctx->d_exact.bytes > kKeptBytes) ctx->d_exact.release();
+      if (ctx->d_exact.bytes > gw::kKeptBytes) ctx->d_exact.release();
     }
   } release{ctx};
   cudaStream_t st = ctx->stream;
