@@ -902,10 +902,18 @@ cudaError_t launch_clear_queries(const QueryView& qv, const unsigned long long* 
   return cudaGetLastError();
 }
 
-uint32_t topk_segment_slots(const uint32_t* table_mask, uint32_t nq) {
+uint32_t topk_segment_slots(const uint32_t* table_mask, uint32_t nq, uint32_t k) {
   uint64_t few = 0;
-  for (uint32_t q = 0; q < nq && few <= kTopkFewSegments; ++q) few += table_mask[q] / kTopkFewSlots + 1;
-  if (few <= kTopkFewSegments) return kTopkFewSlots;
+  bool merged = true;  // one CTA can hold every query's lists
+  for (uint32_t q = 0; q < nq && few <= kTopkFewSegments; ++q) {
+    const uint64_t segments = table_mask[q] / kTopkFewSlots + 1;
+    few += segments;
+    merged = merged && segments * k <= kTopkFewKeys;
+  }
+  // Past the register path twice the segments only double what one CTA merges
+  // (a call for one query of 300,000 walks, k = 500: 950 us with kTopkFewSlots,
+  // 845 with kTopkSegment; k = 100: 256 and 220).
+  if (few <= kTopkFewSegments && merged) return kTopkFewSlots;
   uint64_t s = kTopkSegment;
   while (s < (1ull << 30) && s / kTopkSegment * 64 < nq) s <<= 1;  // 64 queries per doubling
   return (uint32_t)s;

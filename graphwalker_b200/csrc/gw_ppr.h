@@ -59,11 +59,12 @@ cudaError_t launch_clear_tables(unsigned long long* tables, unsigned long long n
 constexpr uint32_t kClearSlots = 4096;
 cudaError_t launch_clear_queries(const QueryView& qv, const unsigned long long* d_piece_first, uint64_t npieces,
                                  cudaStream_t stream);
-// Table slots per top-k segment for a set of nq queries: kTopkFewSlots when
-// that makes a few segments (one large table is split over many CTAs), else
-// growing with nq, so that a large batch, which fills the GPU with whole
-// tables, is not split into small segments that each pay for their own sorts.
-uint32_t topk_segment_slots(const uint32_t* table_mask, uint32_t nq);
+// Table slots per top-k segment for a set of nq queries ranked in one launch:
+// kTopkFewSlots where topk_is_few then holds (one large table is split over
+// many CTAs), else kTopkSegment, growing with nq, so that a large batch, which
+// fills the GPU with whole tables, is not split into small segments that each
+// pay for their own sorts.
+uint32_t topk_segment_slots(const uint32_t* table_mask, uint32_t nq, uint32_t k);
 // seg_first[q + 1] = seg_first[q] + segments of query q's table (host).
 void topk_segment_prefix(const uint32_t* table_mask, uint32_t nq, uint32_t seg_slots, unsigned long long* seg_first);
 // Top-k of queries [q_begin, q_begin + q_count) into out[q * k + r], one CTA

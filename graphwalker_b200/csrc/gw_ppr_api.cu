@@ -42,7 +42,7 @@ struct QuerySet {
   std::vector<unsigned long long> prefix, id_base, toff;
   std::vector<uint32_t> sources, tmask;
   std::vector<unsigned long long> seg_first;  // top-k segments per query (prefix)
-  uint32_t seg_slots = 0;
+  std::vector<uint32_t> seg_slots;            // table slots of a segment: one for the set, or one per query
   uint64_t walks = 0, slots = 0;
   bool shared = false;        // the context's buffers (tagged), or this set's own (cleared, untagged)
   bool fresh_tables = false;  // d_tables was (re)allocated by upload_set: its content is undefined
@@ -100,10 +100,9 @@ gw_status plan_set(gw_ctx* ctx, const uint32_t* sources, const uint32_t* budgets
   return GW_OK;
 }
 
-// batched: the top-k segments grow with the set (64 queries per doubling),
-// so one launch ranks the whole set; one query at a time (plain), every table
-// splits into kTopkFewSlots-slot segments, so a large table is ranked by many
-// CTAs instead of one.
+// batched: one launch ranks the whole set, and its segments go by all of it;
+// one query at a time (plain), a launch ranks one, and its segments go by that
+// query's table.
 gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool batched) {
   const size_t n = s->qmap.size();
   const void* tables0 = s->d_tables->p;
@@ -111,8 +110,18 @@ gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool
   GW_CUDA(ctx, s->d_tables->ensure(s->slots * 8), "query tables alloc");
   s->fresh_tables = s->d_tables->p != tables0 || s->d_tables->bytes != table_bytes0;
   s->seg_first.resize(n + 1);
-  s->seg_slots = batched ? gw::topk_segment_slots(s->tmask.data(), (uint32_t)n) : gw::kTopkFewSlots;
-  gw::topk_segment_prefix(s->tmask.data(), (uint32_t)n, s->seg_slots, s->seg_first.data());
+  if (batched) {
+    s->seg_slots.assign(1, gw::topk_segment_slots(s->tmask.data(), (uint32_t)n, k));
+    gw::topk_segment_prefix(s->tmask.data(), (uint32_t)n, s->seg_slots[0], s->seg_first.data());
+  } else {
+    s->seg_first[0] = 0;
+    for (size_t q = 0; q < n; ++q) {
+      s->seg_slots.push_back(gw::topk_segment_slots(&s->tmask[q], 1, k));
+      unsigned long long one[2];
+      gw::topk_segment_prefix(&s->tmask[q], 1, s->seg_slots[q], one);
+      s->seg_first[q + 1] = s->seg_first[q] + one[1];
+    }
+  }
   const size_t nseg = s->seg_first[n];
   GW_CUDA(ctx, s->d_cand->ensure(nseg * k * 8 + 8), "top-k candidates");
   // 64-bit arrays first: prefix, seg_first (n + 1 each), id_base, toff, cursors
@@ -141,8 +150,9 @@ gw_status upload_set(gw_ctx* ctx, QuerySet* s, uint32_t k, cudaStream_t st, bool
   s->qv.table_mask = reinterpret_cast<uint32_t*>(put(s->tmask.data(), n, 4));
   s->seg_done = reinterpret_cast<uint32_t*>(put(nullptr, n, 4));
   s->seg_order = reinterpret_cast<uint32_t*>(d + at);
-  gw::topk_segment_order(s->tmask.data(), (uint32_t)n, s->seg_slots, s->seg_first.data(),
-                         reinterpret_cast<uint32_t*>(h + at));
+  if (batched)
+    gw::topk_segment_order(s->tmask.data(), (uint32_t)n, s->seg_slots[0], s->seg_first.data(),
+                           reinterpret_cast<uint32_t*>(h + at));
   Results* const r = reinterpret_cast<Results*>(d + s->back_at);
   s->qv.visits = &r->visits;
   s->status = &r->status;
@@ -209,10 +219,10 @@ cudaError_t run_set(gw_ctx* ctx, const gw_walk_params* p, const gw::WalkArgs& a,
       e = gw::launch_walk_queries((int)p->rule, s->qv, 0, s->walks, ctx->view(), a, s->status, threads_per_sm, st);
     cudaEventRecord(ev[2], st);
     if (e == cudaSuccess)
-      e = gw::launch_topk_segmented(s->qv, 0, n, k, s->ids, s->cnt, s->d_seg_first, s->seg_first.data(), s->seg_slots,
-                                    s->d_cand->as<unsigned long long>(), s->seg_done, s->seg_order, st);
+      e = gw::launch_topk_segmented(s->qv, 0, n, k, s->ids, s->cnt, s->d_seg_first, s->seg_first.data(),
+                                    s->seg_slots[0], s->d_cand->as<unsigned long long>(), s->seg_done, s->seg_order, st);
     cudaEventRecord(ev[3], st);
-    *launches += (s->seg_first[n] > n && !gw::topk_is_few(s->seg_first.data(), n, s->seg_slots, k) ? 3 : 2) + (cleared ? 1 : 0);
+    *launches += (s->seg_first[n] > n && !gw::topk_is_few(s->seg_first.data(), n, s->seg_slots[0], k) ? 3 : 2) + (cleared ? 1 : 0);
   } else {
     cudaEventRecord(ev[1], st);
     *launches += cleared ? 1 : 0;
@@ -223,9 +233,9 @@ cudaError_t run_set(gw_ctx* ctx, const gw_walk_params* p, const gw::WalkArgs& a,
       if (e == cudaSuccess)
         e = gw::launch_walk_queries((int)p->rule, one, s->prefix[q], s->prefix[q + 1], ctx->view(), a, s->status, 0, st);
       if (e == cudaSuccess)
-        e = gw::launch_topk_segmented(s->qv, q, 1, k, s->ids, s->cnt, s->d_seg_first, s->seg_first.data(), s->seg_slots,
-                                      s->d_cand->as<unsigned long long>(), s->seg_done, nullptr, st);
-      if (s->seg_first[q + 1] - s->seg_first[q] > 1 && !gw::topk_is_few(&s->seg_first[q], 1, s->seg_slots, k)) ++*launches;
+        e = gw::launch_topk_segmented(s->qv, q, 1, k, s->ids, s->cnt, s->d_seg_first, s->seg_first.data(),
+                                      s->seg_slots[q], s->d_cand->as<unsigned long long>(), s->seg_done, nullptr, st);
+      if (s->seg_first[q + 1] - s->seg_first[q] > 1 && !gw::topk_is_few(&s->seg_first[q], 1, s->seg_slots[q], k)) ++*launches;
     }
     cudaEventRecord(ev[2], st);
     cudaEventRecord(ev[3], st);

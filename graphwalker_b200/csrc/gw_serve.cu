@@ -276,7 +276,7 @@ bool superstep(gw_server* srv) {
   h.clear_first[n] = pieces;
   // queries whose last walks are in this superstep get their top-k after them;
   // a large table is ranked by several CTAs (segmented top-k)
-  const uint32_t seg_slots = gw::topk_segment_slots(h.tmask, nfin);
+  const uint32_t seg_slots = gw::topk_segment_slots(h.tmask, nfin, k);
   gw::topk_segment_prefix(h.tmask, nfin, seg_slots, h.seg_first);
   h.status[0] = 0;
   *h.cursor = 0;
