@@ -636,17 +636,25 @@ __device__ uint32_t block_select(Src src, uint32_t n, uint32_t k, unsigned long 
 }
 
 // Key of a table slot: count << 32 | ~vertex (larger = more visits, then the
-// smaller vertex id); 0 for a free slot (empty, or another batch's).
+// smaller vertex id); 0 for a free slot (empty, or another batch's).  For
+// kernels that start when the walks have ended: the read-only path streams
+// faster than coherent loads (64 queries of 100,000 walks, k = 100: 273 us of
+// top-k, 286).
 struct SlotKey {
   static constexpr unsigned long long kNone = kEmptySlot;
   const unsigned long long* t;
   uint64_t pol;
   uint32_t tag, tag_mask;
-  __device__ unsigned long long fetch(uint32_t i) const { return load_slot(t + i, pol); }
+  __device__ unsigned long long fetch(uint32_t i) const { return ld_nc_u64(t + i, pol); }
   __device__ unsigned long long key(unsigned long long e) const {
     return slot_free(e, tag, tag_mask) ? 0ull
                                        : ((e & 0xffffffffull) << 32) | (uint32_t)~((uint32_t)(e >> 32) & ~tag_mask);
   }
+};
+
+// The same in a kernel that was launched while the walks ran.
+struct LiveSlotKey : SlotKey {
+  __device__ unsigned long long fetch(uint32_t i) const { return load_slot(t + i, pol); }
 };
 
 struct CandKey {  // candidate lists hold keys already (0 = none)
@@ -781,7 +789,7 @@ __global__ void __launch_bounds__(kTopkFewThreads, 1)
   const uint32_t cap = qv.table_mask[q] + 1, first = (uint32_t)(g - seg_first[q]) * kTopkFewSlots;
   wait_for_previous();
   uint32_t n = block_select<kTopkFewThreads, kTopkFewSlots / kTopkFewThreads>(
-      table_slots(qv, q, first), cap - first < kTopkFewSlots ? cap - first : kTopkFewSlots, k, cand, select);
+      LiveSlotKey{table_slots(qv, q, first)}, cap - first < kTopkFewSlots ? cap - first : kTopkFewSlots, k, cand, select);
   if (nseg > 1) {
     for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) seg_cand[g * k + r] = r < n ? cand[r] : 0ull;
     __threadfence();
