@@ -660,8 +660,15 @@ struct LiveSlotKey : SlotKey {
 struct CandKey {  // candidate lists hold keys already (0 = none)
   static constexpr unsigned long long kNone = 0ull;
   const unsigned long long* c;
-  __device__ unsigned long long fetch(uint32_t i) const { return __ldcg(c + i); }  // other CTAs' lists
+  __device__ unsigned long long fetch(uint32_t i) const { return c[i]; }
   __device__ static unsigned long long key(unsigned long long v) { return v; }
+};
+
+// Lists that other CTAs of the same launch wrote.  (A merge in a launch of its
+// own reads plainly: one query of 300,000 walks, k = 500, 593 us of top-k, 656
+// with __ldcg.)
+struct LiveCandKey : CandKey {
+  __device__ unsigned long long fetch(uint32_t i) const { return __ldcg(c + i); }
 };
 
 // Row q of the result: the n <= k distinct keys of cand by rank, largest
@@ -801,8 +808,8 @@ __global__ void __launch_bounds__(kTopkFewThreads, 1)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    n = block_select<kTopkFewThreads, kTopkFewKeys / kTopkFewThreads>(CandKey{seg_cand + seg_first[q] * k}, nseg * k, k,
-                                                                      cand, select);
+    n = block_select<kTopkFewThreads, kTopkFewKeys / kTopkFewThreads>(LiveCandKey{{seg_cand + seg_first[q] * k}},
+                                                                      nseg * k, k, cand, select);
   }
   write_topk(cand, n, q, k, out_ids, out_counts);
 }

@@ -46,11 +46,12 @@ def test_dependent_kernels_do_not_read_predecessors_through_the_read_only_path()
 
 def test_dependent_kernels_read_tables_and_lists_coherently():
     text = _sources()["gw_ppr.cu"]
-    for reader, load in (("LiveSlotKey : SlotKey", "load_slot"), ("CandKey", "__ldcg")):
+    for reader, load in (("LiveSlotKey : SlotKey", "load_slot"), ("LiveCandKey : CandKey", "__ldcg")):
         fetch = re.search(rf"struct {reader} \{{.*?fetch\(uint32_t i\) const \{{ return (\w+)\(", text, re.S)
         assert fetch.group(1) == load, f"{reader}::fetch reads with {fetch.group(1)}"
     few = _kernels(text)["topk_few_kernel"][1]
     assert "LiveSlotKey{table_slots(" in few and few.count("table_slots(") == 1
+    assert "LiveCandKey{{seg_cand" in few and few.count("CandKey{") == 1
     slot = re.search(r"load_slot\(.*?\n\}", text, re.S).group(0)
     assert "ld.relaxed.gpu.global" in slot and ".nc" not in slot
 
