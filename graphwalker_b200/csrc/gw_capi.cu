@@ -235,16 +235,6 @@ bool fault_now(uint32_t kind) {
 // Errors of entry points that have no context (gw_last_error(NULL)).
 gw_status thread_error(gw_status code, const std::string& msg) { return set_thread_error(code, msg); }
 
-// Grid of a resident walk launch over n walks: the autotuned CTAs per SM
-// (gw_walk_autotune), or 0 for the launch's default shape.
-int resident_grid(gw_ctx* ctx, uint64_t n) {
-  if (ctx->walk_ctas_per_sm <= 0) return 0;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  const uint64_t need = (n + kWalkThreads - 1) / kWalkThreads, full = (uint64_t)sms * ctx->walk_ctas_per_sm;
-  return (int)(need < full ? (need ? need : 1) : full);
-}
-
 }  // namespace gw
 
 extern "C" {
@@ -645,7 +635,7 @@ gw_status gw_simrank_batch(gw_ctx* ctx, const gw_walk_params* params, const uint
   sv.paths = ctx->d_paths.as<uint32_t>();
   sv.plen = ctx->d_plen.as<uint32_t>();
   GW_CUDA(ctx, gw::launch_walk_resident(GW_RULE_RESTART, GW_SINK_PATH_RECORD, false, ctx->d_walks.as<gw_walk_rec>(),
-                                        n, ctx->view(), wa, sv, ctx->d_status.as<uint32_t>(), 0, st, nullptr),
+                                        n, ctx->view(), wa, sv, ctx->d_status.as<uint32_t>(), st, nullptr),
           "simrank walks");
   GW_CUDA(ctx, gw::launch_simrank_meet(ctx->d_paths.as<uint32_t>(), ctx->d_paths.as<uint32_t>(),
                                        ctx->d_sr_rows.as<unsigned long long>(), nq, R, L,
@@ -784,7 +774,7 @@ gw_status gw_run(gw_ctx* ctx, const gw_walk_params* params) {
   const bool use_win = params->sink == GW_SINK_VERTEX_COUNT && ctx->counts_window(sv.counts, &win);
   cudaError_t e = gw::launch_walk_resident((int)params->rule, (int)params->sink, params->aggregate != 0,
                                            ctx->d_walks.as<gw_walk_rec>(), n, ctx->view(), a, sv,
-                                           ctx->d_status.as<uint32_t>(), gw::resident_grid(ctx, n), st,
+                                           ctx->d_status.as<uint32_t>(), st,
                                            use_win ? &win : nullptr);
   cudaEventRecord(e1, st);
   if (e != cudaSuccess) {
@@ -932,7 +922,7 @@ gw_status gw_run_pools(gw_ctx* ctx, const gw_walk_params* params, const uint64_t
     if (e == cudaSuccess)
       e = gw::launch_walk_resident((int)params->rule, (int)params->sink, params->aggregate != 0,
                                    ctx->d_walks.as<gw_walk_rec>() + lo, m, ctx->view(), a, sv,
-                                   ctx->d_status.as<uint32_t>(), gw::resident_grid(ctx, m), ks,
+                                   ctx->d_status.as<uint32_t>(), ks,
                                    use_win ? &win : nullptr);
   }
   // the counts are complete once both compute streams are done
@@ -976,7 +966,7 @@ gw_status gw_walk_device(gw_ctx* ctx, const gw_walk_params* params, const gw_wal
   const bool use_win = params->sink == GW_SINK_VERTEX_COUNT && ctx->counts_window(d_counts, &win);
   cudaError_t e = gw::launch_walk_resident((int)params->rule, (int)params->sink, params->aggregate != 0,
                                            d_walks, n, ctx->view(), a, sv,
-                                           ctx->d_status.as<uint32_t>(), gw::resident_grid(ctx, n), st,
+                                           ctx->d_status.as<uint32_t>(), st,
                                            use_win ? &win : nullptr);
   if (e != cudaSuccess) return ctx->cuda_fail(e, "walk kernel launch");
   return GW_OK;
@@ -997,33 +987,31 @@ gw_status gw_walk_autotune(gw_ctx* ctx, const gw_walk_params* params, const gw_w
   gw::SinkView sv{};
   sv.counts = ctx->d_counts.as<uint32_t>();
   cudaStream_t st = ctx->stream;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  const int full = gw::walk_resident_grid((int)pp.rule, (int)pp.sink, pp.aggregate != 0, (uint64_t)sms * 64 * 1024);
-  const int max_per_sm = std::max(1, full / sms);
+  gw::WalkShapes trial{};  // the count sink's, whatever the caller's
+  gw::GraphPlan plan = ctx->view();
+  plan.shapes = &trial;
+  const gw::WalkShape shape = gw::walk_resident_shape((int)pp.rule, (int)pp.sink, pp.aggregate != 0, n, plan, a);
   cudaAccessPolicyWindow win;
   const bool use_win = ctx->counts_window(sv.counts, &win);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  int best = max_per_sm;
+  int best = shape.fit;
   float best_ms = 1e30f;
   // a quarter to full occupancy: a random-miss-bound kernel often runs best
   // well below full occupancy, where fewer requests queue at the DRAM
-  for (int c = std::max(1, max_per_sm / 4); c <= max_per_sm; ++c) {
-    ctx->walk_ctas_per_sm = c;
+  for (int c = std::max(1, shape.fit / 4); c <= shape.fit; ++c) {
+    trial.ctas[pp.rule][pp.sink][shape.records] = c;
     float sum = 0.f;
     for (int rep = 0; rep < 4; ++rep) {
       cudaEventRecord(e0, st);
-      cudaError_t e = gw::launch_walk_resident((int)pp.rule, (int)pp.sink, pp.aggregate != 0, d_walks, n, ctx->view(),
-                                               a, sv, ctx->d_status.as<uint32_t>(), gw::resident_grid(ctx, n), st,
-                                               use_win ? &win : nullptr);
+      cudaError_t e = gw::launch_walk_resident((int)pp.rule, (int)pp.sink, pp.aggregate != 0, d_walks, n, plan, a, sv,
+                                               ctx->d_status.as<uint32_t>(), st, use_win ? &win : nullptr);
       cudaEventRecord(e1, st);
       if (e == cudaSuccess) e = cudaEventSynchronize(e1);
       if (e != cudaSuccess) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        ctx->walk_ctas_per_sm = 0;
         return ctx->cuda_fail(e, "autotune launch");
       }
       float ms = 0.f;
@@ -1037,9 +1025,24 @@ gw_status gw_walk_autotune(gw_ctx* ctx, const gw_walk_params* params, const gw_w
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  ctx->walk_ctas_per_sm = best;
+  if (params->sink <= GW_SINK_CLOSURE_COUNT) ctx->walk_shapes.ctas[pp.rule][params->sink][shape.records] = best;
   if (ctas_per_sm) *ctas_per_sm = (uint32_t)best;
   return gw::take_status(ctx, st);
+}
+
+gw_status gw_walk_shape(gw_ctx* ctx, const gw_walk_params* params, uint64_t n, uint32_t* records,
+                        uint32_t* ctas_per_sm) {
+  if (!ctx) return set_thread_error(GW_E_INVALID, "NULL context");
+  if (ctx->residency != GW_RESIDENT_HBM) return ctx->fail(GW_E_STATE, "gw_walk_shape needs a resident graph");
+  gw::WalkArgs a;
+  const gw_status s = gw::make_walk_args(ctx, params, &a);
+  if (s != GW_OK) return s;
+  GW_CUDA(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
+  const gw::WalkShape shape = gw::walk_resident_shape((int)params->rule, (int)params->sink, params->aggregate != 0, n,
+                                                      ctx->view(), a);
+  if (records) *records = shape.records ? 1u : 0u;
+  if (ctas_per_sm) *ctas_per_sm = (uint32_t)shape.ctas;
+  return GW_OK;
 }
 
 gw_status gw_set_l2_fetch_granularity(gw_ctx* ctx, uint32_t bytes, uint32_t* previous) {

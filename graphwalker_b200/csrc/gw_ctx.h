@@ -182,7 +182,7 @@ struct gw_ctx {
   gw_hostbuf h_q_stage;           // pinned mirror of d_q_stage
   cudaEvent_t q_events[4] = {};   // a batch's phases
   int ppr_threads_per_sm = 0;  // autotuned launch shape (0 = full occupancy)
-  int walk_ctas_per_sm = 0;    // autotuned resident-walk launch shape (0 = full occupancy)
+  gw::WalkShapes walk_shapes{};  // autotuned resident-walk launch shapes
   uint32_t ppr_chunk = 0;      // autotuned walks per cursor grab (0 = default)
   // Batch tags of d_q_tables: the next tag, and whether every slot is empty
   // or carries a tag below it.
@@ -221,6 +221,7 @@ struct gw_ctx {
   }
   gw::GraphPlan view() const {
     gw::GraphPlan g;
+    g.shapes = &walk_shapes;
     g.vrec = d_vrec.as<const unsigned long long>();
     g.rowptr = d_rowptr.as<const unsigned long long>();
     g.colidx = d_colidx.as<const uint32_t>();
@@ -236,8 +237,6 @@ struct gw_ctx {
 namespace gw {
 // Records an error of an entry point without a context (gw_last_error(NULL)).
 gw_status thread_error(gw_status code, const std::string& msg);
-// Grid of a resident walk launch over n walks (the context's tuned shape).
-int resident_grid(gw_ctx* ctx, uint64_t n);
 // Fills launch constants from the API parameters; validates them.
 gw_status make_walk_args(gw_ctx* ctx, const gw_walk_params* p, WalkArgs* a);
 // Reads and clears the device status word (synchronises ctx->stream).

@@ -136,9 +136,16 @@ struct GraphView {
   uint32_t nv;
 };
 
+// CTAs per SM that the autotuner found for resident walks of a rule and sink
+// over the plain layout [0] and the edge records [1]; 0: not tuned.
+struct WalkShapes {
+  int ctas[GW_RULE_PPR + 1][GW_SINK_CLOSURE_COUNT + 1][2];
+};
+
 // The graph as launches see it: the kernels' view, and what the choice of a
-// layout goes by (host only).
+// layout and a launch shape goes by (host only).
 struct GraphPlan : GraphView {
+  const WalkShapes* shapes;
   uint64_t csr_bytes;  // columns and vertex records: what a walk over the plain layout touches
   uint64_t csr_limit;  // resident walks keep to the plain layout up to this many bytes (csr_walk_limit)
 };

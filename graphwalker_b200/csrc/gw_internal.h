@@ -28,9 +28,14 @@ constexpr uint32_t kDefaultHints = kHintColumnsEvictFirst | kHintCountsEvictLast
 // window (may be NULL): an L2 access policy window attached to the launch.
 cudaError_t launch_walk_resident(int rule, int sink, bool agg, const gw_walk_rec* walks, uint64_t n,
                                  const GraphPlan& g, const WalkArgs& a, const SinkView& s,
-                                 uint32_t* status, int grid, cudaStream_t stream,
+                                 uint32_t* status, cudaStream_t stream,
                                  const cudaAccessPolicyWindow* window = nullptr);
-int walk_resident_grid(int rule, int sink, bool agg, uint64_t n);
+// The layout that launch takes for n walks, its CTAs per SM, and the most that fit.
+struct WalkShape {
+  bool records;
+  int ctas, fit;
+};
+WalkShape walk_resident_shape(int rule, int sink, bool agg, uint64_t n, const GraphPlan& g, const WalkArgs& a);
 
 // ---- codec kernels (gw_walk.cu) ----
 // minhop (may be NULL): atomicMin of the walks' lowest hop.

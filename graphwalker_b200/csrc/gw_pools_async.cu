@@ -134,7 +134,7 @@ extern "C" gw_status gw_run_pools_submit(gw_ctx* ctx, const gw_walk_params* para
     if (e == cudaSuccess)
       e = gw::launch_walk_resident((int)params->rule, (int)params->sink, params->aggregate != 0,
                                    P.walks[s].as<gw_walk_rec>() + l, m, ctx->view(), a, sv, d_status,
-                                   gw::resident_grid(ctx, m), ks, use_win ? &win : nullptr);
+                                   ks, use_win ? &win : nullptr);
   }
   // the run is done once both compute streams are; its counts and status go
   // back on the read-back stream

@@ -455,17 +455,25 @@ int default_ctas_per_sm(bool records, uint64_t n, uint32_t path_stride) {
 }
 
 template <int RULE, int SINK, bool AGG>
+WalkShape resident_shape(uint64_t n, const GraphPlan& g, const WalkArgs& a) {
+  // a kernel's occupancy is asked for once: the call takes as long as a short launch
+  static const int fit[2] = {ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, false>),
+                             ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, true>)};
+  WalkShape s;
+  s.records = walks_use_records<RULE>(g, n);
+  s.fit = fit[s.records];
+  const int tuned = g.shapes ? g.shapes->ctas[RULE][SINK][s.records] : 0;
+  s.ctas = std::min(s.fit, tuned > 0 ? tuned : default_ctas_per_sm<RULE, SINK>(s.records, n, a.path_stride));
+  return s;
+}
+
+template <int RULE, int SINK, bool AGG>
 cudaError_t resident_dispatch(const gw_walk_rec* walks, uint64_t n, const GraphPlan& g,
-                              const WalkArgs& a, const SinkView& s, uint32_t* status, int grid,
+                              const WalkArgs& a, const SinkView& s, uint32_t* status,
                               cudaStream_t stream, const cudaAccessPolicyWindow* window) {
-  const bool records = walks_use_records<RULE>(g, n);
-  auto k = records ? walk_resident_kernel<RULE, SINK, AGG, true> : walk_resident_kernel<RULE, SINK, AGG, false>;
-  if (grid <= 0) {
-    // a kernel's occupancy is asked for once: the call takes as long as a short launch
-    static const int fit[2] = {ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, false>),
-                               ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, true>)};
-    grid = grid_of(std::min(fit[records], default_ctas_per_sm<RULE, SINK>(records, n, a.path_stride)), n);
-  }
+  const WalkShape shape = resident_shape<RULE, SINK, AGG>(n, g, a);
+  const int grid = grid_of(shape.ctas, n);
+  auto k = shape.records ? walk_resident_kernel<RULE, SINK, AGG, true> : walk_resident_kernel<RULE, SINK, AGG, false>;
   if (!window) {
     k<<<grid, kWalkThreads, 0, stream>>>(walks, n, g, a, s, status);
     return cudaGetLastError();
@@ -480,14 +488,6 @@ cudaError_t resident_dispatch(const gw_walk_rec* walks, uint64_t n, const GraphP
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k, walks, n, g, a, s, status);
-}
-
-template <int RULE, int SINK, bool AGG>
-int resident_grid(uint64_t n) {
-  // both variants have the same block shape; the larger register count bounds the grid
-  return grid_of(std::min(ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, false>),
-                          ctas_per_sm(walk_resident_kernel<RULE, SINK, AGG, true>)),
-                 n);
 }
 
 template <int RULE, int SINK, bool AGG>
@@ -530,16 +530,16 @@ cudaError_t block_dispatch(gw_walk_rec* walks, uint64_t n, const GraphView& g,
 
 cudaError_t launch_walk_resident(int rule, int sink, bool agg, const gw_walk_rec* walks, uint64_t n,
                                  const GraphPlan& g, const WalkArgs& a, const SinkView& s,
-                                 uint32_t* status, int grid, cudaStream_t stream,
+                                 uint32_t* status, cudaStream_t stream,
                                  const cudaAccessPolicyWindow* window) {
   if (n == 0) return cudaSuccess;
-  GW_RULE_CASES(resident_dispatch, walks, n, g, a, s, status, grid, stream, window)
+  GW_RULE_CASES(resident_dispatch, walks, n, g, a, s, status, stream, window)
   return cudaErrorInvalidValue;
 }
 
-int walk_resident_grid(int rule, int sink, bool agg, uint64_t n) {
-  GW_RULE_CASES(resident_grid, n)
-  return 0;
+WalkShape walk_resident_shape(int rule, int sink, bool agg, uint64_t n, const GraphPlan& g, const WalkArgs& a) {
+  GW_RULE_CASES(resident_shape, n, g, a)
+  return WalkShape{false, 1, 1};
 }
 
 cudaError_t launch_walk_block(int rule, int sink, bool agg, gw_walk_rec* walks, uint64_t n,

@@ -300,11 +300,19 @@ class Graph:
         return scores, meet
 
     def walk_autotune(self, p: WalkParams, walks, n: int) -> int:
-        """CTAs per SM chosen for this graph's later resident walk launches
-        (gw_walk_autotune), timed on the given device walks."""
+        """CTAs per SM chosen for this graph's later resident walk launches of
+        p's rule and sink over the layout these walks take (gw_walk_autotune),
+        timed on the given device walks."""
         out = c_uint32()
         check(load().gw_walk_autotune(self._h, byref(p), _ptr(walks), n, byref(out)), self._h)
         return out.value
+
+    def walk_shape(self, p: WalkParams, n: int) -> tuple[bool, int]:
+        """Whether a resident launch of n walks reads the edge records, and its
+        CTAs per SM (gw_walk_shape)."""
+        records, ctas = c_uint32(), c_uint32()
+        check(load().gw_walk_shape(self._h, byref(p), n, byref(records), byref(ctas)), self._h)
+        return bool(records.value), ctas.value
 
     def sync(self, stream: int | None = None) -> None:
         check(load().gw_sync(self._h, stream), self._h)

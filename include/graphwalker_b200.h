@@ -366,11 +366,18 @@ gw_status gw_sync(gw_ctx *ctx, void *stream);
 /* Times the resident walk kernel on the caller's device walks (counts into a
    scratch array of the context) at each occupancy from a quarter to full CTAs
    per SM, and keeps the fastest for this context's later resident launches
-   (gw_run, gw_run_pools, gw_walk_device).  The choice changes no result.
+   (gw_run, gw_run_pools, gw_walk_device) of params' rule and sink over the
+   layout that these walks take (gw_walk_shape); launches of another rule, sink
+   or layout keep the shape they have.  The choice changes no result.
    *ctas_per_sm (may be NULL) receives it.  (The reference has no tuner;
    its update loop is an OpenMP loop, graphwalker.hpp:257-270.)            */
 gw_status gw_walk_autotune(gw_ctx *ctx, const gw_walk_params *params, const gw_walk_rec *d_walks, uint64_t n,
                            uint32_t *ctas_per_sm);
+/* What a resident launch of n walks takes: *records (may be NULL) = 1 when it
+   reads the edge records, 0 when the plain CSR; *ctas_per_sm (may be NULL) its
+   CTAs per SM, tuned or by rule.  Nothing is launched.                      */
+gw_status gw_walk_shape(gw_ctx *ctx, const gw_walk_params *params, uint64_t n, uint32_t *records,
+                        uint32_t *ctas_per_sm);
 /* SimRank's meeting reduction (replaces the O(R^2 L) host loop of
    SimRank::computeResult, apps/simrank.cpp:71-84).  d_paths_a / d_paths_b:
    R walks of L visits each, row-major (walk i = row i), 0xFFFFFFFF = no
