@@ -88,7 +88,7 @@ def parse_args():
                     help="rawwalk: the headline raw-random-walk step; msppr: batched vs plain multi-source PPR; "
                          "serve: Poisson-arrival PPR serving, continuous batching vs one query per launch; "
                          "gather: the random 32-B sector probe alone (small profiler captures); "
-                         "walkonly: --steps resident walk launches at full occupancy, no autotuner, no extras "
+                         "walkonly: --steps resident walk launches in the default shape, no autotuner, no extras "
                          "(small profiler captures)")
     ap.add_argument("--probe-mb", type=int, default=2048, help="gather: buffer size")
     ap.add_argument("--probe-loads", type=int, default=1 << 26, help="gather: loads per launch")
@@ -425,7 +425,7 @@ def our_arm(args) -> None:
 
     kb = blocksize_kb_for(args.scale, args.edge_factor, args.nblocks)
     G = gw.Graph.rmat(args.scale, args.edge_factor, seed=args.graph_seed, blocksize_kb=kb, device=local)
-    layout = "erec" if G.set_edge_records(LAYOUT_MODE[args.layout]) else "csr"
+    G.set_edge_records(LAYOUT_MODE[args.layout])
     nv, L = G.nv, args.L
     stream = torch.cuda.current_stream()
     sh = stream.cuda_stream
@@ -440,6 +440,7 @@ def our_arm(args) -> None:
 
     # launch shape (CTAs per SM) timed on these walks before the warm-up
     tuned_ctas = G.walk_autotune(p, walks, nv)
+    layout = "erec" if G.walk_shape(p, nv)[0] else "csr"  # the one these launches read
 
     def barrier():
         if world > 1:
@@ -1246,7 +1247,7 @@ def gather_arm(args) -> None:
 
 def walkonly_arm(args) -> None:
     """`--steps` launches of the resident walk kernel over one walk per vertex
-    (jump rule, counts), at full occupancy and without the autotuner, for
+    (jump rule, counts), in the default launch shape, without the autotuner, for
     profiler captures at a chosen --scale."""
     import torch
 
@@ -1254,7 +1255,7 @@ def walkonly_arm(args) -> None:
     torch.cuda.set_device(0)
     with gw.Graph.rmat(args.scale, args.edge_factor, seed=args.graph_seed,
                        blocksize_kb=blocksize_kb_for(args.scale, args.edge_factor, args.nblocks)) as G:
-        layout = "erec" if G.set_edge_records(LAYOUT_MODE[args.layout]) else "csr"
+        G.set_edge_records(LAYOUT_MODE[args.layout])
         nv = G.nv
         v = torch.arange(nv, dtype=torch.int64, device="cuda")
         walks = torch.stack([v, v, v, torch.zeros_like(v)], 1).to(torch.int32).contiguous()
@@ -1263,6 +1264,7 @@ def walkonly_arm(args) -> None:
         p = gw.params(gw.RULE_JUMP, gw.SINK_VERTEX_COUNT if args.sink == "count" else gw.SINK_NONE, args.L,
                       seed=args.walk_seed, rng=gw.RNG_NATIVE if args.rng == "native" else gw.RNG_PHILOX,
                       cache_hints=None if args.hints < 0 else args.hints)
+        layout = "erec" if G.walk_shape(p, nv)[0] else "csr"  # the one the launches read
         ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
               for _ in range(max(1, args.steps))]
         for a, b in ev:

@@ -421,36 +421,50 @@ int grid_of(int per_sm, uint64_t n) {
 // record is one gather where the CSR takes two, but the records are four times
 // the columns, and a jump over them waits for a bitmap word, the target's
 // record and its edge in turn, in a warp whose other lanes wait for theirs.  So
-// jumping walks on graphs of a few L2 sizes read the CSR, and so do large sets
-// of the rules that end at a failed test (records / CSR, us, warm, random
-// starts, edge factor 16):
-//   jump: 4099 walks at scale 14 17.4 / 11.3 a call; 1 M at 20 169 / 147, at 21
-//     199 / 145; 4 M at 22 850 / 702 and at 23 (603 MB) 911 / 904, recording
-//     paths 819 / 793; one walk per vertex at 24 3742 / 4222;
-//   stop, uncapped: 1 M at 21 86 / 72 and 85 / 80; 4 M at 22 (301 MB) 357 / 323
-//     and 468 / 411, at 23 379 / 377 and 471 / 486; few walks 11.3 / 12.7 (8310
-//     at 18), 48.5 / 53.7 (39 k at 21): a chain of hops with two gathers each;
+// jumping walks read the CSR while its vertex records stay in the L2 beside the
+// visit counters, and so do large sets of the rules that end at a failed test
+// (us a launch, records in their shape / CSR; random starts, counts, the
+// reference's jump probability where none is given):
+//   jump: 4099 walks at R-MAT scale 14 15.4 / 9.8; 4 M at 22 833 / 702, with 40
+//     edges a vertex (671 MB) 925 / 841; 4 M on uniform graphs of 12 edges a
+//     vertex: 5.0 M vertices 1028 / 886, 6.0 M 1057 / 978, 7.0 M 1058 / 1038, 8.4 M
+//     1078 / 1113.  Beyond, and with other jump probabilities, the CSR loses: R-MAT
+//     23, 12 edges a vertex, probability 0.5: 561 / 671; 24 and 6 edges (511 MB):
+//     16.8 M walks 3192 / 3903, 2044 / 3034 with 0.5.  It keeps the chain of hops
+//     short for few walks: 24 and 6 edges 30,000 19.3 / 15.2 but 100,000 29.7 / 32.0;
+//     23 and 16 edges 100,000 30.7 / 27.8, 300,000 76 / 71, 1 M 246 / 237 but 161 / 178
+//     with 0.5.  One walk per vertex at 24 and 16 edges 3638 / 4210.
+//   stop, uncapped: 1 M at 21 91 / 78 and 134 / 119; 4 M at 22 (301 MB) 336 / 308
+//     and 456 / 416, at 23 389 / 398 and 501 / 508, at 24 and 2 edges (255 MB) 252 /
+//     288 (stop); few walks 11.1 / 12.3 (4099 at 23): a chain of hops with two
+//     gathers each;
 //   PPR, restart: their walks go back to a source whose record they hold (PPR:
 //     1 M at 20 148 / 162, 4 M at 22 560 / 656; restart: 127 / 122, 513 / 534).
 template <int RULE>
 bool walks_use_records(const GraphPlan& g, uint64_t n) {
+  constexpr uint32_t kCachedVertices = (48u << 20) / 8;  // whose records take 48 MB
   if (!g.erec) return false;
-  if (RULE == GW_RULE_JUMP) return g.csr_bytes > g.csr_limit;
-  return rule_returns<RULE>() || n < 1u << 19 || g.csr_bytes > g.csr_limit / 2;
+  if (RULE == GW_RULE_JUMP) {
+    const bool few = n < (g.nv <= 1u << 23 ? 1u << 18 : 1u << 16);
+    return g.csr_bytes > g.csr_limit || (g.nv > kCachedVertices && !few);
+  }
+  return rule_returns<RULE>() || n < 1u << 19 || g.csr_bytes > g.csr_limit / 2 || g.nv > kCachedVertices;
 }
 
 // CTAs per SM of a resident launch that no autotuner shaped: all that fit,
 // except where fewer requests in flight queue less at the DRAM: jumps over
 // edge records (one walk per vertex at scale 24: 8 CTAs 4.02 ms, 6 3.81, 5 3.74,
-// 4 3.80; at 23 1749, 1684, 1684, 1714 us), and restarting walks that record
+// 4 3.80; at 23 1749, 1684, 1684, 1714 us; up to a jump probability of about 0.3:
+// 23 and 12 edges a vertex 8 CTAs 803, 5 783 us with 0.25, 680 and 682 with 0.35,
+// 528 and 561 with 0.5), and restarting walks that record
 // paths beyond a third of the L2, whose rows then fill before they are written
 // out (3 M at 22, 11 visits: 8 CTAs 352 us, 6 332; 2 M at 21, 20 visits: 1.08
 // times; under 40 MB 0.94 to 1.04 times).  The PPR rule, whose walks end early,
 // wants them all (24: 2.21 ms with 8, 2.83 with 5).
 template <int RULE, int SINK>
-int default_ctas_per_sm(bool records, uint64_t n, uint32_t path_stride) {
-  if (RULE == GW_RULE_JUMP && records) return 5;
-  if (RULE == GW_RULE_RESTART && SINK == GW_SINK_PATH_RECORD && n * path_stride * 4 >= 40u << 20) return 6;
+int default_ctas_per_sm(bool records, uint64_t n, const WalkArgs& a) {
+  if (RULE == GW_RULE_JUMP && records && a.thr <= 0x80000000u / 10 * 3) return 5;
+  if (RULE == GW_RULE_RESTART && SINK == GW_SINK_PATH_RECORD && n * a.path_stride * 4 >= 40u << 20) return 6;
   return 1 << 16;
 }
 
@@ -463,7 +477,7 @@ WalkShape resident_shape(uint64_t n, const GraphPlan& g, const WalkArgs& a) {
   s.records = walks_use_records<RULE>(g, n);
   s.fit = fit[s.records];
   const int tuned = g.shapes ? g.shapes->ctas[RULE][SINK][s.records] : 0;
-  s.ctas = std::min(s.fit, tuned > 0 ? tuned : default_ctas_per_sm<RULE, SINK>(s.records, n, a.path_stride));
+  s.ctas = std::min(s.fit, tuned > 0 ? tuned : default_ctas_per_sm<RULE, SINK>(s.records, n, a));
   return s;
 }
 

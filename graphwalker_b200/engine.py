@@ -360,7 +360,8 @@ class Graph:
         check(load().gw_set_l2_persisting(self._h, nbytes), self._h)
 
     def set_edge_records(self, mode: int) -> bool:
-        """EDGE_RECORDS_OFF / _ON / _AUTO (gw_set_edge_records); True when in use."""
+        """EDGE_RECORDS_OFF / _ON / _AUTO (gw_set_edge_records); True when
+        built (walk_shape tells whether a launch reads them)."""
         built = c_uint32()
         check(load().gw_set_edge_records(self._h, mode, byref(built)), self._h)
         return bool(built.value)

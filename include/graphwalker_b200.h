@@ -460,16 +460,23 @@ gw_status gw_convert_edgelist(const char *path, uint64_t blocksize_kb, int32_t d
 /* ---- graph layout -------------------------------------------------------- */
 /* Edge records: a second copy of the column array in which each edge also
    carries its target's packed (first-edge offset, out-degree) record, 16 bytes
-   per edge.  A resident walk then moves along an edge with one random gather
-   instead of two (the record of the vertex it stands on comes with the edge
-   that led there).  Walks, counts and top-k lists are the same either way.
+   per edge.  A resident walk over them moves along an edge with one random
+   gather instead of two (the record of the vertex it stands on comes with the
+   edge that led there).  Queries, and restart and PPR walks, read them wherever
+   they are built.  Other resident walks read them where that is faster, by a
+   rule on the graph's and the set's sizes: on graphs of a few L2 sizes jumping
+   walks, and large sets of stop and uncapped walks, read the plain CSR beside
+   them (gw_walk_shape tells).  The environment's GW_CSR_WALK_BYTES, read when a
+   graph is opened, is the largest CSR read so (default 671088640, half of it
+   for stop and uncapped walks); with 0 every resident walk reads the records.
+   Walks, counts and top-k lists are the same either way.
    No counterpart in the reference, whose graph is the plain CSR
    (graphwalker.hpp:168-209 loads beg_pos and csr only).
    OFF frees them; ON builds them (GW_E_NOMEM if the device lacks the room);
    AUTO, the default of a resident graph, builds them when they take at most
    half of the free device memory (environment GW_EDGE_RECORDS=0 makes OFF
    the default).  Streamed residency drops them; a return to HBM residency
-   applies the mode again.  *built (may be NULL) = 1 when they are in use.   */
+   applies the mode again.  *built (may be NULL) = 1 when they are built.    */
 #define GW_EDGE_RECORDS_OFF 0u
 #define GW_EDGE_RECORDS_ON 1u
 #define GW_EDGE_RECORDS_AUTO 2u

@@ -28,6 +28,8 @@ def test_tuning_one_rule_leaves_the_others(cuda_device, monkeypatch, limit):
         if limit == "0":
             assert all(records for records, _ in before.values())
             assert before[gw.RULE_JUMP, gw.SINK_VERTEX_COUNT] == (True, 5)
+            often = G.walk_shape(gw.params(gw.RULE_JUMP, gw.SINK_VERTEX_COUNT, 12, jump_prob=0.5), n)
+            assert often[0] and often[1] > 5
         assert before[gw.RULE_RESTART, gw.SINK_PATH_RECORD][1] == 6
         expect = dict(before)
         walks = _walks(n, G.nv)
@@ -54,3 +56,43 @@ def test_a_shape_is_kept_per_layout(cuda_device):
         G.set_residency(gw.STREAM_PINNED, 2)
         with pytest.raises(gw.GwError):
             G.walk_shape(p, few)
+
+
+@pytest.mark.parametrize("scale,edges,rule,n,records",
+                         [(22, 2, "jump", 1 << 22, False), (23, 2, "jump", (1 << 18) - 1, False),
+                          (23, 2, "jump", 1 << 18, True), (24, 1, "jump", (1 << 16) - 1, False),
+                          (24, 1, "jump", 1 << 16, True), (22, 2, "stop", 1 << 19, False),
+                          (22, 2, "stop", (1 << 19) - 1, True), (23, 1, "stop", 1 << 19, True),
+                          (22, 2, "prob", 1 << 19, False), (23, 1, "prob", 1 << 19, True),
+                          (14, 2, "ppr", 1 << 19, True), (14, 2, "restart", 1 << 19, True)])
+def test_layout_by_sizes(cuda_device, scale, edges, rule, n, records):
+    """Vertices whose records leave the L2, and few walks."""
+    import graphwalker_b200 as gw
+    rule = {"jump": gw.RULE_JUMP, "stop": gw.RULE_STOP, "prob": gw.RULE_PROB, "ppr": gw.RULE_PPR,
+            "restart": gw.RULE_RESTART}[rule]
+    with gw.Graph.rmat(scale, edges, seed=2, blocksize_kb=1 << 16) as G:
+        assert G.set_edge_records(gw.EDGE_RECORDS_ON)
+        assert G.walk_shape(gw.params(rule, gw.SINK_VERTEX_COUNT, 10), n)[0] is records
+
+
+def test_jumps_over_many_vertices_are_not_slower_with_records(cuda_device):
+    """4 M jumping walks over 16.8 M vertices of two edges, a 255 MB CSR: the
+    records built beside it make them a quarter faster, when they are read."""
+    import torch
+
+    import graphwalker_b200 as gw
+    n, p = 1 << 22, gw.params(gw.RULE_JUMP, gw.SINK_VERTEX_COUNT, 10)
+    with gw.Graph.rmat(24, 2, seed=2, blocksize_kb=1 << 16) as G:
+        walks = _walks(n, G.nv)
+        counts = torch.zeros(G.nv, dtype=torch.int32, device="cuda")
+        ms = {}
+        for mode in (gw.EDGE_RECORDS_OFF, gw.EDGE_RECORDS_ON):
+            G.set_edge_records(mode)
+            for _ in range(5):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                G.walk_device(p, walks, n, counts=counts)
+                b.record()
+                b.synchronize()
+                ms[mode] = min(ms.get(mode, 1e9), a.elapsed_time(b))
+    assert ms[gw.EDGE_RECORDS_ON] < 0.92 * ms[gw.EDGE_RECORDS_OFF]
