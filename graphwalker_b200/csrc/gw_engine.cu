@@ -336,7 +336,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   // pool table, and the superstep clock
   GW_CUDA(ctx, ctx->d_minhop.ensure((size_t)nb * 4), "minhop alloc");
   GW_CUDA(ctx, cudaMemsetAsync(ctx->d_minhop.p, 0xff, (size_t)nb * 4, st), "minhop clear");
-  const size_t entries = PoolTable::stride(nb), table_bytes = 4 * entries * 8 + 8 + 4 * 8;
+  const size_t entries = PoolTable::stride(nb), table_bytes = 4 * entries * 8 + 8 + kClockWords * 8;
   GW_CUDA(ctx, ctx->d_pool_table.ensure(table_bytes), "pool table alloc");
   GW_CUDA(ctx, cudaMemsetAsync(ctx->d_pool_table.p, 0, table_bytes, st), "pool table clear");
   PoolTable table;
@@ -673,7 +673,7 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   if (e != cudaSuccess) return ctx->cuda_fail(e, "blocked engine");
   struct {
     uint32_t full, unused;
-    unsigned long long clock[4];
+    unsigned long long clock[kClockWords];
   } last = {};  // the end of the pool table's buffer
   GW_CUDA(ctx, cudaMemcpyAsync(&last, table.full, sizeof last, cudaMemcpyDeviceToHost, st), "clock read");
   s = take_status(ctx, st);  // synchronises the stream
@@ -682,8 +682,11 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   cudaEventElapsedTime(&ms, t0, t1);
   ctx->stats.supersteps = superstep;
   ctx->stats.ms_total = ms;
-  ctx->stats.ms_walk = last.clock[2] * 1e-6;  // the device's clock, stamped by the kernels' first CTAs
-  ctx->stats.ms_partition = last.clock[3] * 1e-6;
+  // the device's clock: from the walk kernel's first CTA to the scan's, and from there to the scatter's last
+  if (last.clock[kScatterEnd] > last.clock[kPartStart])
+    last.clock[kPartSum] += last.clock[kScatterEnd] - last.clock[kPartStart];
+  ctx->stats.ms_walk = last.clock[kWalkSum] * 1e-6;
+  ctx->stats.ms_partition = last.clock[kPartSum] * 1e-6;
   ctx->stats.ms_copy_wait = ms_copy_wait;
   ctx->last_nwalks = nwalks;
   ctx->last_sink = p->sink;

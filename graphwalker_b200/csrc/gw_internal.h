@@ -121,8 +121,12 @@ struct PartitionScratch {
   uint32_t* dest;       // per walk: destination | rank in the tile << 16, or kNoDest
   uint32_t* tile_hist;  // [bucket * ntiles + tile]: walk counts, then their exclusive scan per bucket
   uint32_t* minhop;     // per bucket: lowest hop of the walks that move there (0xffffffff = none)
-  unsigned long long* clock;  // NULL, or device clock: walk start, partition start, ns walking, ns partitioning
+  unsigned long long* clock;  // NULL, or the superstep clock, kClockWords of device ns
 };
+// The superstep clock: when the walk and the partition of the last superstep
+// started and when its scatter ended (the latest CTA's stamp), and what the
+// supersteps before it took in sum, walking and partitioning.
+enum : uint32_t { kWalkStart, kPartStart, kScatterEnd, kWalkSum, kPartSum, kClockWords };
 
 // The device pools a superstep's walks move to, one entry per block.  The scan
 // places the new walks behind the n held, advances n and empties the block

@@ -44,9 +44,10 @@ __global__ void __launch_bounds__(kScanThreads)
   let_next_start();
   wait_for_previous();
   if (ps.clock && b == 0 && threadIdx.x == 0) {
-    const unsigned long long t = device_ns();
-    ps.clock[2] += t - ps.clock[0];
-    ps.clock[1] = t;
+    const unsigned long long t = device_ns(), end = ps.clock[kScatterEnd];
+    if (end > ps.clock[kPartStart]) ps.clock[kPartSum] += end - ps.clock[kPartStart];  // the superstep before
+    ps.clock[kWalkSum] += t - ps.clock[kWalkStart];
+    ps.clock[kPartStart] = t;
   }
   uint32_t* const row = ps.tile_hist + (uint64_t)b * plan.ntiles;
   uint32_t carry = 0;
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(256)
     const uint64_t pos = place[d] + ps.tile_hist[(uint64_t)d * plan.ntiles + tile] + (x >> 16);
     *(reinterpret_cast<uint4*>(ptr[d]) + pos) = w;
   }
-  if (ps.clock && blockIdx.x == 0 && threadIdx.x == 0) ps.clock[3] += device_ns() - ps.clock[1];
+  if (ps.clock && threadIdx.x == 0) atomicMax(ps.clock + kScatterEnd, device_ns());
 }
 
 }  // namespace

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kWalkThreads)
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t base = (uint64_t)blockIdx.x * plan.tile();
   let_next_start();
-  if (ps.clock && blockIdx.x == 0 && threadIdx.x == 0) ps.clock[0] = clock_ns();
+  if (ps.clock && blockIdx.x == 0 && threadIdx.x == 0) ps.clock[kWalkStart] = clock_ns();
   uint64_t i = base + threadIdx.x;
   uint4 w = make_uint4(0, 0, 0, 0);
   if (i < n) w = *(reinterpret_cast<const uint4*>(walks) + i);

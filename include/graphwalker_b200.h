@@ -132,7 +132,7 @@ typedef struct gw_run_stats {
   uint64_t bytes_h2d;      /* graph bytes copied host->device (streaming)    */
   double ms_total;         /* device time of the last gw_run                 */
   double ms_walk;          /* of which walk kernels                          */
-  double ms_partition;     /* of which pool partitioning                     */
+  double ms_partition;     /* of which pool partitioning, to the scatter's end */
   double ms_copy_wait;     /* of which waiting for block copies              */
   uint64_t mapped_supersteps; /* block executions read in place from pinned
                                  host memory (streaming, gw_set_mapped_block_walks) */
