@@ -332,10 +332,13 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
   uint64_t* const m_moved = static_cast<uint64_t*>(m_xfer);
   const uint64_t* const m_table = m_moved + nb;
   std::vector<uint32_t> h_minhop(nb), h_totals(nb);
-  // device: minimum hops (reset by each scan after it has read them), the
-  // pool table, and the superstep clock
-  GW_CUDA(ctx, ctx->d_minhop.ensure((size_t)nb * 4), "minhop alloc");
-  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_minhop.p, 0xff, (size_t)nb * 4, st), "minhop clear");
+  // device: minimum hops (reset by each scan after it has read them; the
+  // initial pools' lie behind them, side by side), the pool table, and the
+  // superstep clock
+  const size_t minhop_words = (size_t)nb * (kMinhopStride + 1);
+  GW_CUDA(ctx, ctx->d_minhop.ensure(minhop_words * 4), "minhop alloc");
+  GW_CUDA(ctx, cudaMemsetAsync(ctx->d_minhop.p, 0xff, minhop_words * 4, st), "minhop clear");
+  uint32_t* const pool_minhop = ctx->d_minhop.as<uint32_t>() + (size_t)nb * kMinhopStride;
   const size_t entries = PoolTable::stride(nb), table_bytes = 4 * entries * 8 + 8 + kClockWords * 8;
   GW_CUDA(ctx, ctx->d_pool_table.ensure(table_bytes), "pool table alloc");
   GW_CUDA(ctx, cudaMemsetAsync(ctx->d_pool_table.p, 0, table_bytes, st), "pool table clear");
@@ -362,14 +365,13 @@ gw_status run_blocked(gw_ctx* ctx, const gw_walk_params* p) {
                                    cudaMemcpyHostToDevice, st), "id upload");
     GW_CUDA(ctx, launch_unpack_words(ctx->d_words.as<uint64_t>(),
                                      ctx->pools_have_ids ? ctx->d_ids.as<uint32_t>() : nullptr, m,
-                                     ctx->blocks[b], ctx->pools[b].as<gw_walk_rec>(), st, ps.minhop + b), "unpack");
+                                     ctx->blocks[b], ctx->pools[b].as<gw_walk_rec>(), st, pool_minhop + b), "unpack");
     ctx->pool_size[b] = m;
     walksum += m;
     bool moved = false;
     GW_CUDA(ctx, spill_to_budget(&moved), "pool spill");
   }
-  GW_CUDA(ctx, cudaMemcpyAsync(h_minhop.data(), ps.minhop, (size_t)nb * 4, cudaMemcpyDeviceToHost, st), "minimum hops");
-  GW_CUDA(ctx, cudaMemsetAsync(ps.minhop, 0xff, (size_t)nb * 4, st), "minhop clear");
+  GW_CUDA(ctx, cudaMemcpyAsync(h_minhop.data(), pool_minhop, (size_t)nb * 4, cudaMemcpyDeviceToHost, st), "minimum hops");
   GW_CUDA(ctx, cudaStreamSynchronize(st), "walk upload");
   for (uint32_t b = 0; b < nb; ++b) {
     ctx->minstep[b] = std::min<uint32_t>(h_minhop[b], 0xffffu);

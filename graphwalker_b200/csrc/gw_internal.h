@@ -116,11 +116,18 @@ struct PartitionPlan {
 };
 PartitionPlan partition_plan(uint64_t n, uint32_t nbuckets);
 
+// Every tile adds its lowest hops to the buckets' by atomics, so each bucket's
+// has a 128-byte line of its own: side by side, what they cost went by the
+// address the allocator gave the array (R-MAT scale 20, 261 blocks, 4000 walks a
+// superstep: 12.4 or 16.3 us of partition a superstep, 7.7 so; in 32-byte sectors
+// 8.8).
+constexpr uint32_t kMinhopStride = 32;
+
 // Device arrays a superstep's kernels hand on.
 struct PartitionScratch {
   uint32_t* dest;       // per walk: destination | rank in the tile << 16, or kNoDest
   uint32_t* tile_hist;  // [bucket * ntiles + tile]: walk counts, then their exclusive scan per bucket
-  uint32_t* minhop;     // per bucket: lowest hop of the walks that move there (0xffffffff = none)
+  uint32_t* minhop;     // per bucket, kMinhopStride apart: lowest hop of the walks that move there (0xffffffff = none)
   unsigned long long* clock;  // NULL, or the superstep clock, kClockWords of device ns
 };
 // The superstep clock: when the walk and the partition of the last superstep

@@ -76,8 +76,9 @@ __global__ void __launch_bounds__(kScanThreads)
     carry += __shfl_sync(~0u, y, kScanWarps - 1);
   }
   if (threadIdx.x != 0) return;
-  const uint32_t low = ps.minhop[b];
-  ps.minhop[b] = 0xffffffffu;  // for the next superstep
+  uint32_t* const minhop = ps.minhop + (size_t)b * kMinhopStride;
+  const uint32_t low = *minhop;
+  *minhop = 0xffffffffu;  // for the next superstep
   if (!moved) {
     totals[b] = carry;
     minhop_out[b] = low;

@@ -34,7 +34,7 @@ constexpr uint64_t align256(uint64_t x) { return (x + 255) & ~255ull; }
 constexpr uint64_t kOffDest = 0;
 constexpr uint64_t kOffHist = align256(kOffDest + kStaticMaxWalks * 4);
 constexpr uint64_t kOffMinhop = align256(kOffHist + kStaticMaxTiles * kStaticMaxBlocks * 4);
-constexpr uint64_t kOffTotals = align256(kOffMinhop + kStaticMaxBlocks * 4);
+constexpr uint64_t kOffTotals = align256(kOffMinhop + (uint64_t)kStaticMaxBlocks * kMinhopStride * 4);
 constexpr uint64_t kOffPtr = align256(kOffTotals + kStaticMaxBlocks * 4);
 constexpr uint64_t kOffPlace = align256(kOffPtr + kStaticMaxBlocks * 8);
 constexpr uint64_t kStaticBytes = align256(kOffPlace + kStaticMaxBlocks * 8);
@@ -180,7 +180,7 @@ extern "C" gw_status gw_superstep_static(gw_ctx* ctx, const gw_walk_params* para
   SinkView sv{};
   sv.counts = d_counts;
   // minhop starts at "no walk", whatever an interrupted call left there
-  GW_CUDA(ctx, cudaMemsetAsync(ps.minhop, 0xff, nb * sizeof(uint32_t), st), "clear minhop");
+  GW_CUDA(ctx, cudaMemsetAsync(ps.minhop, 0xff, (size_t)nb * kMinhopStride * sizeof(uint32_t), st), "clear minhop");
   if (n) {
     GW_CUDA(ctx, launch_walk_block((int)params->rule, (int)params->sink, params->aggregate != 0, d_walks, n,
                                    ctx->view(), nullptr, nullptr, a, sv, ctx->d_blocks.as<uint32_t>(), plan, ps,

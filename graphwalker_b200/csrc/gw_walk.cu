@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kWalkThreads)
   __syncthreads();
   for (uint32_t b = threadIdx.x; b < nb; b += kWalkThreads) {
     ps.tile_hist[(uint64_t)b * plan.ntiles + blockIdx.x] = total[b];
-    if (total[b]) atomicMin(ps.minhop + b, minhop[b]);
+    if (total[b]) atomicMin(ps.minhop + (size_t)b * kMinhopStride, minhop[b]);
   }
   if (st) atomicOr(status, st);
   if (SINK == GW_SINK_CLOSURE_COUNT && clos) atomicAdd(s.closure, (unsigned long long)clos);
