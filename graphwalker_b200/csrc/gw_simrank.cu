@@ -20,13 +20,18 @@
 //    keeps who has met, as in the pairs kernel, so a matching pair costs one
 //    bit, however many match.  111 us for the same queries (251 with the
 //    walks in hash chains and each match checked against all earlier
-//    positions, which also grew with coinciding walks: 3000 walks x 40 on 100
-//    vertices took 600 us, 120 with every pair compared, 150 so); bound by
-//    issue slots and the latency of two barriers and a few shared-memory
-//    round trips per position.
+//    positions); bound by issue slots and the latency of two barriers and a
+//    few shared-memory round trips per position.  Where walks coincide, most
+//    of a tile's are candidates at position after position: tiles of 128 and
+//    256 then compare every pair, a thread its walk with all of b's, and look
+//    again at every fourth position (one query of 3000 walks x 40 on 16
+//    vertices: 241 us a call with candidates alone, 197 all pairs, 185 so; 2000
+//    queries of 100 walks x 30 there: 1087, 664, 629).  Tiles of 512 belong to
+//    batches that joining serves best even so (512 queries on 16 vertices 977
+//    us, 1759 all pairs), and the code would cost them registers.
 //
 // Every position being a round of such latency, small batches keep comparing
-// pairs (kPairWork).  The grid's z dimension runs over queries: query q
+// pairs (kJoinPairs).  The grid's z dimension runs over queries: query q
 // compares the R walks at row offset rows[2q] of `a` with those at
 // rows[2q + 1] of `b`.
 #include <algorithm>
@@ -93,9 +98,43 @@ __global__ void __launch_bounds__(kPairThreads)
 constexpr uint32_t kNoVisit = 0xffffffffu;
 constexpr uint32_t kSrChunk = 6;  // positions staged at a time (12 leave two CTAs an SM, 4 are read in shorter pieces)
 
+// Every pair of a tile of TILE walks a side at one position: a thread compares
+// its walk of a with all of b, and keeps who has met in words (word w of walk i
+// at pairs[w * (TILE + 1) + i]) that it alone changes from one such position to
+// the next.  Returns the pairs that met now.
+template <uint32_t TILE>
+__device__ __forceinline__ uint32_t compare_all(const uint32_t* sa, const uint32_t* sb, uint32_t* pairs) {
+  const uint32_t p = sa[threadIdx.x];
+  uint32_t n = 0;
+#pragma unroll 1
+  for (uint32_t k = 0; k < TILE / 128; ++k) {
+    uint32_t* const mine = pairs + 4 * k * (TILE + 1) + threadIdx.x;
+    uint32_t old[4], now[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) old[e] = mine[e * (TILE + 1)];
+    if (__all_sync(~0u, (old[0] & old[1] & old[2] & old[3]) == ~0u)) continue;
+#pragma unroll 8
+    for (uint32_t w = 0; w < 32; ++w) {
+      const uint4 v = *reinterpret_cast<const uint4*>(sb + 128 * k + 4 * w);
+      const uint32_t bit = 1u << w;
+      if (p == v.x) now[0] |= bit;
+      if (p == v.y) now[1] |= bit;
+      if (p == v.z) now[2] |= bit;
+      if (p == v.w) now[3] |= bit;
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+      const uint32_t fresh = p == kNoVisit ? 0u : now[e] & ~old[e];
+      n += __popc(fresh);
+      if (fresh) mine[e * (TILE + 1)] = old[e] | fresh;
+    }
+  }
+  return n;
+}
+
 // LOG: a tile is 2^LOG walks of each side, one of each per thread.
 template <int LOG>
-__global__ void __launch_bounds__(1 << LOG)
+__global__ void __launch_bounds__(1 << LOG, LOG == 8 ? 8 : 0)
     simrank_join_kernel(const uint32_t* __restrict__ a0, const uint32_t* __restrict__ b0,
                         const unsigned long long* __restrict__ rows, uint32_t q0, uint32_t R, uint32_t L,
                         unsigned long long* __restrict__ meet0) {
@@ -105,8 +144,12 @@ __global__ void __launch_bounds__(1 << LOG)
   extern __shared__ __align__(16) uint32_t staged[];
   uint32_t(*const sa)[kRow] = reinterpret_cast<uint32_t(*)[kRow]>(staged);
   uint32_t(*const sb)[kRow] = sa + kSrChunk;
-  // a bit per pair that has met, by walk of a
-  uint32_t(*const pairs)[kWords] = reinterpret_cast<uint32_t(*)[kWords]>(staged + 2 * kSrChunk * kRow);
+  // a bit per pair that has met, word w of walk i of a: by words where threads
+  // compare a walk each, by walks where warps do
+  uint32_t* const pairs = staged + 2 * kSrChunk * kRow;
+  auto pair_word = [&](uint32_t w, uint32_t i) -> uint32_t& {
+    return pairs[LOG < 9 ? w * (kSrTile + 1) + i : i * kWords + w];
+  };
   __shared__ __align__(16) uint32_t bits[2][kBits / 32];  // one is cleared while the other is read
   __shared__ uint16_t cand[kSrTile];                       // a's walks whose vertex has its bit set
   __shared__ uint32_t ncand[2];
@@ -122,12 +165,15 @@ __global__ void __launch_bounds__(1 << LOG)
     for (uint32_t w = x; w < kBits / 128; w += kSrTile) reinterpret_cast<uint4*>(bits[t])[w] = make_uint4(0, 0, 0, 0);
   };
   clear(0);
-  for (uint32_t w = 0; w < kWords; ++w) pairs[0][w * kSrTile + x] = 0;
+  for (uint32_t w = x; w < kWords * (kSrTile + 1); w += kSrTile) pairs[w] = 0;
   if (x == 0) met = ncand[0] = ncand[1] = 0;
   if (x < kSrChunk) found[x] = 0;
   uint32_t l0 = 0;  // first position staged
+  uint32_t t = 0;   // the bitmap in use
+  bool dense = false;
   for (uint32_t l = 0; l < L; ++l) {
-    const uint32_t t = l & 1, c = l % kSrChunk;
+    const uint32_t c = l % kSrChunk;
+    if (LOG == 9) t = l & 1;
     if (c == 0) {
       __syncthreads();  // the candidates before are done with the rows staged before
       if (x < kSrChunk && found[x]) {
@@ -150,28 +196,40 @@ __global__ void __launch_bounds__(1 << LOG)
       l0 = l;
       __syncthreads();
     }
-    // mark b's vertices; half of a position's walks can stand on one vertex
-    // (the source they return to), so a bit that is set is left alone
-    const uint32_t u = sb[c][x], h = bit_of(u), m = 1u << (h & 31u);
-    if (u != kNoVisit && !(*reinterpret_cast<volatile uint32_t*>(&bits[t][h >> 5]) & m)) atomicOr(&bits[t][h >> 5], m);
-    __syncthreads();
-    if (met == na * nb) break;  // met changes only after the next barrier
-    // a's walks that may stand on one of them
-    const uint32_t v = sa[c][x], hv = bit_of(v);
-    const bool may = v != kNoVisit && ((bits[t][hv >> 5] >> (hv & 31u)) & 1u);
-    const uint32_t mine = __ballot_sync(~0u, may);
-    if (mine) {
-      uint32_t at = 0;
-      if (lane == 0) at = atomicAdd(&ncand[t], (uint32_t)__popc(mine));
-      at = __shfl_sync(~0u, at, 0) + __popc(mine & ((1u << lane) - 1u));
-      if (may) cand[at] = (uint16_t)x;
+    uint32_t count = 0;
+    // Where most of a's walks were candidates (all but an eighth in tiles of
+    // 256, where a candidate costs less), the next three positions are compared
+    // without looking.
+    if (!dense || (l & 3u) == 0) {
+      // mark b's vertices; half of a position's walks can stand on one vertex
+      // (the source they return to), so a bit that is set is left alone
+      const uint32_t u = sb[c][x], h = bit_of(u), m = 1u << (h & 31u);
+      if (u != kNoVisit && !(*reinterpret_cast<volatile uint32_t*>(&bits[t][h >> 5]) & m)) atomicOr(&bits[t][h >> 5], m);
+      __syncthreads();
+      if (met == na * nb) break;  // met changes only after the next barrier
+      // a's walks that may stand on one of them
+      const uint32_t v = sa[c][x], hv = bit_of(v);
+      const bool may = v != kNoVisit && ((bits[t][hv >> 5] >> (hv & 31u)) & 1u);
+      const uint32_t mine = __ballot_sync(~0u, may);
+      if (mine) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&ncand[t], (uint32_t)__popc(mine));
+        at = __shfl_sync(~0u, at, 0) + __popc(mine & ((1u << lane) - 1u));
+        if (may) cand[at] = (uint16_t)x;
+      }
+      clear(t ^ 1);
+      if (x == 0) ncand[t ^ 1] = 0;
+      __syncthreads();
+      count = ncand[t];
+      if (LOG < 9) t ^= 1;
+      dense = LOG == 7 ? 2 * count > na : LOG == 8 && 8 * count > 7 * na;
     }
-    clear(t ^ 1);
-    if (x == 0) ncand[t ^ 1] = 0;
-    __syncthreads();
-    // a warp per two candidates, its lanes over b's walks
     uint32_t n = 0;
-    for (uint32_t y = 2 * warp, count = ncand[t]; y < count; y += 2 * kWarps) {
+    if constexpr (LOG < 9) {
+      if (dense) n = compare_all<kSrTile>(sa[c], sb[c], pairs);
+    }
+    // a warp per two candidates, its lanes over b's walks
+    for (uint32_t y = LOG < 9 && dense ? count : 2 * warp; y < count; y += 2 * kWarps) {
       const bool two = y + 1 < count;
       const uint32_t i0 = cand[y], i1 = cand[two ? y + 1 : y], p0 = sa[c][i0], p1 = sa[c][i1];
       uint32_t now0 = 0, now1 = 0;  // lane w: word w of a walk's matches
@@ -190,14 +248,14 @@ __global__ void __launch_bounds__(1 << LOG)
         }
       }
       if (now0) {
-        const uint32_t old = pairs[i0][lane];
+        const uint32_t old = pair_word(lane, i0);
         n += __popc(now0 & ~old);
-        pairs[i0][lane] = old | now0;
+        pair_word(lane, i0) = old | now0;
       }
       if (two && now1) {
-        const uint32_t old = pairs[i1][lane];
+        const uint32_t old = pair_word(lane, i1);
         n += __popc(now1 & ~old);
-        pairs[i1][lane] = old | now1;
+        pair_word(lane, i1) = old | now1;
       }
     }
     n = __reduce_add_sync(~0u, n);
@@ -238,24 +296,29 @@ cudaError_t launch_simrank_meet(const uint32_t* a, const uint32_t* b, const unsi
                                 uint32_t R, uint32_t L, unsigned long long* meet, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(meet, 0, (size_t)nq * L * sizeof(unsigned long long), stream);
   if (e != cudaSuccess || R == 0 || L == 0) return e;
-  // Comparisons up to which pairs are compared.  A call of 8 queries of
-  // R = 1000, L = 11 takes 92 us so and 81 joined, 12 take 106 and 81, 64 take
-  // 283 and 97; 1000 walks on four vertices, one query: 34 us compared, 100
-  // joined (one walk compared at a time).
-  constexpr uint64_t kPairWork = 1ull << 27;
-  const uint64_t compares = (uint64_t)R * R * L;
-  const bool join = compares >= kPairWork / std::max(nq, 1u);
+  // Pairs of walks from which on they are joined, whatever the length: a
+  // position costs a tile the same few round trips, so what counts is how many
+  // pairs share them (calls of queries on uniform graphs of 8 edges a vertex, us,
+  // compared / joined; 100,000 vertices: one of R = 1000, 50 positions 122 / 136, of
+  // 2000 160 / 136, of 3000 214 / 142; 16 of 1000 310 / 158; on 300 vertices 124 / 162,
+  // 160 / 172, 222 / 188 and 320 / 235; one of 1000, 135 positions, on 16 vertices 80 /
+  // 170).  Up to 64 walks a query, half of the smallest tile joined is empty
+  // (5000 queries of 64: 1426 / 1493).
+  constexpr uint64_t kJoinPairs = 6000000;
+  const bool join = R > 64 && (uint64_t)R * R >= (kJoinPairs + nq - 1) / std::max(nq, 1u);
   // Joined tiles of 512 walks repeat the marking least (a call of 512 queries:
   // 0.30 ms, 0.34 in tiles of 256, 0.44 of 128) but need 592 tiles, four an
   // SM, to fill the chip (24 queries: 107 us, 85 and 93; one dense query of
   // 3000 walks x 40: 717, 379 and 270; all with one walk compared at a time).
-  uint32_t log = 9;
+  // Queries of up to 256 walks fit no larger one better (1000 of 200 walks, 50
+  // positions, 300 vertices: 864 us in tiles of 256, 747 of 128).
+  uint32_t log = R > 256 ? 9 : 7;
   for (; log > 7; --log) {
     const uint64_t wide = (R + (1ull << log) - 1) >> log;
     if (wide * wide * nq >= 592) break;
   }
   const uint32_t tile = join ? 1u << log : (uint32_t)kPairTile, tiles = (R + tile - 1) / tile;
-  const size_t smem = join ? (2 * kSrChunk * (size_t)(tile + 4) + tile * tile / 32) * 4 : 0;
+  const size_t smem = join ? (2 * kSrChunk * (size_t)(tile + 4) + tile / 32 * (size_t)(tile + 1)) * 4 : 0;
   auto k = !join ? simrank_pairs_kernel
            : log == 9 ? simrank_join_kernel<9> : log == 8 ? simrank_join_kernel<8> : simrank_join_kernel<7>;
   if (join) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
