@@ -26,6 +26,7 @@ struct gw_devbuf {
     bytes = 0;
     cudaError_t e = cudaMalloc(&p, n ? n : 16);
     if (e == cudaSuccess) bytes = n;
+    else cudaGetLastError();  // the caller's to report, not a later launch's
     return e;
   }
   // ensure() for a buffer whose need creeps up call after call: a growth
@@ -59,6 +60,7 @@ struct gw_hostbuf {
     bytes = 0;
     cudaError_t e = cudaHostAlloc(&p, n ? n : 16, cudaHostAllocDefault);
     if (e == cudaSuccess) bytes = n;
+    else cudaGetLastError();
     return e;
   }
   void release() {
@@ -217,6 +219,7 @@ struct gw_ctx {
     return code;
   }
   gw_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here: not an error of the next launch
     return fail(e == cudaErrorMemoryAllocation ? GW_E_NOMEM : GW_E_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
   gw::GraphPlan view() const {

@@ -108,3 +108,32 @@ def test_outgrown_pools(cuda_device, oracle, nblocks, budget):
                     assert np.array_equal(G.read_pool(b), np.stack(want, axis=1) if len(want[0])
                                           else np.zeros((0, 4), np.uint32)), f"block {b}"
     assert grown
+
+
+def test_a_call_that_runs_out_of_memory_leaves_no_error_behind(cuda_device, oracle):
+    """A query batch whose tables do not fit fails with GW_E_NOMEM; the next
+    call, and a graph opened after it, do not meet the allocation's error."""
+    import torch
+
+    import graphwalker_b200 as gw
+    rp, ci = oracle.rmat_csr(11, 8, seed=5)
+    blocks = oracle.compute_blocks(rp, 8)
+    cur = np.arange(len(rp) - 1, dtype=np.uint32)
+    p = gw.params(gw.RULE_JUMP, gw.SINK_VERTEX_COUNT, 10, seed=5)
+    ref = oracle.run_walks(rp, ci, cur, rule=0, L=10, seed=5)["counts"]
+    with gw.Graph.from_csr(rp, ci, blocks) as G:
+        torch.cuda.empty_cache()
+        held = [torch.empty(max(0, torch.cuda.mem_get_info()[0] - 256 * MB), dtype=torch.uint8, device="cuda")]
+        try:
+            with pytest.raises(gw.GwError) as e:  # 2^26 slots of 8 bytes
+                G.ppr(gw.params(gw.RULE_PPR, gw.SINK_NONE, 4), np.array([int(np.diff(rp).argmax())], np.uint32),
+                      np.array([1 << 23], np.uint32))
+            assert e.value.code == gw._lib.GW_E_NOMEM
+        finally:
+            held.clear()
+            torch.cuda.empty_cache()
+        for H in (G, gw.Graph.from_csr(rp, ci, blocks)):
+            H.add_walks_at(cur)
+            H.run(p)
+            assert np.array_equal(H.read_counts(), ref)
+        H.close()
