@@ -459,8 +459,9 @@ bool walks_use_records(const GraphPlan& g, uint64_t n) {
 // 528 and 561 with 0.5), and restarting walks that record
 // paths beyond a third of the L2, whose rows then fill before they are written
 // out (3 M at 22, 11 visits: 8 CTAs 352 us, 6 332; 2 M at 21, 20 visits: 1.08
-// times; under 40 MB 0.94 to 1.04 times).  The PPR rule, whose walks end early,
-// wants them all (24: 2.21 ms with 8, 2.83 with 5).
+// times; under 40 MB 0.94 to 1.04 times; stop walks' paths take 1.03 to 1.1
+// times as long with 6, PPR's 0.92 to 1.1).  The PPR rule, whose walks end
+// early, wants them all (24: 2.21 ms with 8, 2.83 with 5).
 template <int RULE, int SINK>
 int default_ctas_per_sm(bool records, uint64_t n, const WalkArgs& a) {
   if (RULE == GW_RULE_JUMP && records && a.thr <= 0x80000000u / 10 * 3) return 5;
